@@ -830,6 +830,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
       CFG_CUDA(cudaMemcpyAsync(p->horner_d, p->horner.data(), sizeof(T) * p->horner.size(),
                                cudaMemcpyHostToDevice, p->stream));
     }
+    if constexpr (sizeof(T) == 8) df_coeffs(p->sp, p->horner, &p->dfc);
     CFG_CUDA(cudaStreamSynchronize(p->stream));
     p->planned = true;
     return 0;
@@ -888,6 +889,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
     CFG_CUDA(cudaMemcpyAsync(p->horner_d, p->horner.data(), sizeof(T) * p->horner.size(),
                              cudaMemcpyHostToDevice, p->stream));
   }
+  if constexpr (sizeof(T) == 8) df_coeffs(p->sp, p->horner, &p->dfc);
   CFG_CUDA(cudaStreamSynchronize(p->stream));
   p->planned = true;
   return 0;

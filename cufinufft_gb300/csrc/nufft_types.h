@@ -45,15 +45,20 @@ constexpr int kMaxHornerRows = kMaxNS + 4;  // degree <= ns + 3
 // z^(deg-k) for tap j.  The coefficients travel inside the kernel's
 // parameter block, so the unrolled evaluation reads them straight from the
 // constant bank.
-// FP64 plans also carry the fitted polynomials as FP32 pairs (hi + lo, the
-// double-float interpolation kernel evaluates them without FP64 units),
-// scaled by 2^-E with E = round(beta log2 e) so that kernel values are ~1
-// (the kernel's peak e^beta, and the grid's 1/e^(d beta) scale, would leave
-// FP32's exponent range in 3D at wide kernels).
+// FP64 plans also carry the kernel for the double-float kernels (df.cuh), as
+// FP32 pairs and scaled by 2^-E with E = round(beta log2 e) so that kernel
+// values are ~1 (the kernel's peak e^beta, and the grid's 1/e^(d beta) scale,
+// would leave FP32's exponent range in 3D at wide kernels): the fitted
+// polynomials of taps p and ns-1-p as the (even, odd) parts of tap p's, row k
+// the coefficients of z^(2 (K - k)) and z^(2 (K - k) + 1), K = degree / 2;
+// and, for the exp form, c, beta log2 e and e^beta 2^-E 2^(k/64).
+constexpr int kMaxHornerHalf = kMaxHornerRows / 2 + 1;
 template <typename T> struct DFCoef {};
 template <> struct DFCoef<double> {
-  float hi[kMaxHornerRows * kMaxNS];
-  float lo[kMaxHornerRows * kMaxNS];
+  float2 ph[kMaxHornerHalf * (kMaxNS / 2)];
+  float2 pl[kMaxHornerHalf * (kMaxNS / 2)];
+  float2 exp2_tab[64];
+  float c_h, c_l, b_h, b_l;
 };
 
 template <typename T> struct KernelCoeffs {

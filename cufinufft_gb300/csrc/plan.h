@@ -56,6 +56,7 @@ template <typename T> struct Plan {
   T* fac[3] = {nullptr, nullptr, nullptr};
   std::vector<T> horner;  // fitted kernel polynomials (kerevalmeth 1), [k][j]
   T* horner_d = nullptr;  // device copy of the same
+  DFCoef<T> dfc{};        // FP64: the kernel's double-float constants
   // sorted points and bin tables
   int* idx = nullptr;
   int* i0[3] = {nullptr, nullptr, nullptr};
@@ -224,15 +225,8 @@ inline SpreadArgs<T> spread_args(Plan<T>* p) {
   a.kc.bl2e = (T)(p->sp.beta * 1.44269504088896340736);
   a.kc.horner = p->horner.empty() ? 0 : 1;
   a.kc.coef_g = p->horner_d;
-  for (size_t k = 0; k < p->horner.size() && k < (size_t)(kMaxHornerRows * kMaxNS); ++k) {
-    a.kc.coef[k] = p->horner[k];
-    if constexpr (sizeof(T) == 8) {
-      // scaled by 2^-E, E = round(beta log2 e): kernel values ~1, see df_scale_exp
-      const double v = std::ldexp(p->horner[k], -(int)std::lround(p->sp.beta * 1.44269504088896340736));
-      a.kc.df.hi[k] = (float)v;
-      a.kc.df.lo[k] = (float)(v - (double)a.kc.df.hi[k]);
-    }
-  }
+  for (size_t k = 0; k < p->horner.size() && k < (size_t)(kMaxHornerRows * kMaxNS); ++k) a.kc.coef[k] = p->horner[k];
+  a.kc.df = p->dfc;
   a.g.Nf = grid_cells(p);
   a.M = p->M;
   a.variant = p->variant;

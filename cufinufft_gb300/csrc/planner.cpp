@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 
 namespace cfg {
 
@@ -216,6 +217,36 @@ std::vector<double> horner_fit(const SpreaderParams& sp, int degree) {
     for (int r = 0; r <= K; ++r) coef[(size_t)r * ns + j] = (double)mono[K - r];
   }
   return coef;
+}
+
+static void split_pair(long double v, float* h, float* l) {
+  *h = (float)v;
+  *l = (float)(v - (long double)*h);
+}
+
+void df_coeffs(const SpreaderParams& sp, const std::vector<double>& horner, DFCoef<double>* out) {
+  std::memset(out, 0, sizeof(*out));
+  const double log2e = 1.44269504088896340736;
+  const int E = (int)std::lround(sp.beta * log2e);
+  split_pair(sp.c, &out->c_h, &out->c_l);
+  split_pair((long double)sp.beta * 1.442695040888963407359924681L, &out->b_h, &out->b_l);
+  for (int k = 0; k < 64; ++k)
+    split_pair(std::exp((long double)sp.beta - E * 0.693147180559945309417232121L) * std::exp2((long double)k / 64.0L),
+               &out->exp2_tab[k].x, &out->exp2_tab[k].y);
+  if (horner.empty()) return;
+  const int ns = sp.ns, deg = horner_degree<double>(ns), K = deg / 2, np = (ns + 1) / 2;
+  for (int p = 0; p < np; ++p)
+    for (int k = 0; k <= K; ++k) {
+      // powers m (even) and m + 1 (odd) of z; row r of the fit is z^(deg - r)
+      const int m = 2 * (K - k);
+      auto coef = [&](int power, int j) -> long double {
+        return power > deg ? 0.0L : (long double)horner[(size_t)(deg - power) * ns + j];
+      };
+      const long double even = 0.5L * (coef(m, p) + coef(m, ns - 1 - p));
+      const long double odd = 0.5L * (coef(m + 1, p) - coef(m + 1, ns - 1 - p));
+      split_pair(std::ldexp(even, -E), &out->ph[k * np + p].x, &out->pl[k * np + p].x);
+      split_pair(std::ldexp(odd, -E), &out->ph[k * np + p].y, &out->pl[k * np + p].y);
+    }
 }
 
 }  // namespace cfg

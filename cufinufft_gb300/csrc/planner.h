@@ -58,4 +58,8 @@ double es_kernel(double x, const SpreaderParams& sp);
 // by Chebyshev interpolation in long double.
 std::vector<double> horner_fit(const SpreaderParams& sp, int degree);
 
+// The kernel's constants for the double-float kernels (DFCoef); horner: the
+// FP64 fit of horner_fit at horner_degree<double>(ns), empty for the exp form.
+void df_coeffs(const SpreaderParams& sp, const std::vector<double>& horner, DFCoef<double>* out);
+
 }  // namespace cfg

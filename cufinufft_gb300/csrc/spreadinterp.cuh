@@ -27,7 +27,7 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "device_common.cuh"
+#include "df.cuh"
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -593,69 +593,57 @@ k_interp_sm(SpreadArgs<T> a, const __grid_constant__ CUtensorMap gmap, int tma) 
 
 // ---------------------------------------------------------------------------
 // Double-float interpolation for FP64 plans (SpreadArgs::fp64_df).  GB300's
-// FP64 units are a small fraction of its FP32 throughput, and the FP64 tap
-// loop (2 FMAs per tap, ns^d taps) plus the FP64 kernel evaluation (a Horner
-// step per tap value and degree) bound FP64 interpolation.  Here the tile
-// (loaded as for k_interp_sm) is converted in place to FP32 pairs (hi, lo per
-// component, the same 16 bytes per cell), the kernel rows are evaluated in
-// double-float (the fitted polynomials from FP32-pair coefficients, or the
-// FP64 exp form rounded to pairs), and the taps accumulate as a float sum
-// plus a float error term (two-sum and FMA product errors): ~2^-46
-// relative, ample for tol >= 1e-13, with FP32 instructions only.
-struct DFAcc {
-  float s, t;
-  __device__ __forceinline__ void zero() { s = t = 0.f; }
-  // += a * b
-  __device__ __forceinline__ void add_prod(DF a, float bh, float bl) {
-    const float p = __fmul_rn(a.h, bh);
-    float pe = __fmaf_rn(a.h, bh, -p);
-    pe = __fmaf_rn(a.h, bl, pe);
-    pe = __fmaf_rn(a.l, bh, pe);
-    float ns, e;
-    two_sum(s, p, ns, e);
-    s = ns;
-    t = __fadd_rn(t, __fadd_rn(e, pe));
-  }
-  __device__ __forceinline__ DF value() const { return df_renorm(s, t); }
-};
-
-// The kernel's power-of-two scale E = round(beta log2 e): kernel values are
-// taken times 2^-E and grid values times 2^(dim E), products unchanged
-// (exact scalings), every factor near 1 in FP32's exponent range.
-__device__ __forceinline__ int df_scale_exp(double beta) { return (int)rint(beta * 1.44269504088896340736); }
-
-// Kernel value phi(d - ns/2 + j) 2^-E in double-float.
-template <int NS, int HD>
-__device__ __forceinline__ DF df_kernel_tap(double d, int j, const KernelCoeffs<double>& kc) {
-  if (kc.horner) {
-    const DF z = df_from(2.0 * d - 1.0);
-    DF v;
-    v.h = kc.df.hi[j];
-    v.l = kc.df.lo[j];
-#pragma unroll
-    for (int k = 1; k <= HD; ++k) {
-      DF c;
-      c.h = kc.df.hi[k * NS + j];
-      c.l = kc.df.lo[k * NS + j];
-      v = df_fma(v, z, c);
-    }
-    return v;
-  }
-  const double x = d - 0.5 * NS + j;
-  return df_from(ldexp(es_value(kc.c * x * x, kc.beta), -df_scale_exp(kc.beta)));
+// FP64 units do about 2 FMAs per clock and SM, and the FP64 tap loop plus the
+// FP64 kernel evaluation bound FP64 interpolation.  Here the tile (loaded as
+// for k_interp_sm) is converted in place to FP32 pairs -- (re hi, im hi, re
+// lo, im lo) per cell, the same 16 bytes -- by integer operations, scaled by
+// the power of two that brings the tile's largest value to [1, 2); kernel rows
+// come from df.cuh; every product and sum is one packed FP32 instruction for
+// both components.
+//
+// What bounds it: the FMA pipe (a packed instruction takes two issue slots of
+// it), then shared memory (16 bytes per tap).  A tap added with a full
+// two-sum costs twelve packed instructions; with a biased sum (df2_acc_biased)
+// six, but its error is ~2^-48 of the largest possible row sum instead of
+// the actual one, ten times the two-sum's on its own.  So the biased form
+// takes the taps whose kernel weight is small enough that this is lost in the
+// error of the others: whole rows with ky kz below 2^-4 (84 of 121 rows at
+// ns = 11), and in the remaining rows the outer x taps, below 2^-3, biased
+// by the outer taps' own bound.  Emulated on random tiles the result keeps the
+// two-sum's error, 1.2e-14 at ns = 11 in 3D (all rows biased: 2.2e-13).
+// Measured against FP64 instructions: 1.4e-14 (3D, tol 1e-9), 1.5e-14 (2D,
+// tol 1e-12).  3.2e7 half-clustered points, 128^3 modes, ns 11: 51.6 -> 30.3 ms
+// against scalar two-sums, FP64 conversions of the tile and one Horner chain
+// per tap; 2^20 radial points, 1024^2 modes, ns 14: 0.73 -> 0.35 ms.
+//
+// log2 phi(x) <= -(2 / ln 2) (beta / ns) x^2 / ns relative to the peak, by
+// the square root's expansion, so both cuts are on squared distances.
+__host__ __device__ constexpr int df_outer_taps(int ns) {
+  // taps j with |x| >= m for every offset, m^2 the 2^-3 distance at beta =
+  // 2.3 ns: x_min(j) = ns/2 - 1 - j >= m
+  int n = 0;
+  while (2 * (n + 1) < ns && (ns - 2 - 2 * n) * (ns - 2 - 2 * n) * 6.636 >= 4 * 3.0 * ns && ns - 2 - 2 * n > 0) ++n;
+  return n;
 }
+
+// The kernel values' power-of-two scale (DFCoef).
+__device__ __forceinline__ int df_scale_exp(double beta) { return (int)rint(beta * 1.44269504088896340736); }
 
 template <int DIM, int NS>
 __global__ void __launch_bounds__(interp_threads_f64<DIM>(), interp_blocks_f64<DIM>())
 k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, int tma) {
   using C = double2;
-  constexpr int HD = horner_degree<double>(NS);
   constexpr int NY = DIM > 1 ? NS : 1;
   constexpr int NZ = DIM > 2 ? NS : 1;
+  constexpr int NO = df_outer_taps(NS);  // outer x taps on either side
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long tile_bar;
+  __shared__ float2 s_tab[64];
+  __shared__ unsigned s_max;
   C* tile = reinterpret_cast<C*>(tma ? smem_align128(smem_raw) : smem_raw);
   if (tma && threadIdx.x == 0) mbar_init(&tile_bar, 1);
+  if (threadIdx.x == 0) s_max = 0;
+  if (!a.kc.horner) df_table_fill(s_tab, a.kc);
   SubTile st = sub_tile_hdr<DIM, NS>(a.bins, blockIdx.x);
   if (tma) __syncthreads();
   const int t = blockIdx.y;
@@ -665,72 +653,118 @@ k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, i
   if (!bulk) tile_load_periodic<double>(tile, src, st, a.g);
   if (bulk) tile_copy_wait<double>(tile, &tile_bar, src, st, a.g, a.status, a.tma_wait_test);
   __syncthreads();
-  // the tile in place as FP32 pairs: (re hi, re lo, im hi, im lo) per cell,
-  // scaled by 2^(DIM E) (exact)
+  // the largest finite magnitude (high words compare as integers)
   float4* tdf = reinterpret_cast<float4*>(tile);
-  const double gscale = ldexp(1.0, DIM * df_scale_exp(a.kc.beta));
-  for (int i = threadIdx.x; i < st.ntile; i += blockDim.x) {
-    const C v = tile[i];
-    const DF r = df_from(v.x * gscale), m = df_from(v.y * gscale);
-    tdf[i] = make_float4(r.h, r.l, m.h, m.l);
+  {
+    unsigned m = 0;
+    for (int i = threadIdx.x; i < st.ntile; i += blockDim.x) {
+      const uint4 v = reinterpret_cast<const uint4*>(tile)[i];
+      const unsigned x = v.y & 0x7fffffffu, y = v.w & 0x7fffffffu;
+      if (x < 0x7ff00000u) m = max(m, x);
+      if (y < 0x7ff00000u) m = max(m, y);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
   }
   __syncthreads();
+  const unsigned hmax = s_max;
+  const int shift = 1023 - (int)(hmax >> 20);
+  // an upper bound of the scaled magnitudes, in (1, 2]
+  const float vmax = 1.f + (float)((hmax & 0xfffffu) + 1u) * 9.5367431640625e-07f;
+  for (int i = threadIdx.x; i < st.ntile; i += blockDim.x) {
+    const C v = tile[i];
+    const DF r = df_split(v.x, shift), m = df_split(v.y, shift);
+    tdf[i] = make_float4(r.h, m.h, r.l, m.l);
+  }
+  __syncthreads();
+  // kernel values carry 2^-E per axis, the tile 2^shift
+  const double oscale = ldexp(1.0, DIM * df_scale_exp(a.kc.beta) - shift);
+  const float row_cut = 4.f * NS * NS / (2.8853901f * (float)a.kc.beta);  // squared distance of weight 2^-4
   const int p_end = st.p0 + st.np;
   for (int p = st.p0 + threadIdx.x; p < p_end; p += blockDim.x) {
-    const int lx = a.pts.i0[0][p] - st.ox;
-    const int ly = DIM > 1 ? a.pts.i0[1][p] - st.oy : 0;
-    const int lz = DIM > 2 ? a.pts.i0[2][p] - st.oz : 0;
-    DF kx[NS], ky[NY];
-    const double d1 = a.pts.d[0][p];
+    int lc[3] = {0, 0, 0};
+    float kh[DIM][NS], kl[DIM][NS];
+#pragma unroll 1
+    for (int ax = 0; ax < DIM; ++ax) df_kernel_row<NS>(a.pts.d[ax][p], a.kc, s_tab, kh[ax], kl[ax]);
+    lc[0] = a.pts.i0[0][p] - st.ox;
+    if (DIM > 1) lc[1] = a.pts.i0[1][p] - st.oy;
+    if (DIM > 2) lc[2] = a.pts.i0[2][p] - st.oz;
+    float kx[NS], kxl[NS], outer = 0.f, all = 0.f;
 #pragma unroll
-    for (int j = 0; j < NS; ++j) kx[j] = df_kernel_tap<NS, HD>(d1, j, a.kc);
-    if (DIM > 1) {
-      const double d2 = a.pts.d[1][p];
-#pragma unroll
-      for (int j = 0; j < NY; ++j) ky[j] = df_kernel_tap<NS, HD>(d2, j, a.kc);
-    } else {
-      ky[0].h = 1.f;
-      ky[0].l = 0.f;
+    for (int j = 0; j < NS; ++j) {
+      kx[j] = kh[0][j];
+      kxl[j] = kl[0][j];
+      all += kx[j];
+      if (j < NO || j >= NS - NO) outer += kx[j];
     }
-    const double d3 = DIM > 2 ? a.pts.d[2][p] : 0.0;
-    DFAcc are, aim;
-    are.zero();
-    aim.zero();
+    const float2 bias_all = dup2(bias_for(fmaxf(all * vmax * 1.001f, 1e-20f)));
+    const float2 bias_out = dup2(bias_for(fmaxf(outer * vmax * 1.001f, 1e-20f)));
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 ts = zero, tt = zero;  // the point's sum and its error term
 #pragma unroll 1
     for (int dz = 0; dz < NZ; ++dz) {
-      DF kz;
-      if (DIM > 2) kz = df_kernel_tap<NS, HD>(d3, dz, a.kc);
-      const float4* plane = tdf + ((lz + dz) * st.TY + ly) * st.TX + lx;
-      // rows rolled: a fully unrolled ns x ns body of double-float taps
-      // outgrows the instruction cache (ncu: instruction-fetch stalls first);
-      // ky[dy] is then read from an L1-resident local array.  Measured: 3D
-      // ns 11 interp 66.1 -> 53.7 ms, 2D ns 14 1.01 -> 0.90 ms
+      float cut = row_cut;
+      if (DIM > 2) {
+        const float x = fmaxf(fabsf(dz + 0.5f - 0.5f * NS) - 0.5f, 0.f);
+        cut -= x * x;
+      }
+      float2 ps = zero, pt = zero;  // the plane's sum over rows
+      const float4* row = tdf + ((lc[2] + dz) * st.TY + lc[1]) * st.TX + lc[0];
+      // rows rolled: a fully unrolled ns x ns body outgrows the instruction cache
 #pragma unroll 1
-      for (int dy = 0; dy < NY; ++dy) {
-        const float4* row = plane + dy * st.TX;
-        DFAcc rre, rim;
-        rre.zero();
-        rim.zero();
+      for (int dy = 0; dy < NY; ++dy, row += st.TX) {
+        const float x = fmaxf(fabsf(dy + 0.5f - 0.5f * NS) - 0.5f, 0.f);
+        float2 s, e = zero, u = zero;
+        if (DIM == 1 || x * x < cut) {
+          if (NO > 0) {
+            s = bias_out;
 #pragma unroll
-        for (int dx = 0; dx < NS; ++dx) {
-          const float4 g = row[dx];
-          rre.add_prod(kx[dx], g.x, g.y);
-          rim.add_prod(kx[dx], g.z, g.w);
+            for (int j = 0; j < NO; ++j) {
+              const float4 g = row[j], f = row[NS - 1 - j];
+              df2_acc_biased(s, e, u, make_float2(g.x, g.y), make_float2(g.z, g.w), dup2(kx[j]), dup2(kxl[j]));
+              df2_acc_biased(s, e, u, make_float2(f.x, f.y), make_float2(f.z, f.w), dup2(kx[NS - 1 - j]),
+                             dup2(kxl[NS - 1 - j]));
+            }
+            s = sub2(s, bias_out);
+            e = add2(e, u);
+          } else {
+            s = zero;
+          }
+#pragma unroll
+          for (int j = NO; j < NS - NO; ++j) {
+            const float4 g = row[j];
+            df2_acc(s, e, make_float2(g.x, g.y), make_float2(g.z, g.w), dup2(kx[j]), dup2(kxl[j]));
+          }
+        } else {
+          s = bias_all;
+#pragma unroll
+          for (int j = 0; j < NS; ++j) {
+            const float4 g = row[j];
+            df2_acc_biased(s, e, u, make_float2(g.x, g.y), make_float2(g.z, g.w), dup2(kx[j]), dup2(kxl[j]));
+          }
+          s = sub2(s, bias_all);
+          e = add2(e, u);
         }
-        DF w = ky[dy];
-        if (DIM > 2) w = df_mul(w, kz);
-        const DF vr = rre.value(), vi = rim.value();
-        are.add_prod(w, vr.h, vr.l);
-        aim.add_prod(w, vi.h, vi.l);
+        if (DIM > 1) {
+          df2_acc(ps, pt, s, e, dup2(kh[DIM > 1 ? 1 : 0][dy]), dup2(kl[DIM > 1 ? 1 : 0][dy]));
+        } else {
+          ps = s;
+          pt = e;
+        }
+      }
+      if (DIM > 2) {
+        df2_acc(ts, tt, ps, pt, dup2(kh[DIM - 1][dz]), dup2(kl[DIM - 1][dz]));
+      } else {
+        ts = ps;
+        tt = pt;
       }
     }
     C o;
-    o.x = df_to(are.value());
-    o.y = df_to(aim.value());
+    o.x = ((double)ts.x + (double)tt.x) * oscale;
+    o.y = ((double)ts.y + (double)tt.y) * oscale;
     a.c_out[(size_t)t * a.M + a.pts.idx[p]] = o;
   }
 }
-
 
 // ---------------------------------------------------------------------------
 // Warp-cooperative variants.  A warp works on PPW = 32 / L points at a time;
