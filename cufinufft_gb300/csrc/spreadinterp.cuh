@@ -1321,6 +1321,10 @@ k_spread_sm_priv(SpreadArgs<T> a, int split) {
   cplx_flush<T>(tile0, a.fw + (size_t)t * a.g.Nf, st, a.g, PX);
 }
 
+}  // namespace cfg
+#include "spread_df.cuh"
+namespace cfg {
+
 // CUFINUFFT_SPREAD_PRIV=0: 2D subproblem spreading by the warp-cooperative
 // atomic kernel instead of the private-tile one.
 inline bool priv_spread_enabled() {
@@ -1933,6 +1937,27 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
       bool tc = false;
       if constexpr (sizeof(T) == 4 && NS <= 8) tc = tc_spread_enabled();
       split = slab && a.run && a.sub_ndense != nullptr && !tc;
+    }
+    // FP64 plans in double-float: every point of every subproblem (a dense
+    // run in FP64 registers costs five times the double-float taps, so the
+    // cell-run layout needs no second kernel)
+    if constexpr (sizeof(T) == 8 && DIM == 2) {
+      if (a.fp64_df && priv) {
+        const size_t smb = priv_df_bytes(NS, a.bins);
+        cudaError_t e = prepare_smem(k_spread_sm_priv_df<NS>, smb);
+        if (e != cudaSuccess) return e;
+        k_spread_sm_priv_df<NS><<<dim3(a.bins.nsub, a.ntr), 32 * kPrivDfWarps, smb, s>>>(a);
+        return cudaGetLastError();
+      }
+    }
+    if constexpr (sizeof(T) == 8 && DIM == 3) {
+      if (a.fp64_df && slab) {
+        const size_t smb = slab_df_bytes(NS, a.bins);
+        cudaError_t e = prepare_smem(k_spread_sm_slab_df<NS>, smb);
+        if (e != cudaSuccess) return e;
+        k_spread_sm_slab_df<NS><<<dim3(a.bins.nsub, a.ntr), 32 * NS, smb, s>>>(a);
+        return cudaGetLastError();
+      }
     }
     auto sparse = [&]() -> cudaError_t {
       if constexpr (DIM == 2) {
