@@ -70,31 +70,61 @@ __device__ __forceinline__ void df_flush(const float4* tile, double2* grid, cons
   }
 }
 
-// 3D: planes owned by warps, as k_spread_sm_slab.  A chunk of points is
-// staged by one thread per (point, axis): c kx as pairs, ky and kz.
-__host__ __device__ constexpr int slab_df_chunk(int) { return 32; }
-// bytes of one stage buffer
-__host__ __device__ constexpr size_t slab_df_stage(int ns) {
-  return (size_t)slab_df_chunk(ns) * (ns * (sizeof(float4) + 2 * sizeof(float2)) + sizeof(int2));
+// 3D: planes owned by warps, as k_spread_sm_slab, but with two warps to a
+// plane, one for the even tile rows and one for the odd ones: the FP64 tile
+// (110 KB at ns 10 with 16x16x2 bins) leaves one block per SM, and with one
+// warp per plane the SM had 2.5 warps per scheduler, waiting on their own
+// dependent sums (ncu: 37% of cycles issued, FMA pipe 33%, shared memory 40%).
+// A chunk of 32 points is staged by one warp per (tap pair, axis), lanes over
+// points: with one thread per (point, axis) row three warps worked while the
+// others waited at the barrier about as long as the chunk's taps take.  Staged
+// values are [tap][point], pitch 33 (conflict-free stores; the lanes of a row
+// read distinct banks).  81x96x75 modes, 2e6 points, tol 1e-9: 15.6 ms (FP64)
+// -> 6.8 ms (one warp per plane, one thread per row) -> 5.9 ms; now shared
+// memory is 69% busy and the FMA pipe 50%.
+constexpr int kSlabDfChunk = 32;
+constexpr int kSlabDfPitch = kSlabDfChunk + 1;
+// tile row pitch: the rows of one instruction are two tile rows apart, so
+// 2 pitch = NS (mod 8 cells of 16 bytes) puts its lanes in distinct banks
+// (odd widths: NS + 1, one conflict)
+__host__ __device__ constexpr int slab_df_pitch(int tx, int ns) {
+  return tx + ((((ns + 1) / 2 - tx) % 4) + 4) % 4;
 }
-inline size_t slab_df_bytes(int ns, const BinTables& bt) {
-  const size_t px = slab_pitch(bt.bs[0] + ns - 1, ns);
-  return px * (bt.bs[1] + ns - 1) * (bt.bs[2] + ns - 1) * sizeof(float4) + 2 * slab_df_stage(ns);
+__host__ __device__ constexpr int slab_df_instrs(int ns) { return ((ns + 1) / 2 + 32 / ns - 1) / (32 / ns); }
+// bytes of one stage buffer: c kx, ky, kz [NS] x pitch, tile offsets
+__host__ __device__ constexpr size_t slab_df_stage(int ns) {
+  return (size_t)kSlabDfPitch * 3 * ns * sizeof(float4) + kSlabDfChunk * sizeof(int2);
+}
+// The widest tiles give up the row padding (ns 13 with 16x16x2 bins), then the
+// second stage buffer (ns 14), before the kernel is given up.
+struct SlabDfShape {
+  int pitch, nbuf;
+  size_t bytes;
+};
+inline SlabDfShape slab_df_shape(int ns, const BinTables& bt, size_t limit) {
+  const int tx = bt.bs[0] + ns - 1;
+  const size_t rows = (size_t)(bt.bs[1] + ns - 1) * (bt.bs[2] + ns - 1) * sizeof(float4), st = slab_df_stage(ns);
+  const int pad = slab_df_pitch(tx, ns);
+  const SlabDfShape v[3] = {{pad, 2, pad * rows + 2 * st}, {tx, 2, tx * rows + 2 * st}, {tx, 1, tx * rows + st}};
+  for (const SlabDfShape& x : v)
+    if (x.bytes <= limit) return x;
+  return SlabDfShape{0, 0, 0};
 }
 
 template <int NS>
-__global__ void __launch_bounds__(32 * NS)
-k_spread_sm_slab_df(SpreadArgs<double> a) {
-  constexpr int R = 32 / NS;            // tile rows per warp instruction
-  constexpr int NR = (NS + R - 1) / R;  // instructions per plane
-  constexpr int CH = slab_df_chunk(NS);
+__global__ void __launch_bounds__(64 * NS)
+k_spread_sm_slab_df(SpreadArgs<double> a, int PX, int nbuf) {
+  constexpr int R = 32 / NS;                        // tile rows per warp instruction
+  constexpr int NR = slab_df_instrs(NS);            // instructions per half plane
+  constexpr int NP = (NS + 1) / 2;                  // tap pairs
+  constexpr int CH = kSlabDfChunk, CP = kSlabDfPitch;
+  constexpr bool kFullRows = 32 % NS == 0 && NS % 2 == 0 && (NS / 2) % R == 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float2 s_tab[64];
   __shared__ unsigned s_max;
   if (threadIdx.x == 0) s_max = 0;
   if (!a.kc.horner) df_table_fill(s_tab, a.kc);
   const SubTile st = sub_tile_block<3, NS>(a.bins, blockIdx.x);  // synchronises
-  const int PX = slab_pitch(st.TX, NS);
   const int PP = PX * st.TY;  // plane stride
   const int ncell = PP * st.TZ;
   float4* tile = reinterpret_cast<float4*>(smem_raw);
@@ -104,60 +134,78 @@ k_spread_sm_slab_df(SpreadArgs<double> a) {
   const double2* cin = a.c_in + (size_t)t * a.M;
   const int shift = strength_shift(cin, a.pts.idx + st.p0, st.np, &s_max);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int dx = lane % NS, dyl = lane / NS;
+  const int residue = warp % NS, half = warp / NS;
+  const int dx = lane % NS, dyl = min(lane / NS, R - 1);
   const bool lane_on = lane < R * NS;
-  constexpr bool kFullRows = 32 % NS == 0 && (NS * NS) % 32 == 0;
   for (int c0 = 0, buf = 0; c0 < st.np; c0 += CH, buf ^= 1) {
+    if (nbuf == 1) {
+      if (c0) __syncthreads();  // the previous chunk's reads of the one buffer
+      buf = 0;
+    }
     unsigned char* sb = stage0 + buf * slab_df_stage(NS);
-    float4* s_ck = reinterpret_cast<float4*>(sb);                // [CH][NS]
-    float2* s_ky = reinterpret_cast<float2*>(s_ck + CH * NS);    // [CH][NS]
-    float2* s_kz = s_ky + CH * NS;                               // [CH][NS]
-    int2* s_bl = reinterpret_cast<int2*>(s_kz + CH * NS);
+    // kernel values duplicated, (h, h, l, l): the packed operands of both
+    // components come with one load
+    float4* s_ck = reinterpret_cast<float4*>(sb);  // [NS][CP] c kx
+    float4* s_ky = s_ck + NS * CP;                 // [NS][CP]
+    float4* s_kz = s_ky + NS * CP;                 // [NS][CP]
+    int2* s_bl = reinterpret_cast<int2*>(s_kz + NS * CP);      // tile offset, lz mod NS and ly's parity
     const int nq = min(CH, st.np - c0);
-    for (int i = threadIdx.x; i < 3 * CH; i += blockDim.x) {
-      const int ax = i / CH, q = i - ax * CH;
-      if (q >= nq) continue;
-      const int p = st.p0 + c0 + q;
-      float kh[NS], kl[NS];
-      df_kernel_row<NS>(a.pts.d[ax][p], a.kc, s_tab, kh, kl);
-      if (ax == 0) {
-        const double2 v = cin[a.pts.idx[p]];
-        const DF re = df_split(v.x, shift), im = df_split(v.y, shift);
-        const DF2 c = DF2{make_float2(re.h, im.h), make_float2(re.l, im.l)};
-#pragma unroll
-        for (int j = 0; j < NS; ++j) {
-          const DF2 w = df2_mul(c, DF2{dup2(kh[j]), dup2(kl[j])});
-          s_ck[q * NS + j] = make_float4(w.h.x, w.h.y, w.l.x, w.l.y);
+    for (int w = warp; w < 3 * NP; w += 2 * NS) {  // warp-uniform (axis, tap pair)
+      const int ax = w % 3, tp = w / 3;
+      if (lane < nq) {
+        const int p = st.p0 + c0 + lane;
+        const DF2 k = df_kernel_pair<NS>(a.pts.d[ax][p], tp, a.kc, s_tab);
+        if (ax == 0) {
+          const double2 v = cin[a.pts.idx[p]];
+          const DF re = df_split(v.x, shift), im = df_split(v.y, shift);
+          const DF2 c = DF2{make_float2(re.h, im.h), make_float2(re.l, im.l)};
+          const DF2 u = df2_mul(c, DF2{dup2(k.h.x), dup2(k.l.x)});
+          s_ck[tp * CP + lane] = make_float4(u.h.x, u.h.y, u.l.x, u.l.y);
+          if (tp != NS - 1 - tp) {
+            const DF2 v2 = df2_mul(c, DF2{dup2(k.h.y), dup2(k.l.y)});
+            s_ck[(NS - 1 - tp) * CP + lane] = make_float4(v2.h.x, v2.h.y, v2.l.x, v2.l.y);
+          }
+          if (tp == 0) {
+            const int lx = a.pts.i0[0][p] - st.ox, ly = a.pts.i0[1][p] - st.oy, lz = a.pts.i0[2][p] - st.oz;
+            s_bl[lane] = make_int2((lz * st.TY + ly) * PX + lx, 2 * (lz % NS) + (ly & 1));
+          }
+        } else {
+          float4* dst = ax == 1 ? s_ky : s_kz;
+          dst[tp * CP + lane] = make_float4(k.h.x, k.h.x, k.l.x, k.l.x);
+          dst[(NS - 1 - tp) * CP + lane] = tp == NS - 1 - tp ? make_float4(k.h.x, k.h.x, k.l.x, k.l.x)
+                                                              : make_float4(k.h.y, k.h.y, k.l.y, k.l.y);
         }
-        const int lx = a.pts.i0[0][p] - st.ox, ly = a.pts.i0[1][p] - st.oy, lz = a.pts.i0[2][p] - st.oz;
-        s_bl[q] = make_int2((lz * st.TY + ly) * PX + lx, lz % NS);
-      } else {
-        float2* dst = (ax == 1 ? s_ky : s_kz) + q * NS;
-#pragma unroll
-        for (int j = 0; j < NS; ++j) dst[j] = make_float2(kh[j], kl[j]);
       }
     }
     __syncthreads();  // (also: the tile is zeroed; the other buffer is free)
     for (int q = 0; q < nq; ++q) {
       const int2 bl = s_bl[q];
-      int dz = warp - bl.y;
-      dz += dz < 0 ? NS : 0;  // the plane of residue `warp`
-      const float2 kz = s_kz[q * NS + dz];
-      const float4 ck = s_ck[q * NS + dx];
-      const DF2 u = df2_mul(DF2{make_float2(ck.x, ck.y), make_float2(ck.z, ck.w)}, DF2{dup2(kz.x), dup2(kz.y)});
+      int dz = residue - (bl.y >> 1);
+      dz += dz < 0 ? NS : 0;                     // the plane of this warp's residue
+      const int dy0 = (half ^ bl.y) & 1;         // its rows: ly + dy = half (mod 2)
+      const float4 kz = s_kz[dz * CP + q];
+      const float4 ck = s_ck[dx * CP + q];
+      const DF2 u = df2_mul(DF2{make_float2(ck.x, ck.y), make_float2(ck.z, ck.w)},
+                            DF2{make_float2(kz.x, kz.y), make_float2(kz.z, kz.w)});
+      const float2 nuh = neg2(u.h);
       float4* cell = tile + bl.x + dz * PP + dx;
-      float2 ky[NR];
-#pragma unroll
-      for (int r = 0; r < NR; ++r) ky[r] = s_ky[q * NS + min(r * R + dyl, NS - 1)];
+      // lanes without a tap read one of the point's rows all the same and only
+      // leave out the store (no divergent branch); just the last instruction
+      // can run past the support
+      const int d0 = 2 * dyl + dy0, dlast = min(d0 + 2 * (NR - 1) * R, NS - 1);
+      float4 v[NR], ky[NR];
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
-        const int dy = r * R + dyl;
-        if (kFullRows || (lane_on && dy < NS)) {
-          const float4 v = cell[dy * PX];
-          float2 s = make_float2(v.x, v.y), e = make_float2(v.z, v.w);
-          df2_acc_long(s, e, u.h, u.l, dup2(ky[r].x), dup2(ky[r].y));
-          cell[dy * PX] = make_float4(s.x, s.y, e.x, e.y);
-        }
+        const int dy = r == NR - 1 ? dlast : d0 + 2 * r * R;
+        ky[r] = s_ky[dy * CP + q];
+        v[r] = cell[dy * PX];
+      }
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        float2 s = make_float2(v[r].x, v[r].y), e = make_float2(v[r].z, v[r].w);
+        df2_acc_long(s, e, u.h, nuh, u.l, make_float2(ky[r].x, ky[r].y), make_float2(ky[r].z, ky[r].w));
+        if (kFullRows || (lane_on && (r < NR - 1 || d0 + 2 * r * R < NS)))
+          cell[(r == NR - 1 ? dlast : d0 + 2 * r * R) * PX] = make_float4(s.x, s.y, e.x, e.y);
       }
       __syncwarp();  // this point's stores before the next point's loads
     }
@@ -233,20 +281,23 @@ k_spread_sm_priv_df(SpreadArgs<double> a) {
     __syncwarp();
     for (int q = 0; q < nq; ++q) {
       const float4 ck = s_ck[q * NS + dx];
-      const float2 uh = make_float2(ck.x, ck.y), ul = make_float2(ck.z, ck.w);
+      const float2 uh = make_float2(ck.x, ck.y), ul = make_float2(ck.z, ck.w), nuh = neg2(uh);
       float4* cell = tile + s_base[q] + dx;
+      // lanes without a tap take the point's last row and leave out the store
+      float4 w[NR];
       float2 ky[NR];
 #pragma unroll
-      for (int r = 0; r < NR; ++r) ky[r] = s_ky[q * NS + min(r * R + dyl, NS - 1)];
+      for (int r = 0; r < NR; ++r) {
+        const int dy = min(r * R + dyl, NS - 1);
+        ky[r] = s_ky[q * NS + dy];
+        w[r] = cell[dy * PX];
+      }
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const int dy = r * R + dyl;
-        if (kFullRows || (lane_on && dy < NS)) {
-          const float4 w = cell[dy * PX];
-          float2 s = make_float2(w.x, w.y), e = make_float2(w.z, w.w);
-          df2_acc_long(s, e, uh, ul, dup2(ky[r].x), dup2(ky[r].y));
-          cell[dy * PX] = make_float4(s.x, s.y, e.x, e.y);
-        }
+        float2 s = make_float2(w[r].x, w[r].y), e = make_float2(w[r].z, w[r].w);
+        df2_acc_long(s, e, uh, nuh, ul, dup2(ky[r].x), dup2(ky[r].y));
+        if (kFullRows || (lane_on && dy < NS)) cell[dy * PX] = make_float4(s.x, s.y, e.x, e.y);
       }
       __syncwarp();  // this point's stores before the next point's loads
     }

@@ -1912,6 +1912,7 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
     if (a.bins.nsub == 0) return cudaSuccess;
     // 3D sparse subproblems: the slab-owned kernel unless a variant is forced
     bool slab = false, split = false, priv = false;
+    [[maybe_unused]] SlabDfShape slab_df{0, 0, 0};
     if constexpr (DIM == 2) {
       priv = a.variant == 0 && priv_spread_enabled();
       if (priv) {  // the private copies and stages must fit (else the atomic kernel)
@@ -1930,6 +1931,7 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (e != cudaSuccess) return e;
+        if (a.fp64_df) slab_df = slab_df_shape(NS, a.bins, (size_t)optin - 2048);  // less its static part
         slab = slab_bytes<T>(NS, a.bins) <= (size_t)optin;
       }
       // cell-run layout: the slab kernel also takes the sparse tails of the
@@ -1951,11 +1953,10 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
       }
     }
     if constexpr (sizeof(T) == 8 && DIM == 3) {
-      if (a.fp64_df && slab) {
-        const size_t smb = slab_df_bytes(NS, a.bins);
-        cudaError_t e = prepare_smem(k_spread_sm_slab_df<NS>, smb);
+      if (slab_df.bytes) {
+        cudaError_t e = prepare_smem(k_spread_sm_slab_df<NS>, slab_df.bytes);
         if (e != cudaSuccess) return e;
-        k_spread_sm_slab_df<NS><<<dim3(a.bins.nsub, a.ntr), 32 * NS, smb, s>>>(a);
+        k_spread_sm_slab_df<NS><<<dim3(a.bins.nsub, a.ntr), 64 * NS, slab_df.bytes, s>>>(a, slab_df.pitch, slab_df.nbuf);
         return cudaGetLastError();
       }
     }
