@@ -767,6 +767,124 @@ k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, i
 }
 
 // ---------------------------------------------------------------------------
+// 1D interpolation of FP64 plans in double-float: one thread per point.  In 1D
+// a point has only ns taps, so the kernel row (FP64 sqrt and exp per value,
+// ~20 clocks of an SM's FP64 unit each) was nearly all of the time; in
+// double-float the row is a few hundred FP32 instructions.  The point's cells
+// are split with the power of two of the largest of them, so any grid
+// magnitude passes.  3e6 points, 200001 modes, ns 12: execute 4.09 ->
+// 0.35 ms (the FFT is most of what is left).
+template <int NS>
+__global__ void __launch_bounds__(kSpreadThreads)
+k_interp_gm1_df(SpreadArgs<double> a) {
+  __shared__ float2 s_tab[64];
+  if (!a.kc.horner) {
+    df_table_fill(s_tab, a.kc);
+    __syncthreads();
+  }
+  const int nf0 = a.g.nf[0];
+  const int escale = df_scale_exp(a.kc.beta);
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.M; p += gridDim.x * blockDim.x) {
+    const int i1 = a.pts.i0[0][p];
+    const int dst = a.pts.idx[p];
+    float kh[NS], kl[NS];
+    df_kernel_row<NS>(a.pts.d[0][p], a.kc, s_tab, kh, kl);
+    for (int t = 0; t < a.ntr; ++t) {
+      const double2* base = a.fw_in + (size_t)t * a.g.Nf;
+      double2 g[NS];
+      unsigned m = 0;
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        g[j] = __ldg(base + wrap_idx(i1 + j, nf0));
+        const unsigned x = (unsigned)__double2hiint(g[j].x) & 0x7fffffffu;
+        const unsigned y = (unsigned)__double2hiint(g[j].y) & 0x7fffffffu;
+        if (x < 0x7ff00000u) m = max(m, x);
+        if (y < 0x7ff00000u) m = max(m, y);
+      }
+      const int shift = 1023 - (int)(m >> 20);
+      float2 s = make_float2(0.f, 0.f), e = s;
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        const DF re = df_split(g[j].x, shift), im = df_split(g[j].y, shift);
+        df2_acc(s, e, make_float2(re.h, im.h), make_float2(re.l, im.l), dup2(kh[j]), dup2(kl[j]));
+      }
+      const double oscale = ldexp(1.0, escale - shift);
+      double2 o;
+      o.x = ((double)s.x + (double)e.x) * oscale;
+      o.y = ((double)s.y + (double)e.y) * oscale;
+      a.c_out[(size_t)t * a.M + dst] = o;
+    }
+  }
+}
+
+// The same with eight lanes to a point, one per mirrored tap pair, for calls
+// whose points do not fill the chip with one thread each (kGm1WideMax): a row
+// is then one pair's latency instead of ns / 2 of them.  Stage time against
+// FP64 lanes over taps at ns 10: 2003 points 9.8 -> 8.4 us, 10000 points 22 ->
+// 9.6 us; at 38000 it takes 16.8 us where one thread per point takes 15.4 for
+// 60000, so the line lies at half a wave of threads.
+constexpr int kGm1WideLanes = 8;
+constexpr int kGm1WideMax = 152 * 1024 / kGm1WideLanes;
+constexpr int kGm1WideThreads = 64;
+template <int NS>
+__global__ void __launch_bounds__(kGm1WideThreads)
+k_interp_gm1_df_wide(SpreadArgs<double> a) {
+  constexpr int NP = (NS + 1) / 2;
+  __shared__ float2 s_tab[64];
+  if (!a.kc.horner) {
+    df_table_fill(s_tab, a.kc);
+    __syncthreads();
+  }
+  const int lane = threadIdx.x % kGm1WideLanes;
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) / kGm1WideLanes;
+  const int p = min(q, a.M - 1);  // whole warps run the reductions
+  const int j0 = min(lane, NP - 1), j1 = NS - 1 - j0;
+  const bool on0 = lane < NP, on1 = on0 && j1 != j0;
+  const int i1 = a.pts.i0[0][p];
+  const int x0 = wrap_idx(i1 + j0, a.g.nf[0]), x1 = wrap_idx(i1 + j1, a.g.nf[0]);
+  const int dst = a.pts.idx[p];
+  const DF2 k = df_kernel_pair<NS>(a.pts.d[0][p], j0, a.kc, s_tab);
+  const int escale = df_scale_exp(a.kc.beta);
+  for (int t = 0; t < a.ntr; ++t) {
+    const double2* base = a.fw_in + (size_t)t * a.g.Nf;
+    double2 g0 = __ldg(base + x0), g1 = __ldg(base + x1);
+    if (!on0) g0 = make_double2(0.0, 0.0);
+    if (!on1) g1 = make_double2(0.0, 0.0);
+    unsigned m = 0;
+    const unsigned h[4] = {(unsigned)__double2hiint(g0.x) & 0x7fffffffu, (unsigned)__double2hiint(g0.y) & 0x7fffffffu,
+                           (unsigned)__double2hiint(g1.x) & 0x7fffffffu, (unsigned)__double2hiint(g1.y) & 0x7fffffffu};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (h[i] < 0x7ff00000u) m = max(m, h[i]);
+#pragma unroll
+    for (int o = kGm1WideLanes / 2; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const int shift = 1023 - (int)(m >> 20);
+    float2 s = make_float2(0.f, 0.f), e = s;
+    DF re = df_split(g0.x, shift), im = df_split(g0.y, shift);
+    df2_acc(s, e, make_float2(re.h, im.h), make_float2(re.l, im.l), dup2(k.h.x), dup2(k.l.x));
+    re = df_split(g1.x, shift);
+    im = df_split(g1.y, shift);
+    df2_acc(s, e, make_float2(re.h, im.h), make_float2(re.l, im.l), dup2(k.h.y), dup2(k.l.y));
+#pragma unroll
+    for (int o = kGm1WideLanes / 2; o > 0; o >>= 1) {
+      DF2 v;
+      v.h = make_float2(__shfl_xor_sync(0xffffffffu, s.x, o), __shfl_xor_sync(0xffffffffu, s.y, o));
+      v.l = make_float2(__shfl_xor_sync(0xffffffffu, e.x, o), __shfl_xor_sync(0xffffffffu, e.y, o));
+      v = df2_add(DF2{s, e}, v);
+      s = v.h;
+      e = v.l;
+    }
+    if (lane == 0 && q < a.M) {
+      const double oscale = ldexp(1.0, escale - shift);
+      double2 o;
+      o.x = ((double)s.x + (double)e.x) * oscale;
+      o.y = ((double)s.y + (double)e.y) * oscale;
+      a.c_out[(size_t)t * a.M + dst] = o;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Warp-cooperative variants.  A warp works on PPW = 32 / L points at a time;
 // the L >= ns lanes of a point cover its x taps, so every warp-wide memory
 // instruction touches PPW contiguous runs of ns cells (one row of each
@@ -2025,6 +2143,16 @@ cudaError_t interp_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
   const bool wc = method == 1 ? a.variant != 1 : a.variant == 2;
   if (method == 1) {
+    if constexpr (sizeof(T) == 8 && DIM == 1) {
+      if (a.fp64_df && a.variant == 0) {
+        if (a.M <= kGm1WideMax)
+          k_interp_gm1_df_wide<NS><<<(a.M * kGm1WideLanes + kGm1WideThreads - 1) / kGm1WideThreads, kGm1WideThreads,
+                                     0, s>>>(a);
+        else
+          k_interp_gm1_df<NS><<<grid_for(a.M, kSpreadThreads), kSpreadThreads, 0, s>>>(a);
+        return cudaGetLastError();
+      }
+    }
     if (wc) {
       constexpr int PPW = 32 / lanes_per_point<NS>();
       k_interp_gm_wc<T, DIM, NS><<<grid_for(((long long)a.M + PPW - 1) / PPW * 32, kSpreadThreads),

@@ -29,6 +29,22 @@ def test_df_interp_against_fp64(monkeypatch, dim, modes, tol, scale, kmeth):
 
 
 @pytest.mark.parametrize("kmeth", [0, 1])
+@pytest.mark.parametrize("M,sort", [(1, 1), (255, 0), (3001, 1), (19456, 1), (19457, 1)])
+@pytest.mark.parametrize("tol,scale", [(9e-7, 1.0), (1e-7, 1e60), (1e-8, 1.0), (1e-10, 1e-250), (1e-12, 1.0),
+                                       (1e-13, 1.0)])
+def test_df_interp_1d(monkeypatch, M, sort, tol, scale, kmeth):
+    rng = np.random.default_rng(M)
+    pts = NC.points(rng, 1, M, lo=-3 * np.pi, hi=3 * np.pi, edges=False)
+    fk = NC.coeffs(rng, (501,), 3) * scale
+    kw = dict(gpu_kerevalmeth=kmeth, ntr=3, maxbatchsize=2, gpu_sort=sort)
+    monkeypatch.setenv("CUFINUFFT_FP64_DF", "0")
+    ref, _ = NC.run_gpu(2, (501,), pts, fk, tol, False, **kw)
+    monkeypatch.delenv("CUFINUFFT_FP64_DF")
+    out, _ = NC.run_gpu(2, (501,), pts, fk, tol, False, **kw)
+    assert np.linalg.norm(out / scale - ref / scale) / np.linalg.norm(ref / scale) < 1e-13
+
+
+@pytest.mark.parametrize("kmeth", [0, 1])
 @pytest.mark.parametrize("dim,modes,kw", [
     (2, (45, 38), dict(gpu_method=2)), (2, (64, 30), dict(gpu_method=3)),
     (2, (40, 40), dict(gpu_method=2, gpu_binsizex=7, gpu_binsizey=13, gpu_maxsubprobsize=33)),
