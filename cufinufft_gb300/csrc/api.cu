@@ -808,6 +808,11 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
     const char* v = std::getenv("CUFINUFFT_FP64_DF");
     p->fp64_df = v && v[0] == '0' ? 0 : (v && v[0] == '1' ? 1 : (tol >= 1e-13 ? 1 : 0));
     if (type == 1 && p->spread_only) p->fp64_df = 0;
+    // Below upsampfac 2 the deconvolution factors amplify the grid's rounding
+    // (1.25: ten thousandfold at ns 16, where it would show beside the
+    // kernel's error: 7.79e-10 -> 7.95e-10 in 2D type 1).  Type 1 keeps FP64
+    // there, type 2 the stricter form of the tile kernel (fp64_df 2).
+    if (p->fp64_df && p->opts.upsampfac < 2.0) p->fp64_df = type == 2 ? 2 : 0;
   }
   if constexpr (sizeof(T) == 8) {
     // double-float FFT of 2D power-of-two grids (types 1 and 2), under the

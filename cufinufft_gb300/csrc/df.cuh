@@ -100,21 +100,24 @@ __device__ __forceinline__ float bias_for(float b) {
 
 // v 2^shift as an FP32 pair, by integer operations on the exponent and
 // mantissa fields (a conversion, a subtraction and a second conversion would
-// each occupy the FP64 unit): h the top 24 bits, l the other 29 rounded to
-// 24.  Below 2^-126 (and for FP64 subnormals) the result is zero; infinities
-// and NaNs give NaN.
+// each occupy the FP64 unit): h the top 24 bits rounded to nearest, l the
+// signed rest of 29 bits rounded to 24.  Below 2^-126 (and for FP64 subnormals)
+// the result is zero; infinities and NaNs give NaN.
 __device__ __forceinline__ DF df_split(double v, int shift) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
   const int ef = (int)((hi >> 20) & 0x7ffu);
   const int e = ef - 896 + shift;  // FP32 exponent field of v 2^shift
   const unsigned sign = hi & 0x80000000u;
+  // exponent and mantissa of |v|, half a unit of h added: a carry may reach
+  // the exponent, as it should
+  const unsigned long long up = (b & 0x7fffffffffffffffull) + 0x10000000ull;
   DF r;
-  r.h = __uint_as_float(sign | ((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  r.h = __uint_as_float(sign | ((unsigned)(up >> 29) + ((unsigned)(shift - 896) << 23)));
   const float ls = __uint_as_float(sign | ((unsigned)(e > 52 ? e - 52 : 0) << 23));
-  r.l = __uint2float_rn(lo & 0x1fffffffu) * ls;
+  r.l = __int2float_rn((int)(lo << 3) >> 3) * ls;
   if (ef == 0 || e <= 0) r.h = r.l = 0.f;
-  if (ef == 0x7ff || e >= 255) r.h = __uint_as_float(0x7fc00000u);
+  if (ef == 0x7ff || e >= 254) r.h = __uint_as_float(0x7fc00000u);
   return r;
 }
 

@@ -126,7 +126,7 @@ template <typename T> struct SpreadArgs {
   // next call on the plan reads; null: not recorded.
   int* status;
   int tma_wait_test;        // nonzero: every tile's first wait gives up at once (tests)
-  int fp64_df;              // FP64: subproblem interpolation in double-float (k_interp_sm_df)
+  int fp64_df;              // FP64: double-float kernels (1), or only the tile interpolation, strictest form (2)
 };
 
 // Cells of one subproblem tile: the bin plus the ns-1 cells its points

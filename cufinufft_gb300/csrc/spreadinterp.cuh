@@ -679,13 +679,29 @@ k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, i
   __syncthreads();
   // kernel values carry 2^-E per axis, the tile 2^shift
   const double oscale = ldexp(1.0, DIM * df_scale_exp(a.kc.beta) - shift);
-  const float row_cut = 4.f * NS * NS / (2.8853901f * (float)a.kc.beta);  // squared distance of weight 2^-4
+  // squared distance of weight 2^-4; below upsampfac 2 (see makeplan) no tap is
+  // biased and the exp form's values come from FP64
+  const bool strict = a.fp64_df == 2;
+  const float row_cut = 4.f * NS * NS / (2.8853901f * (float)a.kc.beta);
   const int p_end = st.p0 + st.np;
   for (int p = st.p0 + threadIdx.x; p < p_end; p += blockDim.x) {
     int lc[3] = {0, 0, 0};
     float kh[DIM][NS], kl[DIM][NS];
 #pragma unroll 1
-    for (int ax = 0; ax < DIM; ++ax) df_kernel_row<NS>(a.pts.d[ax][p], a.kc, s_tab, kh[ax], kl[ax]);
+    for (int ax = 0; ax < DIM; ++ax) {
+      const double d = a.pts.d[ax][p];
+      if (strict && !a.kc.horner) {  // the exp form on the FP64 unit
+#pragma unroll 1
+        for (int j = 0; j < NS; ++j) {
+          const double x = d - 0.5 * NS + j;
+          const DF v = df_from(ldexp(es_value(a.kc.c * x * x, a.kc.beta), -df_scale_exp(a.kc.beta)));
+          kh[ax][j] = v.h;
+          kl[ax][j] = v.l;
+        }
+      } else {
+        df_kernel_row<NS>(d, a.kc, s_tab, kh[ax], kl[ax]);
+      }
+    }
     lc[0] = a.pts.i0[0][p] - st.ox;
     if (DIM > 1) lc[1] = a.pts.i0[1][p] - st.oy;
     if (DIM > 2) lc[2] = a.pts.i0[2][p] - st.oz;
@@ -715,7 +731,14 @@ k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, i
       for (int dy = 0; dy < NY; ++dy, row += st.TX) {
         const float x = fmaxf(fabsf(dy + 0.5f - 0.5f * NS) - 0.5f, 0.f);
         float2 s, e = zero, u = zero;
-        if (DIM == 1 || x * x < cut) {
+        if (strict) {
+          s = zero;
+#pragma unroll
+          for (int j = 0; j < NS; ++j) {
+            const float4 g = row[j];
+            df2_acc(s, e, make_float2(g.x, g.y), make_float2(g.z, g.w), dup2(kx[j]), dup2(kxl[j]));
+          }
+        } else if (DIM == 1 || x * x < cut) {
           if (NO > 0) {
             s = bias_out;
 #pragma unroll
@@ -746,14 +769,18 @@ k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, i
           e = add2(e, u);
         }
         if (DIM > 1) {
-          df2_acc(ps, pt, s, e, dup2(kh[DIM > 1 ? 1 : 0][dy]), dup2(kl[DIM > 1 ? 1 : 0][dy]));
+          // normalised first: low parts of several ulps would round the
+          // product's own low part at 2^-45
+          const DF2 r = fast_two_sum2(s, e);
+          df2_acc(ps, pt, r.h, r.l, dup2(kh[DIM > 1 ? 1 : 0][dy]), dup2(kl[DIM > 1 ? 1 : 0][dy]));
         } else {
           ps = s;
           pt = e;
         }
       }
       if (DIM > 2) {
-        df2_acc(ts, tt, ps, pt, dup2(kh[DIM - 1][dz]), dup2(kl[DIM - 1][dz]));
+        const DF2 r = fast_two_sum2(ps, pt);
+        df2_acc(ts, tt, r.h, r.l, dup2(kh[DIM - 1][dz]), dup2(kl[DIM - 1][dz]));
       } else {
         ts = ps;
         tt = pt;
@@ -2144,7 +2171,7 @@ cudaError_t interp_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
   const bool wc = method == 1 ? a.variant != 1 : a.variant == 2;
   if (method == 1) {
     if constexpr (sizeof(T) == 8 && DIM == 1) {
-      if (a.fp64_df && a.variant == 0) {
+      if (a.fp64_df == 1 && a.variant == 0) {
         if (a.M <= kGm1WideMax)
           k_interp_gm1_df_wide<NS><<<(a.M * kGm1WideLanes + kGm1WideThreads - 1) / kGm1WideThreads, kGm1WideThreads,
                                      0, s>>>(a);
