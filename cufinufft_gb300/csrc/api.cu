@@ -126,15 +126,6 @@ template <typename T> static void release(Plan<T>* p) {
   p->t3_pre = p->t3_post = p->t3_c = p->t3_grid = nullptr;
   p->t3_part = nullptr;
   p->t3_capM = p->t3_capN = p->t3_capG = 0;
-  cudaFree(p->n_idx);
-  p->n_idx = nullptr;
-  for (int k = 0; k < 3; ++k) {
-    cudaFree(p->n_i0[k]);
-    cudaFree(p->n_d[k]);
-    p->n_i0[k] = nullptr;
-    p->n_d[k] = nullptr;
-  }
-  p->n_cap = 0;
   cudaFree(p->c32);
   p->c32 = nullptr;
   p->c32_cap = 0;
@@ -165,19 +156,24 @@ template <typename T> static void release(Plan<T>* p) {
     p->df_tw[k] = nullptr;
   }
   p->horner.clear();
-  cudaFree(p->sel_buf);
-  p->sel_buf = nullptr;
+  cudaFree(p->feat);
+  p->feat = nullptr;
+  p->cap_feat = 0;
   cudaFree(p->horner_d);
   p->horner_d = nullptr;
   free_points(p);
   cudaFree(p->count);
   cudaFree(p->start);
   cudaFree(p->sub_start);
-  cudaFree(p->scan_tmp);
+  cudaFree(p->scan_part);
+  p->scan_part = nullptr;
+  cudaFree(p->raw);
+  p->raw = nullptr;
+  p->cap_bins = p->cap_raw = 0;
   cudaFree(p->sub_to_bin);
   cudaFree(p->sub_hdr);
   p->sub_hdr = nullptr;
-  p->count = p->start = p->sub_start = p->scan_tmp = p->sub_to_bin = nullptr;
+  p->count = p->start = p->sub_start = p->sub_to_bin = nullptr;
   p->cap_sub = 0;
   cudaFree(p->cls_count);
   p->cls_count = nullptr;
@@ -196,6 +192,8 @@ template <typename T> static void release(Plan<T>* p) {
   p->cap_sub_dense = 0;
   if (p->h_total) cudaFreeHost(p->h_total);
   p->h_total = nullptr;
+  if (p->ev_total) cudaEventDestroy(p->ev_total);
+  p->ev_total = nullptr;
   if (p->h_status) cudaFreeHost(p->h_status);
   p->h_status = nullptr;
   p->d_status = nullptr;
@@ -692,6 +690,34 @@ static int set_width_rule(int rule, int* previous) {
   return 0;
 }
 
+// Bin tables for nbins bins, kept while they are large enough.
+template <typename T>
+static int alloc_bins(Plan<T>* p, int nbins) {
+  if ((size_t)nbins > p->cap_bins) {
+    cudaFree(p->count);
+    cudaFree(p->start);
+    cudaFree(p->sub_start);
+    cudaFree(p->scan_part);
+    p->count = p->start = p->sub_start = nullptr;
+    p->scan_part = nullptr;
+    p->cap_bins = 0;
+    CFG_CUDA(cudaMalloc(&p->count, sizeof(int) * (size_t)nbins));
+    CFG_CUDA(cudaMalloc(&p->start, sizeof(int) * ((size_t)nbins + 1)));
+    CFG_CUDA(cudaMalloc(&p->sub_start, sizeof(int) * ((size_t)nbins + 1)));
+    CFG_CUDA(cudaMalloc(&p->scan_part, sizeof(unsigned long long) * (size_t)bin_scan_partials(nbins)));
+    p->cap_bins = nbins;
+  }
+  const size_t raw = nbins <= kCountStrideBins ? (size_t)nbins * kCountStride : 0;
+  if (raw > p->cap_raw) {
+    cudaFree(p->raw);
+    p->raw = nullptr;
+    p->cap_raw = 0;
+    CFG_CUDA(cudaMalloc(&p->raw, sizeof(int) * raw));
+    p->cap_raw = raw;
+  }
+  return 0;
+}
+
 // sp_fixed: the kernel (width and shape) chosen by an FP64 plan for its FP32
 // chain, instead of this precision's rule.
 template <typename T>
@@ -793,6 +819,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   CFG_CUDA(cudaStreamCreate(&p->own));  // blocking: ordered after the legacy default stream
   p->stream = p->own;
   CFG_CUDA(cudaMallocHost(&p->h_total, sizeof(int)));
+  CFG_CUDA(cudaEventCreateWithFlags(&p->ev_total, cudaEventDisableTiming));
   if (type == 2) {
     CFG_CUDA(cudaHostAlloc(&p->h_status, 2 * sizeof(int), cudaHostAllocMapped));
     p->h_status[0] = p->h_status[1] = 0;
@@ -824,10 +851,8 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   }
 
   const long long Nf = grid_cells(p);
-  CFG_CUDA(cudaMalloc(&p->count, sizeof(int) * (size_t)p->nbins));
-  CFG_CUDA(cudaMalloc(&p->start, sizeof(int) * ((size_t)p->nbins + 1)));
-  CFG_CUDA(cudaMalloc(&p->sub_start, sizeof(int) * ((size_t)p->nbins + 1)));
-  CFG_CUDA(cudaMalloc(&p->scan_tmp, sizeof(int) * (size_t)scan_tmp_ints(p->nbins)));
+  int e = alloc_bins(p, p->nbins);
+  if (e) return e;
   if (p->spread_only) {
     // no grid, FFT or kernel Fourier series: execute spreads into / reads
     // from the caller's fk
@@ -847,7 +872,6 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   CFG_CUDA(cudaMalloc(&p->fw, sizeof(cplx_t<T>) * (size_t)Nf * p->maxbatch));
   for (int k = 0; k < dim; ++k) CFG_CUDA(cudaMalloc(&p->fac[k], sizeof(T) * (size_t)p->N[k]));
 
-  int e = 0;
   if (use_df_fft(p)) {
     // double-float FFT: no cuFFT plan; scratch for the passes, twiddles per axis
     e = make_df_fft(p);
@@ -1022,12 +1046,176 @@ static int bank_order(Plan<T>* p, int method, const int bs[3], int nbins, BankOr
 }
 
 template <typename T>
-static int build_subproblems(Plan<T>* p);
+static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src);
 
 static int setpts_chain(Plan<double>* p, int M, const double* x, const double* y, const double* z);
 static int execute_chain(Plan<double>* p, double2* c, double2* fk);
 template <typename T>
 static int execute_t3(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk);
+
+template <typename T>
+int resolve_nsub(Plan<T>* p, bool wait) {
+  if (p->nsub_exact) return 0;
+  if (wait) {
+    CFG_CUDA(cudaEventSynchronize(p->ev_total));
+  } else {
+    const cudaError_t e = cudaEventQuery(p->ev_total);
+    if (e == cudaErrorNotReady) {
+      cudaGetLastError();
+      return 0;
+    }
+    CFG_CUDA(e);
+  }
+  p->nsub = *p->h_total;
+  p->nsub_exact = true;
+  return 0;
+}
+template int resolve_nsub<float>(Plan<float>*, bool);
+template int resolve_nsub<double>(Plan<double>*, bool);
+
+// The sort of setpts and set_layout on the plan stream, no readback waited for:
+// counters, ranks, starts, permutation, and for method 2 the subproblem
+// headers.  a: the point source and the sorted arrays to fill; the layout is
+// the plan's.
+template <typename T>
+static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
+  p->nsub = 0;
+  p->nsub_exact = true;
+  for (int k = 0; k < 3; ++k) {
+    a.bs[k] = p->bs[k];
+    a.nb[k] = p->nb[k];
+  }
+  a.dim = p->dim;
+  a.M = p->M;
+  a.count = p->count;
+  a.rank = p->rank;
+  a.start = p->start;
+  if (p->M == 0) return 0;
+  const int ms = p->method == 2 ? p->opts.gpu_maxsubprobsize : 0;
+  int e = bank_order(p, p->method, p->bs, p->nbins, &a.bank, p->cell_order);  // zeroes its counters
+  if (e) return e;
+  BinScanArgs sc;
+  std::memset(&sc, 0, sizeof(sc));
+  sc.raw = p->count;
+  sc.raw_stride = sc.per = 1;
+  if (a.bank.cls_count && !a.bank.cell_order) {
+    sc.raw = a.bank.cls_count;
+    sc.raw_stride = sc.per = a.bank.ncls;
+  } else if (!a.bank.cls_count && p->nbins <= kCountStrideBins) {
+    sc.raw = p->raw;
+    sc.raw_stride = kCountStride;
+  }
+  a.raw = const_cast<int*>(sc.raw);
+  a.raw_stride = sc.raw_stride;
+  if (!a.bank.cls_count || a.bank.cell_order)
+    CFG_CUDA(cudaMemsetAsync(a.raw, 0, sizeof(int) * (size_t)p->nbins * sc.raw_stride, p->stream));
+  sc.nbins = p->nbins;
+  sc.maxsub = ms;
+  sc.count = p->count;
+  sc.start = p->start;
+  sc.sub_start = p->sub_start;
+  sc.partial = p->scan_part;
+  CFG_CUDA(launch_bin_count<T>(a, p->stream));
+  CFG_CUDA(launch_bin_scan(sc, p->stream));
+  if (a.bank.cell_order)
+    CFG_CUDA(launch_scan(p->cls_count, p->cls_start, p->nbins * a.bank.ncls, 2, dense_run(p->dim), p->cls_tmp,
+                         p->stream));
+  SubHdrArgs h;
+  std::memset(&h, 0, sizeof(h));
+  if (ms > 0) {
+    // a bin of c > 0 points holds at most 1 + (c - 1) / ms subproblems
+    const int bound = (int)std::min<long long>((long long)std::min(p->nbins, p->M) + p->M / ms, 0x7fffffffLL);
+    if ((size_t)bound > p->cap_sub) {
+      cudaFree(p->sub_to_bin);
+      cudaFree(p->sub_hdr);
+      p->sub_to_bin = nullptr;
+      p->sub_hdr = nullptr;
+      p->cap_sub = 0;
+      CFG_CUDA(cudaMalloc(&p->sub_to_bin, sizeof(int) * (size_t)bound));
+      CFG_CUDA(cudaMalloc(&p->sub_hdr, sizeof(SubHdr) * (size_t)bound));
+      p->cap_sub = bound;
+    }
+    h.sub_start = p->sub_start;
+    h.nbins = p->nbins;
+    h.nsub = bound;
+    h.maxsub = ms;
+    h.sub_to_bin = p->sub_to_bin;
+    h.hdr = p->sub_hdr;
+  }
+  CFG_CUDA(launch_permute<T>(a, h, p->stream));
+  if (ms == 0) return 0;
+  if (p->cell_order) {
+    if ((size_t)h.nsub > p->cap_sub_dense) {
+      cudaFree(p->sub_dense);
+      cudaFree(p->sub_ndense);
+      p->sub_dense = nullptr;
+      p->sub_ndense = nullptr;
+      p->cap_sub_dense = 0;
+      CFG_CUDA(cudaMalloc(&p->sub_dense, (size_t)h.nsub));
+      CFG_CUDA(cudaMalloc(&p->sub_ndense, sizeof(int) * (size_t)h.nsub));
+      p->cap_sub_dense = h.nsub;
+    }
+    SubClassArgs c;
+    std::memset(&c, 0, sizeof(c));
+    c.sub_to_bin = p->sub_to_bin;
+    c.sub_start = p->sub_start;
+    c.sub_total = p->sub_start + p->nbins;
+    c.start = p->start;
+    c.cls_count = p->cls_count;
+    for (int k = 0; k < 3; ++k) {
+      c.i0[k] = a.i0[k];
+      c.bs[k] = p->bs[k];
+    }
+    c.dim = p->dim;
+    c.maxsub = ms;
+    c.ncls = a.bank.ncls;
+    c.nsub = h.nsub;
+    c.dense_min = dense_run(p->dim);
+    c.dense = p->sub_dense;
+    c.cls_start = p->cls_start;
+    c.count = p->count;
+    c.ndense = p->sub_ndense;
+    CFG_CUDA(launch_classify_subproblems(c, p->stream));
+  }
+  p->nsub = h.nsub;
+  p->nsub_exact = false;
+  CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + p->nbins, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+  CFG_CUDA(cudaEventRecord(p->ev_total, p->stream));
+  return 0;
+}
+
+// The part of setpts that FP32, FP64 and chained plans share: `a` says where
+// the points come from (their source, coordinates and axis maps).
+template <typename T>
+static int setpts_from(Plan<T>* p, int M, PlaceArgs<T> a) {
+  p->pts_set = false;
+  ++p->version;  // point arrays may be reallocated below
+  int e = ensure_points(p, M);
+  if (e) return e;
+  p->M = M;
+  p->nsub = 0;
+  p->nsub_exact = true;
+  a.dim = p->dim;
+  a.M = M;
+  e = choose_layout(p, a);  // gpu_method 0: before the sort, from the points' occupancy
+  if (e) return e;
+  a.idx = p->idx;
+  for (int k = 0; k < 3; ++k) {
+    a.i0[k] = p->i0[k];
+    a.d[k] = p->d[k];
+    a.bs[k] = p->bs[k];
+    a.nb[k] = p->nb[k];
+  }
+  if (p->method == 1 && p->sort == 0) {
+    CFG_CUDA(launch_place_unsorted<T>(a, p->stream));
+  } else {
+    e = sort_points(p, a);
+    if (e) return e;
+  }
+  CFG_CUDA(cudaGetLastError());
+  p->pts_set = true;
+  return 0;
+}
 
 template <typename T>
 static int setpts_impl(Plan<T>* p, int M, const T* x, const T* y, const T* z) {
@@ -1039,48 +1227,14 @@ static int setpts_impl(Plan<T>* p, int M, const T* x, const T* y, const T* z) {
   const T* xs[3] = {x, y, z};
   for (int k = 0; k < p->dim; ++k)
     if (M > 0 && xs[k] == nullptr) return CUFINUFFT_ERR_ARG;
-  p->pts_set = false;
-  ++p->version;  // point arrays may be reallocated below
-  int e = ensure_points(p, M);
-  if (e) return e;
-  p->M = M;
-  p->nsub = 0;
   PlaceArgs<T> a;
   std::memset(&a, 0, sizeof(a));
+  a.src = kSrcCoords;
   for (int k = 0; k < 3; ++k) {
     a.x[k] = k < p->dim ? xs[k] : nullptr;
     a.ax[k] = axis_map<T>(p->nf[k], p->sp.ns);
-    a.bs[k] = p->bs[k];
-    a.nb[k] = p->nb[k];
-    a.i0[k] = p->i0[k];
-    a.d[k] = p->d[k];
   }
-  a.dim = p->dim;
-  a.M = M;
-  a.idx = p->idx;
-  a.count = p->count;
-  a.rank = p->rank;
-  a.start = p->start;
-  if (p->method == 1 && p->sort == 0) {
-    CFG_CUDA(launch_place_unsorted<T>(a, p->stream));
-  } else {
-    CFG_CUDA(cudaMemsetAsync(p->count, 0, sizeof(int) * (size_t)p->nbins, p->stream));
-    e = bank_order(p, p->method, p->bs, p->nbins, &a.bank, p->cell_order);
-    if (e) return e;
-    CFG_CUDA(launch_bin_count<T>(a, p->stream));
-    CFG_CUDA(launch_scan(p->count, p->start, p->nbins, 0, 1, p->scan_tmp, p->stream));
-    if (a.bank.cell_order)
-      CFG_CUDA(launch_scan(p->cls_count, p->cls_start, p->nbins * a.bank.ncls, 2, dense_run(p->dim), p->cls_tmp,
-                           p->stream));
-    CFG_CUDA(launch_permute<T>(a, p->stream));
-    if (p->method == 2) {
-      e = build_subproblems(p);
-      if (e) return e;
-    }
-  }
-  CFG_CUDA(cudaGetLastError());
-  p->pts_set = true;
-  return select_layout(p);
+  return setpts_from(p, M, a);
 }
 
 static int max_smem_optin(int device) {
@@ -1254,9 +1408,9 @@ static bool graphs_enabled() {
   return !(v && v[0] == '0');
 }
 
-// execute: with stage timing off, the launch sequence is captured once as a
-// CUDA graph (for these caller arrays and this plan state) and replayed, which
-// removes most of the gaps between its kernels.  A plan stream that is already
+// execute: with stage timing off, a call that repeats the last one (same
+// caller arrays and plan state) captures the launch sequence as a CUDA graph,
+// and later ones replay it, which removes most of the gaps between its kernels.  A plan stream that is already
 // being captured (a batch recording this plan), or a capture that fails, runs
 // the kernels directly.
 // A tile wait of an earlier execute ran out (SpreadArgs::status): its result
@@ -1291,19 +1445,30 @@ static int execute_impl(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
     CFG_CUDA(cudaGraphLaunch(p->gexec, p->stream));
     return 0;
   }
-  drop_graph(p);
+  // capture pays from the second call on: it costs more than the direct
+  // launches it saves (new points or arrays on every call would capture every
+  // time: 2D 256^2, 1e5 points, setpts and execute 130 us, of which 75 us of
+  // host time in capture, instantiation and destruction)
+  const bool again = p->last_c == c && p->last_fk == fk && p->last_version == p->version;
+  p->last_c = c;
+  p->last_fk = fk;
+  p->last_version = p->version;
+  if (const int e = resolve_nsub(p, false)) return e;
+  if (!again || !p->nsub_exact) return execute_direct(p, c, fk);
   if (cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
     const int e = execute_direct(p, c, fk);
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(p->stream, &g);
-    if (e == 0 && ce == cudaSuccess && g != nullptr &&
-        cudaGraphInstantiate(&p->gexec, g, 0) == cudaSuccess) {
-      p->graph = g;
-      p->g_c = c;
-      p->g_fk = fk;
-      p->g_version = p->version;
-      CFG_CUDA(cudaGraphLaunch(p->gexec, p->stream));
-      return 0;
+    if (e == 0 && ce == cudaSuccess && g != nullptr) {
+      drop_graph(p);
+      if (cudaGraphInstantiate(&p->gexec, g, 0) == cudaSuccess) {
+        p->graph = g;
+        p->g_c = c;
+        p->g_fk = fk;
+        p->g_version = p->version;
+        CFG_CUDA(cudaGraphLaunch(p->gexec, p->stream));
+        return 0;
+      }
     }
     if (g) cudaGraphDestroy(g);
     p->gexec = nullptr;
@@ -1395,62 +1560,6 @@ static int makeplan_chain(Plan<double>* p, int type, int dim, const int* nmodes,
   return 0;
 }
 
-// Sort of points already placed (first taps and FP32 offsets in caller
-// order): the counting sort of setpts, fed from stored arrays instead of
-// coordinates (the rebin kernels).
-static int setpts_placed(Plan<float>* q, int M, const int* s_idx, int* const s_i0[3], float* const s_d[3]) {
-  if (!q->planned) return CUFINUFFT_ERR_GENERIC;
-  q->pts_set = false;
-  ++q->version;
-  int e = ensure_points(q, M);
-  if (e) return e;
-  q->M = M;
-  q->nsub = 0;
-  if (M > 0 && q->method == 1 && q->sort == 0) {
-    CFG_CUDA(cudaMemcpyAsync(q->idx, s_idx, sizeof(int) * (size_t)M, cudaMemcpyDeviceToDevice, q->stream));
-    for (int k = 0; k < q->dim; ++k) {
-      CFG_CUDA(cudaMemcpyAsync(q->i0[k], s_i0[k], sizeof(int) * (size_t)M, cudaMemcpyDeviceToDevice,
-                               q->stream));
-      CFG_CUDA(cudaMemcpyAsync(q->d[k], s_d[k], sizeof(float) * (size_t)M, cudaMemcpyDeviceToDevice,
-                               q->stream));
-    }
-  } else if (!(q->method == 1 && q->sort == 0)) {
-    RebinArgs<float> a;
-    std::memset(&a, 0, sizeof(a));
-    a.dim = q->dim;
-    a.M = M;
-    for (int k = 0; k < 3; ++k) {
-      a.bs[k] = q->bs[k];
-      a.nb[k] = q->nb[k];
-      a.src_i0[k] = k < q->dim ? s_i0[k] : nullptr;
-      a.src_d[k] = k < q->dim ? s_d[k] : nullptr;
-      a.i0[k] = q->i0[k];
-      a.d[k] = q->d[k];
-    }
-    a.src_idx = s_idx;
-    a.idx = q->idx;
-    a.count = q->count;
-    a.rank = q->rank;
-    a.start = q->start;
-    CFG_CUDA(cudaMemsetAsync(q->count, 0, sizeof(int) * (size_t)q->nbins, q->stream));
-    e = bank_order(q, q->method, q->bs, q->nbins, &a.bank, q->cell_order);
-    if (e) return e;
-    CFG_CUDA(launch_rebin_count<float>(a, q->stream));
-    CFG_CUDA(launch_scan(q->count, q->start, q->nbins, 0, 1, q->scan_tmp, q->stream));
-    if (a.bank.cell_order)
-      CFG_CUDA(launch_scan(q->cls_count, q->cls_start, q->nbins * a.bank.ncls, 2, dense_run(q->dim),
-                           q->cls_tmp, q->stream));
-    CFG_CUDA(launch_rebin_permute<float>(a, q->stream));
-    if (q->method == 2) {
-      e = build_subproblems(q);
-      if (e) return e;
-    }
-  }
-  CFG_CUDA(cudaGetLastError());
-  q->pts_set = true;
-  return select_layout(q);
-}
-
 static int setpts_chain(Plan<double>* p, int M, const double* x, const double* y, const double* z) {
   Plan<float>* q = p->lo;
   if (!q->planned) return CUFINUFFT_ERR_GENERIC;
@@ -1460,41 +1569,22 @@ static int setpts_chain(Plan<double>* p, int M, const double* x, const double* y
     if (M > 0 && xs[k] == nullptr) return CUFINUFFT_ERR_ARG;
   ++p->version;
   p->pts_set = q->pts_set = false;
-  if ((size_t)M > p->n_cap || p->n_idx == nullptr) {
-    cudaFree(p->n_idx);
-    p->n_idx = nullptr;
-    for (int k = 0; k < 3; ++k) {
-      cudaFree(p->n_i0[k]);
-      cudaFree(p->n_d[k]);
-      p->n_i0[k] = nullptr;
-      p->n_d[k] = nullptr;
-    }
+  const size_t nc = (size_t)std::max(M, 1) * (size_t)p->ntransf;
+  if (nc > p->c32_cap || p->c32 == nullptr) {
     cudaFree(p->c32);
     p->c32 = nullptr;
-    p->n_cap = p->c32_cap = 0;
-    const size_t n = (size_t)std::max(M, 1);
-    CFG_CUDA(cudaMalloc(&p->n_idx, sizeof(int) * n));
-    for (int k = 0; k < p->dim; ++k) {
-      CFG_CUDA(cudaMalloc(&p->n_i0[k], sizeof(int) * n));
-      CFG_CUDA(cudaMalloc(&p->n_d[k], sizeof(float) * n));
-    }
-    CFG_CUDA(cudaMalloc(&p->c32, sizeof(cplx_t<float>) * n * (size_t)p->ntransf));
-    p->n_cap = n;
-    p->c32_cap = n * (size_t)p->ntransf;
+    p->c32_cap = 0;
+    CFG_CUDA(cudaMalloc(&p->c32, sizeof(cplx_t<float>) * nc));
+    p->c32_cap = nc;
   }
-  NarrowPlaceArgs na;
-  std::memset(&na, 0, sizeof(na));
+  PlaceArgs<float> a;
+  std::memset(&a, 0, sizeof(a));
+  a.src = kSrcNarrow;
   for (int k = 0; k < 3; ++k) {
-    na.x[k] = k < p->dim ? xs[k] : nullptr;
-    na.ax[k] = axis_map<double>(q->nf[k], q->sp.ns);
-    na.i0[k] = p->n_i0[k];
-    na.d[k] = p->n_d[k];
+    a.xd[k] = k < p->dim ? xs[k] : nullptr;
+    a.axd[k] = axis_map<double>(q->nf[k], q->sp.ns);
   }
-  na.dim = p->dim;
-  na.M = M;
-  na.idx = p->n_idx;
-  CFG_CUDA(launch_place_narrow(na, q->stream));
-  const int e = setpts_placed(q, M, p->n_idx, p->n_i0, p->n_d);
+  const int e = setpts_from(q, M, a);
   sync_from_lo(p);
   return e;
 }
@@ -1771,7 +1861,8 @@ template int plan_use_stream<float>(Plan<float>*, cudaStream_t);
 template int plan_use_stream<double>(Plan<double>*, cudaStream_t);
 
 template <typename T>
-static void fill_info(const Plan<T>* p, cufinufft_plan_info* info) {
+static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
+  resolve_nsub(p, true);
   std::memset(info, 0, sizeof(*info));
   info->type = p->type;
   info->dim = p->dim;
@@ -1806,90 +1897,10 @@ static void fill_info(const Plan<T>* p, cufinufft_plan_info* info) {
 // ---------------------------------------------------------------------------
 // Layout changes and autotuning (extensions).
 
-// Reallocate the bin tables for nbins bins.
+// The plan's layout becomes this method / bin size / subproblem cap, for the
+// next sort; refusals leave the plan as it was.
 template <typename T>
-static int alloc_bins(Plan<T>* p, int nbins) {
-  cudaFree(p->count);
-  cudaFree(p->start);
-  cudaFree(p->sub_start);
-  cudaFree(p->scan_tmp);
-  p->count = p->start = p->sub_start = p->scan_tmp = nullptr;
-  CFG_CUDA(cudaMalloc(&p->count, sizeof(int) * (size_t)nbins));
-  CFG_CUDA(cudaMalloc(&p->start, sizeof(int) * ((size_t)nbins + 1)));
-  CFG_CUDA(cudaMalloc(&p->sub_start, sizeof(int) * ((size_t)nbins + 1)));
-  CFG_CUDA(cudaMalloc(&p->scan_tmp, sizeof(int) * (size_t)scan_tmp_ints(nbins)));
-  return 0;
-}
-
-// Subproblem tables of the current layout (method 2): one readback of the
-// total, as in setpts.
-template <typename T>
-static int build_subproblems(Plan<T>* p) {
-  p->nsub = 0;
-  if (p->M == 0) return 0;
-  const int ms = p->opts.gpu_maxsubprobsize;
-  CFG_CUDA(launch_scan(p->count, p->sub_start, p->nbins, 1, ms, p->scan_tmp, p->stream));
-  CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + p->nbins, sizeof(int), cudaMemcpyDeviceToHost,
-                           p->stream));
-  CFG_CUDA(cudaStreamSynchronize(p->stream));
-  const int nsub = *p->h_total;
-  if ((size_t)nsub > p->cap_sub) {
-    cudaFree(p->sub_to_bin);
-    cudaFree(p->sub_hdr);
-    p->sub_to_bin = nullptr;
-    p->sub_hdr = nullptr;
-    p->cap_sub = 0;
-    CFG_CUDA(cudaMalloc(&p->sub_to_bin, sizeof(int) * (size_t)nsub));
-    CFG_CUDA(cudaMalloc(&p->sub_hdr, sizeof(SubHdr) * (size_t)nsub));
-    p->cap_sub = nsub;
-  }
-  CFG_CUDA(launch_sub_headers(p->sub_start, p->start, p->count, p->nbins, nsub, ms, p->bs, p->nb,
-                              p->sub_to_bin, p->sub_hdr, p->stream));
-  p->nsub = nsub;
-  if (p->cell_order) {
-    if ((size_t)nsub > p->cap_sub_dense) {
-      cudaFree(p->sub_dense);
-      cudaFree(p->sub_ndense);
-      p->sub_dense = nullptr;
-      p->sub_ndense = nullptr;
-      p->cap_sub_dense = 0;
-      CFG_CUDA(cudaMalloc(&p->sub_dense, (size_t)nsub));
-      CFG_CUDA(cudaMalloc(&p->sub_ndense, sizeof(int) * (size_t)nsub));
-      p->cap_sub_dense = nsub;
-    }
-    SubClassArgs c;
-    std::memset(&c, 0, sizeof(c));
-    c.sub_to_bin = p->sub_to_bin;
-    c.sub_start = p->sub_start;
-    c.start = p->start;
-    c.cls_count = p->cls_count;
-    for (int k = 0; k < 3; ++k) {
-      c.i0[k] = p->i0[k];
-      c.bs[k] = p->bs[k];
-    }
-    c.dim = p->dim;
-    c.maxsub = ms;
-    c.ncls = 1;
-    for (int k = 0; k < p->dim; ++k) c.ncls *= p->bs[k];
-    c.nsub = nsub;
-    c.dense_min = dense_run(p->dim);
-    c.dense = p->sub_dense;
-    c.cls_start = p->cls_start;
-    c.count = p->count;
-    c.ndense = p->sub_ndense;
-    CFG_CUDA(launch_classify_subproblems(c, p->stream));
-  }
-  return 0;
-}
-
-// Switch a plan with points set to another method / bin size / subproblem
-// cap by re-sorting its stored points (the caller's coordinates are not
-// needed).  Results are unchanged; only the work schedule moves.
-template <typename T>
-static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub) {
-  if (!p->planned) return CUFINUFFT_ERR_GENERIC;
-  if (p->type == 3) return CUFINUFFT_ERR_METHOD;  // type 3 lays out its inner plans itself
-  ++p->version;  // the sorted arrays and bin tables are about to move
+static int adopt_layout(Plan<T>* p, int method, const int bsz[3], int maxsub) {
   // method 5: method 2 spreading over cell-ordered points (cell-run kernel)
   const bool cell = method == 5;
   if (cell) {
@@ -1918,54 +1929,8 @@ static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub)
     return CUFINUFFT_ERR_SHMEM;
   if (cell && !cell_order_fits(p, bs, nbins)) return CUFINUFFT_ERR_ARG;
   if (cell && run_smem_bytes(p, bs) > (size_t)max_smem_optin(p->device)) return CUFINUFFT_ERR_SHMEM;
-  int e = alloc_bins(p, (int)nbins);
+  const int e = alloc_bins(p, (int)nbins);
   if (e) return e;
-  if (p->pts_set && p->M > 0) {
-    // fresh arrays for the re-sorted points
-    int* idx = nullptr;
-    int* i0[3] = {nullptr, nullptr, nullptr};
-    T* d[3] = {nullptr, nullptr, nullptr};
-    CFG_CUDA(cudaMalloc(&idx, sizeof(int) * p->capM));
-    for (int k = 0; k < p->dim; ++k) {
-      CFG_CUDA(cudaMalloc(&i0[k], sizeof(int) * p->capM));
-      CFG_CUDA(cudaMalloc(&d[k], sizeof(T) * p->capM));
-    }
-    RebinArgs<T> a;
-    std::memset(&a, 0, sizeof(a));
-    a.dim = p->dim;
-    a.M = p->M;
-    for (int k = 0; k < 3; ++k) {
-      a.bs[k] = bs[k];
-      a.nb[k] = nb[k];
-      a.src_i0[k] = p->i0[k];
-      a.src_d[k] = p->d[k];
-      a.i0[k] = i0[k];
-      a.d[k] = d[k];
-    }
-    a.src_idx = p->idx;
-    a.idx = idx;
-    a.count = p->count;
-    a.rank = p->rank;
-    a.start = p->start;
-    e = bank_order(p, method, bs, (int)nbins, &a.bank, cell);
-    if (e) return e;
-    CFG_CUDA(cudaMemsetAsync(p->count, 0, sizeof(int) * (size_t)nbins, p->stream));
-    CFG_CUDA(launch_rebin_count<T>(a, p->stream));
-    CFG_CUDA(launch_scan(p->count, p->start, (int)nbins, 0, 1, p->scan_tmp, p->stream));
-    if (a.bank.cell_order)
-      CFG_CUDA(launch_scan(p->cls_count, p->cls_start, (int)nbins * a.bank.ncls, 2, dense_run(p->dim), p->cls_tmp,
-                           p->stream));
-    CFG_CUDA(launch_rebin_permute<T>(a, p->stream));
-    CFG_CUDA(cudaStreamSynchronize(p->stream));
-    cudaFree(p->idx);
-    p->idx = idx;
-    for (int k = 0; k < p->dim; ++k) {
-      cudaFree(p->i0[k]);
-      cudaFree(p->d[k]);
-      p->i0[k] = i0[k];
-      p->d[k] = d[k];
-    }
-  }
   p->method = method;
   p->cell_order = cell;
   p->sort = 1;
@@ -1981,17 +1946,53 @@ static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub)
   if (method == 2) p->opts.gpu_maxsubprobsize = maxsub;
   p->nbins = (int)nbins;
   p->nsub = 0;
-  if (method == 2 && p->pts_set) {
-    e = build_subproblems(p);
-    if (e) return e;
-  }
+  p->nsub_exact = true;
   return 0;
+}
+
+// Switch a plan with points set to another method / bin size / subproblem
+// cap by re-sorting its stored points (the caller's coordinates are not
+// needed).  Results are unchanged; only the work schedule moves.
+template <typename T>
+static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub) {
+  if (!p->planned) return CUFINUFFT_ERR_GENERIC;
+  if (p->type == 3) return CUFINUFFT_ERR_METHOD;  // type 3 lays out its inner plans itself
+  ++p->version;  // the sorted arrays and bin tables are about to move
+  int e = adopt_layout(p, method, bsz, maxsub);
+  if (e) return e;
+  if (!p->pts_set || p->M == 0) return 0;
+  // fresh arrays for the re-sorted points
+  PlaceArgs<T> a;
+  std::memset(&a, 0, sizeof(a));
+  a.src = kSrcStored;
+  a.src_idx = p->idx;
+  CFG_CUDA(cudaMalloc(&a.idx, sizeof(int) * p->capM));
+  for (int k = 0; k < p->dim; ++k) {
+    a.src_i0[k] = p->i0[k];
+    a.src_d[k] = p->d[k];
+    CFG_CUDA(cudaMalloc(&a.i0[k], sizeof(int) * p->capM));
+    CFG_CUDA(cudaMalloc(&a.d[k], sizeof(T) * p->capM));
+  }
+  e = sort_points(p, a);
+  if (e) return e;
+  CFG_CUDA(cudaStreamSynchronize(p->stream));
+  cudaFree(p->idx);
+  p->idx = a.idx;
+  for (int k = 0; k < p->dim; ++k) {
+    cudaFree(p->i0[k]);
+    cudaFree(p->d[k]);
+    p->i0[k] = a.i0[k];
+    p->d[k] = a.d[k];
+  }
+  return resolve_nsub(p, true);
 }
 
 // Device time (ms) of the plan's spread (type 1) or interp (type 2) stage for
 // one batch, median of `reps` runs after one warm-up, on synthetic values.
 template <typename T>
 static int time_stage(Plan<T>* p, cplx_t<T>* scratch, cplx_t<T>* grid, int reps, float* ms) {
+  CFG_CUDA(cudaStreamSynchronize(p->stream));
+  if (const int er = resolve_nsub(p, true)) return er;
   SpreadArgs<T> a = spread_args(p);
   a.ntr = p->maxbatch;
   cudaEvent_t e0, e1;
@@ -2141,30 +2142,31 @@ static int autotune_impl(Plan<T>* p, cufinufft_tune_entry* out, int max_out, int
 // ---------------------------------------------------------------------------
 // Features and the learned selector.
 
+// src: the points (their count in p->M), stored or not.
 template <typename T>
-static int features_impl(Plan<T>* p, float* f) {
-  if (p->type == 3) return CUFINUFFT_ERR_METHOD;
-  if (!p->planned || !p->pts_set) return CUFINUFFT_ERR_GENERIC;
-  int fb[3] = {1, 1, 1}, nb[3] = {1, 1, 1};
+static int features_of(Plan<T>* p, PlaceArgs<T> src, float* f) {
   long long nbins = 1;
-  for (int k = 0; k < p->dim; ++k) {
-    fb[k] = std::min(p->dim == 1 ? 64 : (p->dim == 2 ? 16 : 8), p->nf[k]);
-    nb[k] = (p->nf[k] + fb[k] - 1) / fb[k];
-    nbins *= nb[k];
+  for (int k = 0; k < 3; ++k) {
+    src.bs[k] = k < p->dim ? std::min(p->dim == 1 ? 64 : (p->dim == 2 ? 16 : 8), p->nf[k]) : 1;
+    src.nb[k] = k < p->dim ? (p->nf[k] + src.bs[k] - 1) / src.bs[k] : 1;
+    nbins *= src.nb[k];
   }
   std::vector<int> h((size_t)nbins, 0);
   if (p->M > 0) {
-    int* counts = nullptr;
-    CFG_CUDA(cudaMalloc(&counts, sizeof(int) * (size_t)nbins));
-    CFG_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nbins, p->stream));
-    const int* i0[3] = {p->i0[0], p->i0[1], p->i0[2]};
-    cudaError_t e = launch_feature_count(p->dim, p->M, i0, fb, nb, counts, p->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h.data(), counts, sizeof(int) * (size_t)nbins, cudaMemcpyDeviceToHost,
-                          p->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
-    cudaFree(counts);
-    CFG_CUDA(e);
+    if ((size_t)nbins > p->cap_feat) {
+      cudaFree(p->feat);
+      p->feat = nullptr;
+      p->cap_feat = 0;
+      CFG_CUDA(cudaMalloc(&p->feat, sizeof(int) * (size_t)nbins));
+      p->cap_feat = nbins;
+    }
+    CFG_CUDA(cudaMemsetAsync(p->feat, 0, sizeof(int) * (size_t)nbins, p->stream));
+    src.dim = p->dim;
+    src.M = p->M;
+    src.count = p->feat;
+    CFG_CUDA(launch_feature_count<T>(src, p->stream));
+    CFG_CUDA(cudaMemcpyAsync(h.data(), p->feat, sizeof(int) * (size_t)nbins, cudaMemcpyDeviceToHost, p->stream));
+    CFG_CUDA(cudaStreamSynchronize(p->stream));
   }
   double sum = 0, sumsq = 0, mx = 0, occ = 0, sq_occ = 0;
   for (int c : h) {
@@ -2198,42 +2200,62 @@ static int features_impl(Plan<T>* p, float* f) {
   return 0;
 }
 
+// Features of the points that are set.
 template <typename T>
-static int apply_layout_class(Plan<T>* p, int cls);
+static int features_impl(Plan<T>* p, float* f) {
+  if (p->type == 3) return CUFINUFFT_ERR_METHOD;
+  if (!p->planned || !p->pts_set) return CUFINUFFT_ERR_GENERIC;
+  PlaceArgs<T> a;
+  std::memset(&a, 0, sizeof(a));
+  a.src = kSrcStored;
+  for (int k = 0; k < 3; ++k) {
+    a.src_i0[k] = p->i0[k];
+    a.src_d[k] = p->d[k];
+  }
+  return features_of(p, a, f);
+}
+
+// The network's outputs for one normalised feature vector, on the host: the
+// sums of cufinufft_mlp_forward in the same order (a batch of one is 2 kflops;
+// two copies, three launches and a wait cost ~40 us).
+static void selector_forward(const float* x, float* y) {
+  constexpr int F = CUFINUFFT_MLP_FEATURES, H = CUFINUFFT_MLP_HIDDEN, K = CUFINUFFT_MLP_CLASSES;
+  float h1[H], h2[H];
+  const float* w = kSelParams;
+  auto dense = [&](const float* in, int ni, float* out, int no, bool relu) {
+    const float* bias = w + no * ni;
+    for (int o = 0; o < no; ++o) {
+      float s = bias[o];
+      for (int i = 0; i < ni; ++i) s = std::fmaf(w[o * ni + i], in[i], s);
+      out[o] = relu && s < 0.f ? 0.f : s;
+    }
+    w = bias + no;
+  };
+  dense(x, F, h1, H, true);
+  dense(h1, H, h2, H, true);
+  dense(h2, H, y, K, false);
+}
 
 // gpu_method 0 with a trained network: predict the twelve classes' relative
-// times from the plan's features and switch to the fastest runnable one.
+// times from the points' features and take the fastest runnable one for the
+// coming sort.
 template <typename T>
-static int select_layout(Plan<T>* p) {
-  if (!kSelectorTrained || !p->auto_method || !p->pts_set || p->M == 0) return 0;
-  float f[CUFINUFFT_MLP_FEATURES];
-  int e = features_impl(p, f);
+static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
+  if (!kSelectorTrained || !p->auto_method || p->M == 0) return 0;
+  float f[CUFINUFFT_MLP_FEATURES], y[CUFINUFFT_MLP_CLASSES];
+  const int e = features_of(p, src, f);
   if (e) return e;
   for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - kSelMean[k]) / kSelStd[k];
-  const int B = 1, Hd = CUFINUFFT_MLP_HIDDEN, K = CUFINUFFT_MLP_CLASSES;
-  const size_t nfl = CUFINUFFT_MLP_PARAMS + CUFINUFFT_MLP_FEATURES + K + 2 * B * Hd;
-  if (p->sel_buf == nullptr) {
-    CFG_CUDA(cudaMalloc(&p->sel_buf, sizeof(float) * nfl));
-    CFG_CUDA(cudaMemcpyAsync(p->sel_buf, kSelParams, sizeof(float) * CUFINUFFT_MLP_PARAMS,
-                             cudaMemcpyHostToDevice, p->stream));
-  }
-  float* params = p->sel_buf;
-  float* X = params + CUFINUFFT_MLP_PARAMS;
-  float* Y = X + CUFINUFFT_MLP_FEATURES;
-  float* work = Y + K;
-  CFG_CUDA(cudaMemcpyAsync(X, f, sizeof(f), cudaMemcpyHostToDevice, p->stream));
-  if (cufinufft_mlp_forward(params, X, B, Y, work, p->stream) != 0) return CUFINUFFT_ERR_CUDA;
-  float y[CUFINUFFT_MLP_CLASSES];
-  CFG_CUDA(cudaMemcpyAsync(y, Y, sizeof(y), cudaMemcpyDeviceToHost, p->stream));
-  CFG_CUDA(cudaStreamSynchronize(p->stream));
+  selector_forward(f, y);
   int best = -1;
-  for (int k = 0; k < K; ++k) {
-    cufinufft_tune_entry c = tune_candidates(p)[k];
-    if (c.ms == -2.f) continue;
+  const std::vector<cufinufft_tune_entry> cand = tune_candidates(p);
+  for (int k = 0; k < CUFINUFFT_MLP_CLASSES; ++k) {
+    if (cand[k].ms == -2.f) continue;
     if (best < 0 || y[k] < y[best]) best = k;
   }
   if (best < 0) return 0;
-  return apply_layout_class(p, best);
+  const int bs[3] = {cand[best].binsizex, cand[best].binsizey, cand[best].binsizez};
+  return adopt_layout(p, cand[best].method, bs, cand[best].maxsubprobsize);
 }
 
 template <typename T>

@@ -227,6 +227,13 @@ static int batch_make(Batch<T>* b, int nplans, Plan<T>** plans) {
     if (p->opts.gpu_kerevalmeth != 0) return CUFINUFFT_ERR_ARG;
     if (p->spread_only) return CUFINUFFT_ERR_ARG;  // the batch runs whole transforms
     if (p->type == 3) return CUFINUFFT_ERR_ARG;    // types 1 and 2 only
+    if (p->lo) {
+      const int e = resolve_nsub(p->lo, true);
+      if (e) return e;
+    } else {
+      const int e = resolve_nsub(p, true);
+      if (e) return e;
+    }
     b->plans.push_back(p);
   }
   CFG_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
@@ -322,8 +329,9 @@ static int batch_execute(Batch<T>* b, cplx_t<T>** c, cplx_t<T>** fk) {
   const int n = (int)b->plans.size();
   if (c == nullptr || fk == nullptr) return CUFINUFFT_ERR_ARG;
   // the previous replay must have copied the descriptor table before it is
-  // rewritten
-  if (b->launched) CFG_CUDA(cudaEventSynchronize(b->done));
+  // rewritten (the graph of per-plan executes holds no table: its replays
+  // queue behind one another without the host)
+  if (b->launched && !b->by_plans) CFG_CUDA(cudaEventSynchronize(b->done));
   for (int i = 0; i < n; ++i) {
     if ((b->plans[i]->M > 0 && c[i] == nullptr) || fk[i] == nullptr) return CUFINUFFT_ERR_ARG;
     if (b->by_plans) continue;
@@ -343,6 +351,7 @@ static int batch_execute(Batch<T>* b, cplx_t<T>** c, cplx_t<T>** fk) {
   if (b->by_plans && b->gexec != nullptr &&
       !(std::equal(b->cap_c.begin(), b->cap_c.end(), c) && std::equal(b->cap_fk.begin(), b->cap_fk.end(), fk))) {
     // other caller arrays: capture again
+    if (b->launched) CFG_CUDA(cudaStreamSynchronize(b->stream));
     cudaGraphExecDestroy(b->gexec);
     cudaGraphDestroy(b->graph);
     b->gexec = nullptr;

@@ -42,67 +42,70 @@ struct BankOrder {
   int dense_min;         // dense_run(dim) (cell_order only)
 };
 
+// Where a sort's points come from: the caller's coordinates, stored first taps
+// and offsets (any order, src_idx the caller's index), or FP64 coordinates
+// placed in FP64 (fold, rescale, first tap) with the tap offset in [0,1)
+// rounded to the plan's FP32 (the FP32 chain of an FP64 plan).
+enum PointSrc { kSrcCoords = 0, kSrcStored = 1, kSrcNarrow = 2 };
+
 template <typename T> struct PlaceArgs {
-  const T* x[3];           // caller's coordinates (device)
+  int src;                 // PointSrc
+  const T* x[3];           // kSrcCoords: caller's coordinates (device)
   AxisMap<T> ax[3];
+  const double* xd[3];     // kSrcNarrow
+  AxisMap<double> axd[3];
+  const int* src_idx;      // kSrcStored
+  const int* src_i0[3];
+  const T* src_d[3];
   int dim;
   int M;
   int bs[3];               // bin size per axis (cells)
   int nb[3];               // bins per axis
+  unsigned magic[3];       // set by the launchers
   // outputs
   int* idx;                // sorted position -> caller index
   int* i0[3];
   T* d[3];
-  int* count;              // [nbins] (must be zeroed before bin_count)
+  int* count;              // [nbins]
   int* rank;               // [M] rank of the point inside its bin (or its class)
   const int* start;        // [nbins+1] exclusive scan of count
+  // plain bin order: the counter of bin b is raw[b raw_stride] (zeroed)
+  int* raw;
+  int raw_stride;
   BankOrder bank;
 };
-template <typename T> cudaError_t launch_bin_count(const PlaceArgs<T>& a, cudaStream_t s);
-template <typename T> cudaError_t launch_permute(const PlaceArgs<T>& a, cudaStream_t s);
-template <typename T> cudaError_t launch_place_unsorted(const PlaceArgs<T>& a, cudaStream_t s);
+// Bins whose counters, one int each, would share few L2 sectors (all atomics
+// of a sort meet there: 1e5 points in 256 bins, 19 us) get a sector each.
+constexpr int kCountStride = 8, kCountStrideBins = 8192;
 
-// FP64 coordinates placed in FP64 (fold, rescale, first tap) with the tap
-// offset in [0,1) rounded to FP32, in caller order (idx[i] = i): the input
-// of an FP32 chain's sort in an FP64 plan.
-struct NarrowPlaceArgs {
-  const double* x[3];
-  AxisMap<double> ax[3];
-  int dim, M;
-  int* idx;
-  int* i0[3];
-  float* d[3];
+// Subproblem headers to write beside the permutation (nsub: their upper bound;
+// 0: none).
+struct SubHdrArgs {
+  const int* sub_start;    // [nbins+1]
+  int nbins, nsub, maxsub;
+  int* sub_to_bin;
+  SubHdr* hdr;
 };
-cudaError_t launch_place_narrow(const NarrowPlaceArgs& a, cudaStream_t s);
+// raw: per counters of bin b at raw + b raw_stride; count may equal raw when
+// both are plain.  partial: bin_scan_partials(nbins) words.
+struct BinScanArgs {
+  const int* raw;
+  int raw_stride, per, nbins, maxsub;
+  int *count, *start, *sub_start;
+  unsigned long long* partial;
+};
+int bin_scan_partials(int nbins);
+cudaError_t launch_bin_scan(const BinScanArgs& a, cudaStream_t s);
+template <typename T> cudaError_t launch_bin_count(PlaceArgs<T> a, cudaStream_t s);
+template <typename T> cudaError_t launch_permute(PlaceArgs<T> a, const SubHdrArgs& h, cudaStream_t s);
+template <typename T> cudaError_t launch_place_unsorted(PlaceArgs<T> a, cudaStream_t s);
 
 // Complex FP64 <-> FP32 conversion of n values.
 cudaError_t launch_narrow_complex(const double2* in, float2* out, long long n, cudaStream_t s);
 cudaError_t launch_widen_complex(const float2* in, double2* out, long long n, cudaStream_t s);
 
-// Re-binning of already placed points (no caller coordinates needed): the
-// bin of a point depends only on its first taps i0, so a new bin layout is a
-// counting sort of the stored arrays into fresh ones.
-template <typename T> struct RebinArgs {
-  int dim, M;
-  int bs[3], nb[3];
-  const int* src_idx;
-  const int* src_i0[3];
-  const T* src_d[3];
-  int* idx;
-  int* i0[3];
-  T* d[3];
-  int* count;      // [nbins], zeroed before rebin_count
-  int* rank;       // [M]
-  const int* start;
-  BankOrder bank;
-};
-template <typename T> cudaError_t launch_rebin_count(const RebinArgs<T>& a, cudaStream_t s);
-template <typename T> cudaError_t launch_rebin_permute(const RebinArgs<T>& a, cudaStream_t s);
-
-// Point counts over fixed feature bins (fb cells per axis) from the stored
-// first taps; counts must be zeroed.
-cudaError_t launch_feature_count(int dim, int M, const int* const i0[3], const int fb[3],
-                                 const int nb[3], int* counts, cudaStream_t s);
+// Point counts over the bins a.bs x a.nb into a.count (zeroed).
+template <typename T> cudaError_t launch_feature_count(PlaceArgs<T> a, cudaStream_t s);
 
 // Exclusive scan of n ints: out[0..n] (out[n] = total).  mode 0 scans the
 // values, mode 1 scans ceil(v / div), mode 2 scans v where v >= div (else
@@ -110,7 +113,6 @@ cudaError_t launch_feature_count(int dim, int M, const int* const i0[3], const i
 int scan_tmp_ints(int n);
 cudaError_t launch_scan(const int* in, int* out, int n, int mode, int div, int* tmp,
                         cudaStream_t s);
-// sub_to_bin[s] = the bin b with sub_start[b] <= s < sub_start[b+1].
 // Cell order: flag the subproblems whose first point lies on a dense cell
 // (those go to the cell-run kernel, the others to the warp-cooperative one).
 struct SubClassArgs {
@@ -121,6 +123,7 @@ struct SubClassArgs {
   const int* cls_count;
   int bs[3];
   int dim, maxsub, ncls, nsub, dense_min;
+  const int* sub_total;  // subproblems in all (device); nsub is their upper bound
   unsigned char* dense;
   // optional: per subproblem, its leading points on dense cells (a bin's
   // dense cells come first), from the scanned dense counts and bin counts
@@ -133,14 +136,6 @@ cudaError_t launch_classify_subproblems(const SubClassArgs& a, cudaStream_t s);
 // the driver has none).  makeplan looks it up for type-2 plans, so the first
 // lookup does not happen inside a stream capture.
 void* tma_encoder();
-
-cudaError_t launch_sub_to_bin(const int* sub_start, int nbins, int nsub, int* sub_to_bin,
-                              cudaStream_t s);
-// sub_to_bin plus the subproblem headers (hdr[nsub]) of bins bs x nb holding
-// count[b] points from start[b] on, at most maxsub per subproblem.
-cudaError_t launch_sub_headers(const int* sub_start, const int* start, const int* count, int nbins,
-                               int nsub, int maxsub, const int bs[3], const int nb[3], int* sub_to_bin,
-                               SubHdr* hdr, cudaStream_t s);
 
 // deconv.cu
 struct FseriesNodes {

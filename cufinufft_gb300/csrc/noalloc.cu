@@ -245,9 +245,12 @@ extern "C" int cufinufftf_spread2d_noalloc(int M, const float* x, const float* y
   pa.count = count;
   pa.rank = rank;
   pa.start = start;
+  pa.raw = count;
+  pa.raw_stride = 1;
   e = launch_bin_count<float>(pa, stream);
   if (e == cudaSuccess) e = launch_scan(count, start, (int)nbins, 0, 1, scan_tmp, stream);
-  if (e == cudaSuccess) e = launch_permute<float>(pa, stream);
+  const SubHdrArgs no_headers{};
+  if (e == cudaSuccess) e = launch_permute<float>(pa, no_headers, stream);
   if (e == cudaSuccess) e = launch_scan(count, sub_start, (int)nbins, 1, kNaMaxSub, scan_tmp, stream);
   const int nsub_max = (int)nbins + (M + kNaMaxSub - 1) / kNaMaxSub;
   if (e == cudaSuccess) {

@@ -28,7 +28,6 @@ template <typename T> struct Plan {
                    // (layout method 5 = method 2 with cell_order, see set_layout)
   int variant = 0; // kernel family: 0 default, 1 one thread per point, 2 warp-cooperative
   bool auto_method = false;  // gpu_method 0: chosen by the library
-  float* sel_buf = nullptr;  // selector network parameters and scratch (device)
   int sort = 1;
   int bs[3] = {1, 1, 1}, nb[3] = {1, 1, 1};
   int nbins = 1;
@@ -62,11 +61,15 @@ template <typename T> struct Plan {
   int* i0[3] = {nullptr, nullptr, nullptr};
   T* d[3] = {nullptr, nullptr, nullptr};
   int* rank = nullptr;
+  int* feat = nullptr;         // occupancy counts of the selector's features
+  size_t cap_feat = 0;
   size_t capM = 0;
   int* count = nullptr;
   int* start = nullptr;
   int* sub_start = nullptr;
-  int* scan_tmp = nullptr;
+  unsigned long long* scan_part = nullptr;  // block sums of the bin scan
+  int* raw = nullptr;          // sector-strided bin counters (kCountStride), small nbins
+  size_t cap_bins = 0, cap_raw = 0;
   int* sub_to_bin = nullptr;
   SubHdr* sub_hdr = nullptr;  // [cap_sub] subproblem headers
   size_t cap_sub = 0;
@@ -83,13 +86,9 @@ template <typename T> struct Plan {
   int* sub_ndense = nullptr;  // cell order: leading dense points per subproblem
   // FP64 plans whose tolerance allows it run the spread/interp, FFT and
   // deconvolution chain in FP32: `lo` is that FP32 plan (null otherwise).
-  // This side folds and rescales the points in FP64 (n_* arrays: caller
-  // order, input of lo's sort) and converts c / fk (c32, fk32).
+  // Its sort folds and rescales this side's FP64 points in FP64 (kSrcNarrow);
+  // this side converts c / fk (c32, fk32).
   Plan<float>* lo = nullptr;
-  int* n_idx = nullptr;
-  int* n_i0[3] = {nullptr, nullptr, nullptr};
-  float* n_d[3] = {nullptr, nullptr, nullptr};
-  size_t n_cap = 0;
   cplx_t<float>* c32 = nullptr;
   size_t c32_cap = 0;
   cplx_t<float>* fk32 = nullptr;
@@ -108,19 +107,26 @@ template <typename T> struct Plan {
   cplx_t<T>* t3_grid = nullptr;       // [ntransf nf] spread grid
   size_t t3_capM = 0, t3_capN = 0, t3_capG = 0;
   double* t3_part = nullptr;          // min/max partials (device)
-  int* h_total = nullptr;  // pinned readback of the subproblem count
+  // subproblem count: nsub is its upper bound (surplus headers are empty) until
+  // the pinned readback h_total of the last sort has landed (ev_total)
+  int* h_total = nullptr;
+  cudaEvent_t ev_total = nullptr;
+  bool nsub_exact = true;
   // interpolation tile-wait status (SpreadArgs::status): host-mapped, two ints
   int* h_status = nullptr;
   int* d_status = nullptr;
   int tma_wait_test = 0;   // CUFINUFFT_TMA_WAIT_TEST=1 at makeplan
   int fp64_df = 0;         // FP64 type 2: double-float subproblem interpolation
-  // execute as a CUDA graph (timing off): captured for one pair of caller
-  // arrays and one plan state (`version` counts setpts / set_layout)
+  // execute as a CUDA graph (timing off): captured when a call repeats the
+  // last one's caller arrays and plan state (`version` counts setpts /
+  // set_layout); g_*: what the graph was captured for, last_*: the last call
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   const void* g_c = nullptr;
   const void* g_fk = nullptr;
-  unsigned version = 0, g_version = 0;
+  const void* last_c = nullptr;
+  const void* last_fk = nullptr;
+  unsigned version = 0, g_version = 0, last_version = 0;
   // stage timing (extension): events recorded around each stage of execute
   bool timing = false;
   std::vector<cudaEvent_t> ev_pool;   // free events
@@ -245,6 +251,10 @@ template <typename T>
 int execute_plan(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk);
 template <typename T>
 int plan_use_stream(Plan<T>* p, cudaStream_t s);
+// The subproblem count of the last sort from its readback, if that has landed
+// (wait: once it has); until then nsub is an upper bound.
+template <typename T>
+int resolve_nsub(Plan<T>* p, bool wait);
 
 template <typename T>
 inline cudaError_t run_spread(Plan<T>* p, const SpreadArgs<T>& a) {

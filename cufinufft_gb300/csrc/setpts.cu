@@ -4,16 +4,28 @@
 // 386-613): CalcBinSize_noghost (per-point bin + atomic rank), a Thrust
 // exclusive scan, CalcInvertofGlobalSortIdx (scatter of the permutation),
 // then CalcSubProb / inclusive scan / MapBintoSubProb for the subproblem
-// method.  Here:
+// method and a host readback of their number.  Here:
 //   * k_bin_count places every point on the fine grid (place_coord) and ranks
-//     it inside its bin with warp-aggregated atomics (one atomic per distinct
-//     bin in a warp, so clustered points do not serialise on one counter);
-//   * a three-phase block scan produces the bin starts and the subproblem
-//     starts (mode 1 scans ceil(count/maxsub) directly);
+//     it inside its bin -- or directly inside its (bin, bank class), whose
+//     counts sum to the bin's -- with one warp-aggregated atomic (one per
+//     distinct key in a warp, so clustered points do not serialise on one
+//     counter); a few thousand bins or fewer keep their counters a sector
+//     apart (kCountStride), or all atomics meet in a handful of L2 sectors;
+//   * k_bin_scan turns the counters into bin counts, bin starts and
+//     subproblem starts in one pass (two launches beyond 4096 bins);
 //   * k_permute writes the sorted structure-of-arrays copy the spread and
-//     interp kernels stream: caller index, first tap and offset per axis;
-//   * k_sub_to_bin maps subproblems to bins by binary search (one thread per
-//     subproblem, balanced even when one bin holds most of the points).
+//     interp kernels stream -- caller index, first tap and offset per axis --
+//     and, in further blocks of the same launch, the subproblem headers (binary
+//     search, balanced even when one bin holds most of the points).  The
+//     number of subproblems stays on the device: headers are written for its
+//     upper bound, the surplus empty, and the host learns the number when it
+//     next needs it.
+// Points come from the caller's coordinates, from the plan's stored first
+// taps and offsets (a new layout), or from FP64 coordinates for an FP32 chain
+// (placed in FP64, the offset rounded afterwards).
+// 1e5 points, 512^2 grid: 12 launches, a readback and ~45 us of device time ->
+// 5 launches, none waited for; set_pts and execute together 130 -> 33 us a call
+// in a stream of calls.
 #include "device_common.cuh"
 #include "kernels.h"
 
@@ -21,41 +33,47 @@ namespace cfg {
 
 constexpr int kPlaceThreads = 256;
 
-template <typename T>
-__device__ __forceinline__ int point_bin(const PlaceArgs<T>& a, int i, int i0[3], T d[3]) {
+// i / bs by a reciprocal: floor(2^32 / bs) + 1 overestimates by at most one
+// for i, bs < 2^31 with i bs < 2^33, which the check takes back.
+__device__ __forceinline__ int bin_div(int i, int bs, unsigned magic) {
+  int q = bs == 1 ? i : (int)__umulhi((unsigned)i, magic);
+  if (q * bs > i) --q;
+  return q;
+}
+
+// First taps and offsets of point i, and its bin.
+template <typename T, int SRC>
+__device__ __forceinline__ int point_bin(const PlaceArgs<T>& a, int i, int i0[3], T d[3], int lc[3]) {
   int b = 0, mul = 1;
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (k < a.dim) {
-      place_coord<T>(a.x[k][i], a.ax[k], i0[k], d[k]);
-      b += mul * (i0[k] / a.bs[k]);
+      if (SRC == kSrcStored) {
+        i0[k] = a.src_i0[k][i];
+        d[k] = a.src_d[k][i];
+      } else if (SRC == kSrcNarrow) {
+        double dd;
+        place_coord<double>(a.xd[k][i], a.axd[k], i0[k], dd);
+        d[k] = (T)dd;
+      } else {
+        place_coord<T>(a.x[k][i], a.ax[k], i0[k], d[k]);
+      }
+      const int q = bin_div(i0[k], a.bs[k], a.magic[k]);
+      lc[k] = i0[k] - q * a.bs[k];
+      b += mul * q;
       mul *= a.nb[k];
+    } else {
+      lc[k] = 0;
     }
   }
   return b;
 }
 
-// Bank class of a point whose first taps are i0 (see BankOrder).
-__device__ __forceinline__ int bank_class(const BankOrder& o, const int* bs, int dim, const int i0[3]) {
-  const int lx = i0[0] % bs[0];
-  const int ly = dim > 1 ? i0[1] % bs[1] : 0;
-  const int lz = dim > 2 ? i0[2] % bs[2] : 0;
-  return (lx + o.tx * (ly + o.ty * lz)) & (o.ncls - 1);
-}
-
-// Class of a point inside its bin: its bank class, or its cell (cell order).
-__device__ __forceinline__ int order_class(const BankOrder& o, const int* bs, int dim, const int i0[3]) {
-  if (!o.cell_order) return bank_class(o, bs, dim, i0);
-  const int lx = i0[0] % bs[0];
-  const int ly = dim > 1 ? i0[1] % bs[1] : 0;
-  const int lz = dim > 2 ? i0[2] % bs[2] : 0;
-  return lx + bs[0] * (ly + bs[1] * lz);
-}
-
-// Position of a ranked point: cell order reads the scanned (bin, cell)
-// starts; bank order interleaves inside the bin.
-__device__ __forceinline__ int interleave_pos(const BankOrder& o, int b, int c, int r);
-__device__ __forceinline__ int ordered_pos(const BankOrder& o, const int* start, int b, int c, int r) {
-  return start[b] + interleave_pos(o, b, c, r);
+// Class of a point inside its bin, from its cell inside the bin: its bank
+// class (see BankOrder), or the cell (cell order).
+__device__ __forceinline__ int order_class(const BankOrder& o, const int* bs, const int lc[3]) {
+  if (!o.cell_order) return (lc[0] + o.tx * (lc[1] + o.ty * lc[2])) & (o.ncls - 1);
+  return lc[0] + bs[0] * (lc[1] + bs[1] * lc[2]);
 }
 
 // Warp-aggregated rank: one atomic per distinct key in the warp.
@@ -88,16 +106,18 @@ __device__ __forceinline__ int cell_position(const BankOrder& o, const int* star
 // Position inside its bin of the point ranked r in class c: round-robin over
 // the classes, rounds shrinking as classes run out.
 __device__ __forceinline__ int interleave_pos(const BankOrder& o, int b, int c, int r) {
-  const int* cnt = o.cls_count + (long long)b * o.ncls;
+  const int4* cnt = reinterpret_cast<const int4*>(o.cls_count + (long long)b * o.ncls);  // ncls 8 or 16
   int pos = 0;
-  for (int k = 0; k < o.ncls; ++k) {
-    const int n = __ldg(cnt + k);
-    pos += min(n, r) + ((k < c && n > r) ? 1 : 0);
+  for (int k = 0; k < o.ncls; k += 4) {
+    const int4 v = __ldg(cnt + (k >> 2));
+    const int n[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) pos += min(n[u], r) + ((k + u < c && n[u] > r) ? 1 : 0);
   }
   return pos;
 }
 
-template <typename T>
+template <typename T, int SRC>
 __global__ void __launch_bounds__(kPlaceThreads) k_bin_count(PlaceArgs<T> a) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   // warp-uniform trip count so the warp stays converged for __match_any_sync
@@ -107,22 +127,59 @@ __global__ void __launch_bounds__(kPlaceThreads) k_bin_count(PlaceArgs<T> a) {
     const unsigned act = __ballot_sync(0xffffffffu, active);
     if (!active) continue;
     const int i = (int)ii;
-    int i0[3];
+    int i0[3], lc[3];
     T d[3];
-    const int b = point_bin(a, i, i0, d);
-    const int r = agg_rank(act, b, &a.count[b]);
+    const int b = point_bin<T, SRC>(a, i, i0, d, lc);
+    int r;
     if (a.bank.cls_count) {
-      const int key = b * a.bank.ncls + order_class(a.bank, a.bs, a.dim, i0);
-      a.rank[i] = agg_rank(act, key, a.bank.cls_count + key);
+      if (a.bank.cell_order) agg_rank(act, b, &a.count[b]);
+      const int key = b * a.bank.ncls + order_class(a.bank, a.bs, lc);
+      r = agg_rank(act, key, a.bank.cls_count + key);
     } else {
-      a.rank[i] = r;
+      r = agg_rank(act, b, a.raw + (size_t)b * a.raw_stride);
     }
+    a.rank[i] = r;
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
+// Subproblem headers (k_sub_headers' part of k_permute): the subproblem's bin
+// by binary search, its point range (subproblem js of bin b: points start[b] +
+// js maxsub, at most maxsub of them) and its tile origin (the bin's first
+// cell); subproblems past the total, up to the bound the host launches with,
+// are empty.
+__device__ __forceinline__ void write_header(const SubHdrArgs& h, const int* start, const int* count,
+                                             const int* bs, const int* nb, int sidx) {
+  const int total = h.sub_start[h.nbins];
+  SubHdr o;
+  o.p0 = o.np = o.ox = o.oy = o.oz = o.pad0 = o.pad1 = o.pad2 = 0;
+  int lo = 0;
+  if (sidx < total) {
+    int hi = h.nbins;  // invariant: sub_start[lo] <= sidx < sub_start[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (h.sub_start[mid] <= sidx) lo = mid;
+      else hi = mid;
+    }
+    const int js = sidx - h.sub_start[lo];
+    o.p0 = start[lo] + js * h.maxsub;
+    o.np = min(h.maxsub, count[lo] - js * h.maxsub);
+    o.ox = (lo % nb[0]) * bs[0];
+    o.oy = ((lo / nb[0]) % nb[1]) * bs[1];
+    o.oz = (lo / (nb[0] * nb[1])) * bs[2];
+  }
+  h.sub_to_bin[sidx] = lo;
+  h.hdr[sidx] = o;
+}
+
+// Blocks [0, pblocks) permute, the others write headers.
+template <typename T, int SRC>
+__global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a, SubHdrArgs h, int pblocks) {
+  if ((int)blockIdx.x >= pblocks) {
+    const int sidx = ((int)blockIdx.x - pblocks) * blockDim.x + threadIdx.x;
+    if (sidx < h.nsub) write_header(h, a.start, a.count, a.bs, a.nb, sidx);
+    return;
+  }
+  const long long stride = (long long)pblocks * blockDim.x;
   // warp-uniform trip count: cell order ranks sparse points warp-aggregated
   for (long long base = (long long)blockIdx.x * blockDim.x; base < a.M; base += stride) {
     const long long ii = base + threadIdx.x;
@@ -130,14 +187,16 @@ __global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a) {
     const unsigned act = __ballot_sync(0xffffffffu, active);
     if (!active) continue;
     const int i = (int)ii;
-    int i0[3];
+    int i0[3], lc[3];
     T d[3];
-    const int b = point_bin(a, i, i0, d);
+    const int b = point_bin<T, SRC>(a, i, i0, d, lc);
+    const int r = a.rank[i];
     int pos;
-    if (!a.bank.cls_count) pos = a.start[b] + a.rank[i];
-    else if (a.bank.cell_order) pos = cell_position(a.bank, a.start, act, b, order_class(a.bank, a.bs, a.dim, i0), a.rank[i]);
-    else pos = ordered_pos(a.bank, a.start, b, order_class(a.bank, a.bs, a.dim, i0), a.rank[i]);
-    a.idx[pos] = i;
+    if (!a.bank.cls_count) pos = a.start[b] + r;
+    else if (a.bank.cell_order) pos = cell_position(a.bank, a.start, act, b, order_class(a.bank, a.bs, lc), r);
+    else pos = a.start[b] + interleave_pos(a.bank, b, order_class(a.bank, a.bs, lc), r);
+    a.idx[pos] = SRC == kSrcStored ? a.src_idx[i] : i;
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
       if (k < a.dim) {
         a.i0[k][pos] = i0[k];
@@ -149,32 +208,17 @@ __global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a) {
 
 // gpu_sort = 0 with method 1 keeps the caller's order (reference "GM",
 // TrivialGlobalSortIdx, src/precision_independent.cu:98-105).
-template <typename T>
+template <typename T, int SRC>
 __global__ void __launch_bounds__(kPlaceThreads) k_place_unsorted(PlaceArgs<T> a) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.M; i += gridDim.x * blockDim.x) {
+    int i0[3], lc[3];
+    T d[3];
+    point_bin<T, SRC>(a, i, i0, d, lc);
     a.idx[i] = i;
     for (int k = 0; k < 3; ++k) {
       if (k < a.dim) {
-        int i0;
-        T d;
-        place_coord<T>(a.x[k][i], a.ax[k], i0, d);
-        a.i0[k][i] = i0;
-        a.d[k][i] = d;
-      }
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kPlaceThreads) k_place_narrow(NarrowPlaceArgs a) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.M; i += gridDim.x * blockDim.x) {
-    a.idx[i] = i;
-    for (int k = 0; k < 3; ++k) {
-      if (k < a.dim) {
-        int i0;
-        double d;
-        place_coord<double>(a.x[k][i], a.ax[k], i0, d);
-        a.i0[k][i] = i0;
-        a.d[k][i] = (float)d;
+        a.i0[k][i] = i0[k];
+        a.d[k][i] = d[k];
       }
     }
   }
@@ -186,149 +230,72 @@ static int place_grid(int M) {
   return b < 1 ? 1 : (int)b;
 }
 
-template <typename T> cudaError_t launch_bin_count(const PlaceArgs<T>& a, cudaStream_t s) {
+static void set_magic(const int bs[3], unsigned magic[3]) {
+  for (int k = 0; k < 3; ++k) magic[k] = bs[k] > 1 ? (unsigned)((1ull << 32) / (unsigned)bs[k] + 1) : 0u;
+}
+
+// One kernel instance per point source.
+#define CFG_SRC_SWITCH(KERNEL, GRID, ...)                                              \
+  switch (a.src) {                                                                     \
+    case kSrcStored: KERNEL<T, kSrcStored><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break; \
+    case kSrcNarrow: KERNEL<T, kSrcNarrow><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break; \
+    default: KERNEL<T, kSrcCoords><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break;  \
+  }
+
+template <typename T> cudaError_t launch_bin_count(PlaceArgs<T> a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
-  k_bin_count<T><<<place_grid(a.M), kPlaceThreads, 0, s>>>(a);
+  set_magic(a.bs, a.magic);
+  CFG_SRC_SWITCH(k_bin_count, place_grid(a.M), a)
   return cudaGetLastError();
 }
-template <typename T> cudaError_t launch_permute(const PlaceArgs<T>& a, cudaStream_t s) {
+template <typename T> cudaError_t launch_permute(PlaceArgs<T> a, const SubHdrArgs& h, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
-  k_permute<T><<<place_grid(a.M), kPlaceThreads, 0, s>>>(a);
+  set_magic(a.bs, a.magic);
+  const int pb = place_grid(a.M), hb = (h.nsub + kPlaceThreads - 1) / kPlaceThreads;
+  CFG_SRC_SWITCH(k_permute, pb + hb, a, h, pb)
   return cudaGetLastError();
 }
-template <typename T> cudaError_t launch_place_unsorted(const PlaceArgs<T>& a, cudaStream_t s) {
+template <typename T> cudaError_t launch_place_unsorted(PlaceArgs<T> a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
-  k_place_unsorted<T><<<place_grid(a.M), kPlaceThreads, 0, s>>>(a);
+  set_magic(a.bs, a.magic);
+  CFG_SRC_SWITCH(k_place_unsorted, place_grid(a.M), a)
   return cudaGetLastError();
 }
 
-cudaError_t launch_place_narrow(const NarrowPlaceArgs& a, cudaStream_t s) {
-  if (a.M == 0) return cudaSuccess;
-  k_place_narrow<<<place_grid(a.M), kPlaceThreads, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
-template cudaError_t launch_bin_count<float>(const PlaceArgs<float>&, cudaStream_t);
-template cudaError_t launch_bin_count<double>(const PlaceArgs<double>&, cudaStream_t);
-template cudaError_t launch_permute<float>(const PlaceArgs<float>&, cudaStream_t);
-template cudaError_t launch_permute<double>(const PlaceArgs<double>&, cudaStream_t);
-template cudaError_t launch_place_unsorted<float>(const PlaceArgs<float>&, cudaStream_t);
-template cudaError_t launch_place_unsorted<double>(const PlaceArgs<double>&, cudaStream_t);
+template cudaError_t launch_bin_count<float>(PlaceArgs<float>, cudaStream_t);
+template cudaError_t launch_bin_count<double>(PlaceArgs<double>, cudaStream_t);
+template cudaError_t launch_permute<float>(PlaceArgs<float>, const SubHdrArgs&, cudaStream_t);
+template cudaError_t launch_permute<double>(PlaceArgs<double>, const SubHdrArgs&, cudaStream_t);
+template cudaError_t launch_place_unsorted<float>(PlaceArgs<float>, cudaStream_t);
+template cudaError_t launch_place_unsorted<double>(PlaceArgs<double>, cudaStream_t);
 
 // ---------------------------------------------------------------------------
-// Re-binning from stored first taps.
-template <typename T>
-__device__ __forceinline__ int stored_bin(const RebinArgs<T>& a, int i) {
-  int b = 0, mul = 1;
-  for (int k = 0; k < 3; ++k) {
-    if (k < a.dim) {
-      b += mul * (a.src_i0[k][i] / a.bs[k]);
-      mul *= a.nb[k];
-    }
-  }
-  return b;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kPlaceThreads) k_rebin_count(RebinArgs<T> a) {
+// Occupancy counts for the selector's features, over bins a.bs x a.nb, of the
+// points of any source (so that a layout can be chosen before the sort).
+template <typename T, int SRC>
+__global__ void __launch_bounds__(kPlaceThreads) k_feature_count(PlaceArgs<T> a) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long base = (long long)blockIdx.x * blockDim.x; base < a.M; base += stride) {
     const long long ii = base + threadIdx.x;
     const bool active = ii < a.M;
     const unsigned act = __ballot_sync(0xffffffffu, active);
     if (!active) continue;
-    const int i = (int)ii;
-    const int b = stored_bin(a, i);
-    const int r = agg_rank(act, b, &a.count[b]);
-    if (a.bank.cls_count) {
-      const int i0[3] = {a.src_i0[0][i], a.dim > 1 ? a.src_i0[1][i] : 0, a.dim > 2 ? a.src_i0[2][i] : 0};
-      const int key = b * a.bank.ncls + order_class(a.bank, a.bs, a.dim, i0);
-      a.rank[i] = agg_rank(act, key, a.bank.cls_count + key);
-    } else {
-      a.rank[i] = r;
-    }
+    int i0[3], lc[3];
+    T d[3];
+    const int b = point_bin<T, SRC>(a, (int)ii, i0, d, lc);
+    const unsigned peers = __match_any_sync(act, b);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&a.count[b], __popc(peers));
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kPlaceThreads) k_rebin_permute(RebinArgs<T> a) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x; base < a.M; base += stride) {
-    const long long ii = base + threadIdx.x;
-    const bool active = ii < a.M;
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (!active) continue;
-    const int i = (int)ii;
-    const int b = stored_bin(a, i);
-    int pos = a.start[b] + a.rank[i];
-    if (a.bank.cls_count) {
-      const int i0[3] = {a.src_i0[0][i], a.dim > 1 ? a.src_i0[1][i] : 0, a.dim > 2 ? a.src_i0[2][i] : 0};
-      const int c = order_class(a.bank, a.bs, a.dim, i0);
-      pos = a.bank.cell_order ? cell_position(a.bank, a.start, act, b, c, a.rank[i])
-                              : ordered_pos(a.bank, a.start, b, c, a.rank[i]);
-    }
-    a.idx[pos] = a.src_idx[i];
-    for (int k = 0; k < 3; ++k) {
-      if (k < a.dim) {
-        a.i0[k][pos] = a.src_i0[k][i];
-        a.d[k][pos] = a.src_d[k][i];
-      }
-    }
-  }
-}
-
-template <typename T> cudaError_t launch_rebin_count(const RebinArgs<T>& a, cudaStream_t s) {
+template <typename T> cudaError_t launch_feature_count(PlaceArgs<T> a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
-  k_rebin_count<T><<<place_grid(a.M), kPlaceThreads, 0, s>>>(a);
+  set_magic(a.bs, a.magic);
+  CFG_SRC_SWITCH(k_feature_count, place_grid(a.M), a)
   return cudaGetLastError();
 }
-template <typename T> cudaError_t launch_rebin_permute(const RebinArgs<T>& a, cudaStream_t s) {
-  if (a.M == 0) return cudaSuccess;
-  k_rebin_permute<T><<<place_grid(a.M), kPlaceThreads, 0, s>>>(a);
-  return cudaGetLastError();
-}
-template cudaError_t launch_rebin_count<float>(const RebinArgs<float>&, cudaStream_t);
-template cudaError_t launch_rebin_count<double>(const RebinArgs<double>&, cudaStream_t);
-template cudaError_t launch_rebin_permute<float>(const RebinArgs<float>&, cudaStream_t);
-template cudaError_t launch_rebin_permute<double>(const RebinArgs<double>&, cudaStream_t);
-
-// ---------------------------------------------------------------------------
-// Occupancy counts for the selector's features.
-struct FeatureArgs {
-  const int* i0[3];
-  int fb[3], nb[3];
-  int dim, M;
-  int* counts;
-};
-
-__global__ void k_feature_count(FeatureArgs a) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.M; i += gridDim.x * blockDim.x) {
-    int b = 0, mul = 1;
-    for (int k = 0; k < 3; ++k) {
-      if (k < a.dim) {
-        b += mul * (a.i0[k][i] / a.fb[k]);
-        mul *= a.nb[k];
-      }
-    }
-    atomicAdd(&a.counts[b], 1);
-  }
-}
-
-cudaError_t launch_feature_count(int dim, int M, const int* const i0[3], const int fb[3],
-                                 const int nb[3], int* counts, cudaStream_t s) {
-  if (M == 0) return cudaSuccess;
-  FeatureArgs a;
-  for (int k = 0; k < 3; ++k) {
-    a.i0[k] = i0[k];
-    a.fb[k] = fb[k];
-    a.nb[k] = nb[k];
-  }
-  a.dim = dim;
-  a.M = M;
-  a.counts = counts;
-  k_feature_count<<<place_grid(M), kPlaceThreads, 0, s>>>(a);
-  return cudaGetLastError();
-}
+template cudaError_t launch_feature_count<float>(PlaceArgs<float>, cudaStream_t);
+template cudaError_t launch_feature_count<double>(PlaceArgs<double>, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Exclusive scan: 1024 threads x 4 items per block; block totals are scanned
@@ -444,8 +411,120 @@ cudaError_t launch_scan(const int* in, int* out, int n, int mode, int div, int* 
   return cudaGetLastError();
 }
 
+// Bin counts, bin starts and subproblem starts in one pass: the counters of
+// bin b are the `per` ints at raw + b raw_stride (its classes, or itself), a
+// bin of c points holds ceil(c / maxsub) subproblems (maxsub 0: none).  Both
+// running sums travel in one 64-bit scan, points low, subproblems high.
+__device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned long long v, unsigned long long& excl) {
+  __shared__ unsigned long long warp_tot[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long n = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += n;
+  }
+  __syncthreads();
+  if (lane == 31) warp_tot[w] = incl;
+  __syncthreads();
+  unsigned long long before = 0, total = 0;
+  for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+    const unsigned long long t = warp_tot[k];
+    if (k < w) before += t;
+    total += t;
+  }
+  excl = before + incl - v;
+  return total;
+}
+
+__device__ __forceinline__ int bin_total(const BinScanArgs& a, int b) {
+  if (b >= a.nbins) return 0;
+  const int* c = a.raw + (size_t)b * a.raw_stride;
+  int n = 0;
+  if ((a.per & 3) == 0) {  // classes: 8 or 16 counters, 16-byte aligned
+    for (int k = 0; k < a.per; k += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(c + k);
+      n += v.x + v.y + v.z + v.w;
+    }
+    return n;
+  }
+  return c[0];
+}
+__device__ __forceinline__ unsigned long long bin_sums(const BinScanArgs& a, int n) {
+  const unsigned long long subs = a.maxsub > 0 && n > 0 ? ((unsigned)n - 1u) / (unsigned)a.maxsub + 1u : 0u;
+  return (subs << 32) | (unsigned)n;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_bin_sums(BinScanArgs a) {
+  const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  unsigned long long v = 0, excl;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    const int n = bin_total(a, base + k);
+    if (base + k < a.nbins) a.count[base + k] = n;
+    v += bin_sums(a, n);
+  }
+  const unsigned long long total = block_exclusive_scan64(v, excl);
+  if (threadIdx.x == 0) a.partial[blockIdx.x] = total;
+}
+
+// ONE: the only block, which also sums the counters.
+template <bool ONE>
+__global__ void __launch_bounds__(kScanThreads) k_bin_scan(BinScanArgs a) {
+  const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  int n[kScanItems];
+  unsigned long long v = 0, excl, first = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    const int b = base + k;
+    n[k] = ONE ? bin_total(a, b) : (b < a.nbins ? a.count[b] : 0);
+    if (ONE && b < a.nbins) a.count[b] = n[k];
+    v += bin_sums(a, n[k]);
+  }
+  if (!ONE) {  // the blocks before this one
+    unsigned long long w = 0, unused;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) w += a.partial[k];
+    first = block_exclusive_scan64(w, unused);
+  }
+  const unsigned long long total = block_exclusive_scan64(v, excl) + first;
+  excl += first;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    const int b = base + k;
+    if (b < a.nbins) {
+      a.start[b] = (int)(unsigned)excl;
+      a.sub_start[b] = (int)(excl >> 32);
+    }
+    excl += bin_sums(a, n[k]);
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    a.start[a.nbins] = (int)(unsigned)total;
+    a.sub_start[a.nbins] = (int)(total >> 32);
+  }
+}
+
+int bin_scan_partials(int nbins) { return (nbins + kScanTile - 1) / kScanTile; }
+
+cudaError_t launch_bin_scan(const BinScanArgs& a, cudaStream_t s) {
+  const int nb = bin_scan_partials(a.nbins);
+  if (nb < 1) return cudaErrorInvalidValue;
+  if (nb == 1) {
+    k_bin_scan<true><<<1, kScanThreads, 0, s>>>(a);
+  } else {
+    k_bin_sums<<<nb, kScanThreads, 0, s>>>(a);
+    k_bin_scan<false><<<nb, kScanThreads, 0, s>>>(a);
+  }
+  return cudaGetLastError();
+}
+
 __global__ void k_classify_subproblems(SubClassArgs a) {
+  const int total = a.sub_total[0];
   for (int sidx = blockIdx.x * blockDim.x + threadIdx.x; sidx < a.nsub; sidx += gridDim.x * blockDim.x) {
+    if (sidx >= total) {  // past the last subproblem, inside the launch bound
+      a.dense[sidx] = 0;
+      if (a.ndense) a.ndense[sidx] = 0;
+      continue;
+    }
     const int b = a.sub_to_bin[sidx];
     const int p0 = a.start[b] + (sidx - a.sub_start[b]) * a.maxsub;
     const int lx = a.i0[0][p0] % a.bs[0];
@@ -467,79 +546,6 @@ cudaError_t launch_classify_subproblems(const SubClassArgs& a, cudaStream_t s) {
   int blocks = (a.nsub + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
   k_classify_subproblems<<<blocks, 256, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
-__global__ void k_sub_to_bin(const int* sub_start, int nbins, int nsub, int* sub_to_bin) {
-  for (int sidx = blockIdx.x * blockDim.x + threadIdx.x; sidx < nsub; sidx += gridDim.x * blockDim.x) {
-    // largest b with sub_start[b] <= sidx
-    int lo = 0, hi = nbins;  // invariant: sub_start[lo] <= sidx < sub_start[hi]
-    while (hi - lo > 1) {
-      int mid = (lo + hi) >> 1;
-      if (sub_start[mid] <= sidx) lo = mid;
-      else hi = mid;
-    }
-    sub_to_bin[sidx] = lo;
-  }
-}
-
-cudaError_t launch_sub_to_bin(const int* sub_start, int nbins, int nsub, int* sub_to_bin, cudaStream_t s) {
-  if (nsub <= 0) return cudaSuccess;
-  k_sub_to_bin<<<place_grid(nsub), kPlaceThreads, 0, s>>>(sub_start, nbins, nsub, sub_to_bin);
-  return cudaGetLastError();
-}
-
-struct SubHdrArgs {
-  const int *sub_start, *start, *count;
-  int nbins, nsub, maxsub;
-  int bs[3], nb[3];
-  int* sub_to_bin;
-  SubHdr* hdr;
-};
-
-// The same bin search as k_sub_to_bin, then the subproblem's point range
-// (subproblem js of bin b: points start[b] + js maxsub, at most maxsub of
-// them) and its tile origin (the bin's first cell).
-__global__ void k_sub_headers(SubHdrArgs a) {
-  for (int sidx = blockIdx.x * blockDim.x + threadIdx.x; sidx < a.nsub; sidx += gridDim.x * blockDim.x) {
-    int lo = 0, hi = a.nbins;
-    while (hi - lo > 1) {
-      int mid = (lo + hi) >> 1;
-      if (a.sub_start[mid] <= sidx) lo = mid;
-      else hi = mid;
-    }
-    const int b = lo;
-    a.sub_to_bin[sidx] = b;
-    const int js = sidx - a.sub_start[b];
-    SubHdr h;
-    h.p0 = a.start[b] + js * a.maxsub;
-    h.np = min(a.maxsub, a.count[b] - js * a.maxsub);
-    h.ox = (b % a.nb[0]) * a.bs[0];
-    h.oy = ((b / a.nb[0]) % a.nb[1]) * a.bs[1];
-    h.oz = (b / (a.nb[0] * a.nb[1])) * a.bs[2];
-    h.pad0 = h.pad1 = h.pad2 = 0;
-    a.hdr[sidx] = h;
-  }
-}
-
-cudaError_t launch_sub_headers(const int* sub_start, const int* start, const int* count, int nbins,
-                               int nsub, int maxsub, const int bs[3], const int nb[3], int* sub_to_bin,
-                               SubHdr* hdr, cudaStream_t s) {
-  if (nsub <= 0) return cudaSuccess;
-  SubHdrArgs a;
-  a.sub_start = sub_start;
-  a.start = start;
-  a.count = count;
-  a.nbins = nbins;
-  a.nsub = nsub;
-  a.maxsub = maxsub;
-  for (int k = 0; k < 3; ++k) {
-    a.bs[k] = bs[k];
-    a.nb[k] = nb[k];
-  }
-  a.sub_to_bin = sub_to_bin;
-  a.hdr = hdr;
-  k_sub_headers<<<place_grid(nsub), kPlaceThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 

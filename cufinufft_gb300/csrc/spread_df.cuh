@@ -125,6 +125,7 @@ k_spread_sm_slab_df(SpreadArgs<double> a, int PX, int nbuf) {
   if (threadIdx.x == 0) s_max = 0;
   if (!a.kc.horner) df_table_fill(s_tab, a.kc);
   const SubTile st = sub_tile_block<3, NS>(a.bins, blockIdx.x);  // synchronises
+  if (st.np <= 0) return;  // block-uniform
   const int PP = PX * st.TY;  // plane stride
   const int ncell = PP * st.TZ;
   float4* tile = reinterpret_cast<float4*>(smem_raw);
@@ -235,6 +236,7 @@ k_spread_sm_priv_df(SpreadArgs<double> a) {
   if (threadIdx.x == 0) s_max = 0;
   if (!a.kc.horner) df_table_fill(s_tab, a.kc);
   const SubTile st = sub_tile_block<2, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   const int PX = slab_pitch(st.TX, NS);
   const int ncell = PX * st.TY;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

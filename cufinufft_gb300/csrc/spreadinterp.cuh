@@ -95,14 +95,16 @@ __device__ __forceinline__ SubTile sub_tile_hdr(const BinTables& bt, int sub) {
   return s;
 }
 
-// sub_tile computed once per block (three integer divisions) and shared
-// through shared memory; PERSISTENT blocks (several subproblems each) first
-// wait until every thread is done with the previous one.
+// sub_tile once per block, from the header where there is one (three integer
+// divisions otherwise), shared through shared memory.  np is 0 for a launch's
+// surplus subproblems (the host launches with their upper bound).  PERSISTENT
+// blocks (several subproblems each) first wait until every thread is done with
+// the previous one.
 template <int DIM, int NS, bool PERSISTENT = false>
 __device__ __forceinline__ SubTile sub_tile_block(const BinTables& bt, int sub) {
   __shared__ SubTile s_tile;
   if (PERSISTENT) __syncthreads();
-  if (threadIdx.x == 0) s_tile = sub_tile<DIM, NS>(bt, sub);
+  if (threadIdx.x == 0) s_tile = bt.hdr ? sub_tile_hdr<DIM, NS>(bt, sub) : sub_tile<DIM, NS>(bt, sub);
   __syncthreads();
   return s_tile;
 }
@@ -378,6 +380,7 @@ k_spread_sm(SpreadArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tile = reinterpret_cast<C*>(smem_raw);
   const SubTile st = sub_tile_block<DIM, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   const int t = blockIdx.y;
   tile_zero<T>(tile, st.ntile);
   __syncthreads();
@@ -565,6 +568,7 @@ k_interp_sm(SpreadArgs<T> a, const __grid_constant__ CUtensorMap gmap, int tma) 
   C* tile = reinterpret_cast<C*>(tma ? smem_align128(smem_raw) : smem_raw);
   if (tma && threadIdx.x == 0) mbar_init(&tile_bar, 1);
   SubTile st = sub_tile_hdr<DIM, NS>(a.bins, blockIdx.x);  // loads in flight across the barrier
+  if (st.np <= 0) return;  // block-uniform
   if (tma) __syncthreads();                                 // the barrier's init before any wait on it
   if (tma) {  // the tile row widened as the tensor map's box is (bulk_tile_x)
     st.TX = bulk_tile_x<T>(st.TX);
@@ -645,7 +649,8 @@ k_interp_sm_df(SpreadArgs<double> a, const __grid_constant__ CUtensorMap gmap, i
   if (threadIdx.x == 0) s_max = 0;
   if (!a.kc.horner) df_table_fill(s_tab, a.kc);
   SubTile st = sub_tile_hdr<DIM, NS>(a.bins, blockIdx.x);
-  if (tma) __syncthreads();
+  if (st.np <= 0) return;  // block-uniform
+  __syncthreads();
   const int t = blockIdx.y;
   const C* src = a.fw_in + (size_t)t * a.g.Nf;
   const bool bulk = tma && tile_in_grid(st, a.g);
@@ -1081,6 +1086,7 @@ k_spread_sm_wc(SpreadArgs<T> a) {
   if (a.sub_dense && a.sub_dense[blockIdx.x]) return;  // cell-run layout: done by k_spread_sm_run
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SubTile st = sub_tile_block<DIM, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   T* re = reinterpret_cast<T*>(smem_raw);
   T* im = re + st.ntile;
   const int t = blockIdx.y;
@@ -1209,6 +1215,7 @@ k_spread_sm_slab(SpreadArgs<T> a, int split) {
   }
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SubTile st = sub_tile_block<3, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   if (first >= st.np) return;  // block-uniform
   const int PX = slab_pitch(st.TX, NS);
   const int PP = PX * st.TY;                  // plane stride
@@ -1340,6 +1347,7 @@ k_spread_sm_priv(SpreadArgs<T> a, int split) {
   }
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SubTile st = sub_tile_block<2, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   if (first >= st.np) return;  // block-uniform
   const int PX = slab_pitch(st.TX, NS);
   const int ncell = PX * st.TY;
@@ -1709,6 +1717,7 @@ k_spread_sm_run(SpreadArgs<T> a, int split) {
   if (a.sub_dense && !a.sub_dense[blockIdx.x]) return;  // sparse: done by k_spread_sm_wc / slab
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SubTile st = sub_tile_block<DIM, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   const int nd = a.sub_ndense ? a.sub_ndense[blockIdx.x] : 0;  // leading dense points
   if (split) st.np = nd;  // the rest: k_spread_sm_slab
   T* re = reinterpret_cast<T*>(smem_raw);
@@ -1773,6 +1782,7 @@ k_spread_sm_run_tc(SpreadArgs<float> a) {
   __shared__ unsigned tmem_base;
   __shared__ int s_n, s_key;
   const SubTile st = sub_tile_block<3, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   float* A_hi = reinterpret_cast<float*>(smem_raw);
   float* A_lo = A_hi + (kTcK / 8) * 1024;
   float* B_hi = A_lo + (kTcK / 8) * 1024;
@@ -1954,6 +1964,7 @@ k_interp_sm_wc(SpreadArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tile = reinterpret_cast<C*>(smem_raw);
   const SubTile st = sub_tile_block<DIM, NS>(a.bins, blockIdx.x);
+  if (st.np <= 0) return;  // block-uniform
   const int t = blockIdx.y;
   tile_load<T>(tile, a.fw_in + (size_t)t * a.g.Nf, st, a.g);
   __syncthreads();
