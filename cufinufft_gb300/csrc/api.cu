@@ -1091,8 +1091,9 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   a.rank = p->rank;
   a.start = p->start;
   if (p->M == 0) return 0;
-  const int ms = p->method == 2 ? p->opts.gpu_maxsubprobsize : 0;
-  int e = bank_order(p, p->method, p->bs, p->nbins, &a.bank, p->cell_order);  // zeroes its counters
+  const int method = p->tile_m1 ? 2 : p->method;
+  const int ms = method == 2 ? p->opts.gpu_maxsubprobsize : 0;
+  int e = bank_order(p, method, p->bs, p->nbins, &a.bank, p->cell_order);  // zeroes its counters
   if (e) return e;
   BinScanArgs sc;
   std::memset(&sc, 0, sizeof(sc));
@@ -1184,6 +1185,29 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   return 0;
 }
 
+// Method 1 (the default of type 2) gathers every tap from L1 and L2, eight
+// or sixteen lanes to a point; from some density on, the subproblem kernel of
+// method 2 over the same bins is faster, its tile loaded once for all its
+// points: 2D and 3D, sorted points, a layout that the caller left alone.
+// Measured gather / tile times (us) by mean points per bin, default bins:
+//   FP32 tol 1e-6 2D: 31: 19.9 / 19.3, 123: 55.9 / 24.1 (1024^2); small calls
+//     123: 9.0 / 8.3 (256^2); tol 1e-3 123: 7.4 / 8.2 (256^2), 26.9 / 19.1
+//   FP32 tol 1e-6 3D: 15: 177 / 129, 59: 627 / 193 (96^3); tol 1e-3 58: 37 / 27
+//   FP64 tol 1e-9: 8: 101 / 213, 31: 353 / 223 (1024^2); 15: 702 / 494, 58:
+//     2724 / 632 (60^3); tol 1e-12 3D 14: 1051 / 1363, 58: 4092 / 1475
+// so FP32 takes the tile from 100 points per bin in 2D and 48 in 3D (the sort's
+// bank classes cost a little more than plain bins), FP64 from 28.
+template <typename T>
+static bool route_tiles(const Plan<T>* p) {
+  if (p->type != 2 || p->dim < 2 || p->method != 1 || !p->sort || p->auto_method || p->layout_set || p->variant != 0)
+    return false;
+  if (!is_single<T>() && !p->fp64_df) return false;
+  if (p->opts.gpu_maxsubprobsize < 256) return false;
+  if (tile_cells(p->dim, p->sp.ns, p->bs) * sizeof(cplx_t<T>) + 4096 > (size_t)max_smem_optin(p->device)) return false;
+  const int least = is_single<T>() ? (p->dim == 2 ? 100 : 48) : 28;
+  return (long long)p->M >= (long long)least * p->nbins;
+}
+
 // The part of setpts that FP32, FP64 and chained plans share: `a` says where
 // the points come from (their source, coordinates and axis maps).
 template <typename T>
@@ -1199,6 +1223,7 @@ static int setpts_from(Plan<T>* p, int M, PlaceArgs<T> a) {
   a.M = M;
   e = choose_layout(p, a);  // gpu_method 0: before the sort, from the points' occupancy
   if (e) return e;
+  p->tile_m1 = route_tiles(p);
   a.idx = p->idx;
   for (int k = 0; k < 3; ++k) {
     a.i0[k] = p->i0[k];
@@ -1882,7 +1907,7 @@ static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
   info->binsizey = p->bs[1];
   info->binsizez = p->bs[2];
   info->nbins = p->nbins;
-  info->nsubprob = p->nsub;
+  info->nsubprob = p->method == 2 ? p->nsub : 0;
   info->kerevalmeth = p->opts.gpu_kerevalmeth;
   info->beta = p->sp.beta;
   info->es_c = p->sp.c;
@@ -1932,6 +1957,7 @@ static int adopt_layout(Plan<T>* p, int method, const int bsz[3], int maxsub) {
   const int e = alloc_bins(p, (int)nbins);
   if (e) return e;
   p->method = method;
+  p->tile_m1 = false;
   p->cell_order = cell;
   p->sort = 1;
   p->opts.gpu_method = cell ? 5 : method;
@@ -1960,6 +1986,7 @@ static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub)
   ++p->version;  // the sorted arrays and bin tables are about to move
   int e = adopt_layout(p, method, bsz, maxsub);
   if (e) return e;
+  p->layout_set = true;
   if (!p->pts_set || p->M == 0) return 0;
   // fresh arrays for the re-sorted points
   PlaceArgs<T> a;

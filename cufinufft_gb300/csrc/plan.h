@@ -28,6 +28,8 @@ template <typename T> struct Plan {
                    // (layout method 5 = method 2 with cell_order, see set_layout)
   int variant = 0; // kernel family: 0 default, 1 one thread per point, 2 warp-cooperative
   bool auto_method = false;  // gpu_method 0: chosen by the library
+  bool layout_set = false;   // set_layout / autotune: the layout is the caller's
+  bool tile_m1 = false;      // method 1 interpolation on the tile kernels (route_tiles)
   int sort = 1;
   int bs[3] = {1, 1, 1}, nb[3] = {1, 1, 1};
   int nbins = 1;
@@ -267,10 +269,11 @@ inline cudaError_t run_spread(Plan<T>* p, const SpreadArgs<T>& a) {
 
 template <typename T>
 inline cudaError_t run_interp(Plan<T>* p, const SpreadArgs<T>& a) {
+  const int method = p->tile_m1 ? 2 : p->method;
   switch (p->dim) {
-    case 1: return interp_dim<T, 1>(p->method, p->sp.ns, a, p->stream);
-    case 2: return interp_dim<T, 2>(p->method, p->sp.ns, a, p->stream);
-    default: return interp_dim<T, 3>(p->method, p->sp.ns, a, p->stream);
+    case 1: return interp_dim<T, 1>(method, p->sp.ns, a, p->stream);
+    case 2: return interp_dim<T, 2>(method, p->sp.ns, a, p->stream);
+    default: return interp_dim<T, 3>(method, p->sp.ns, a, p->stream);
   }
 }
 
