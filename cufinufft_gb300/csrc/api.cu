@@ -162,14 +162,10 @@ template <typename T> static void release(Plan<T>* p) {
   cudaFree(p->horner_d);
   p->horner_d = nullptr;
   free_points(p);
-  cudaFree(p->count);
-  cudaFree(p->start);
-  cudaFree(p->sub_start);
-  cudaFree(p->scan_part);
-  p->scan_part = nullptr;
   cudaFree(p->raw);
   p->raw = nullptr;
-  p->cap_bins = p->cap_raw = 0;
+  p->scan_part = nullptr;
+  p->cap_bins = 0;
   cudaFree(p->sub_to_bin);
   cudaFree(p->sub_hdr);
   p->sub_hdr = nullptr;
@@ -690,31 +686,24 @@ static int set_width_rule(int rule, int* previous) {
   return 0;
 }
 
-// Bin tables for nbins bins, kept while they are large enough.
+// Bin tables for nbins bins (one allocation), kept while it is large enough.
 template <typename T>
 static int alloc_bins(Plan<T>* p, int nbins) {
-  if ((size_t)nbins > p->cap_bins) {
-    cudaFree(p->count);
-    cudaFree(p->start);
-    cudaFree(p->sub_start);
-    cudaFree(p->scan_part);
-    p->count = p->start = p->sub_start = nullptr;
-    p->scan_part = nullptr;
-    p->cap_bins = 0;
-    CFG_CUDA(cudaMalloc(&p->count, sizeof(int) * (size_t)nbins));
-    CFG_CUDA(cudaMalloc(&p->start, sizeof(int) * ((size_t)nbins + 1)));
-    CFG_CUDA(cudaMalloc(&p->sub_start, sizeof(int) * ((size_t)nbins + 1)));
-    CFG_CUDA(cudaMalloc(&p->scan_part, sizeof(unsigned long long) * (size_t)bin_scan_partials(nbins)));
-    p->cap_bins = nbins;
-  }
-  const size_t raw = nbins <= kCountStrideBins ? (size_t)nbins * kCountStride : 0;
-  if (raw > p->cap_raw) {
+  const size_t n = (size_t)nbins;
+  const size_t raw = nbins <= kCountStrideBins ? n * kCountStride : 0;
+  const size_t part = 2 * (size_t)bin_scan_partials(nbins);  // ints of the 64-bit block sums
+  const size_t ints = raw + part + n + 2 * (n + 1);
+  if (ints > p->cap_bins) {
     cudaFree(p->raw);
     p->raw = nullptr;
-    p->cap_raw = 0;
-    CFG_CUDA(cudaMalloc(&p->raw, sizeof(int) * raw));
-    p->cap_raw = raw;
+    p->cap_bins = 0;
+    CFG_CUDA(cudaMalloc(&p->raw, sizeof(int) * ints));
+    p->cap_bins = ints;
   }
+  p->scan_part = reinterpret_cast<unsigned long long*>(p->raw + raw);
+  p->count = p->raw + raw + part;
+  p->start = p->count + n;
+  p->sub_start = p->start + n + 1;
   return 0;
 }
 
@@ -973,8 +962,12 @@ template <typename T>
 static int bank_order(Plan<T>* p, int method, const int bs[3], int nbins, BankOrder* o,
                       bool cell = false) {
   std::memset(o, 0, sizeof(*o));
-  if (method != 2) return 0;
-  if (cell) {
+  // 1D spreading sums neighbouring points in registers: sorted by cell where
+  // cells hold points to share (half a point each on average), plain bins below
+  const bool by_cell = !cell && p->type == 1 && p->dim == 1 && p->variant == 0 && 2LL * p->M >= p->nf[0] &&
+                       (long long)nbins * bs[0] <= (1LL << 24);
+  if (method != 2 && !by_cell) return 0;
+  if (cell || by_cell) {
     int cells = 1;
     for (int k = 0; k < p->dim; ++k) cells *= bs[k];
     const size_t n = (size_t)nbins * cells;
@@ -994,7 +987,7 @@ static int bank_order(Plan<T>* p, int method, const int bs[3], int nbins, BankOr
       CFG_CUDA(cudaMalloc(&p->cls_tmp, sizeof(int) * (size_t)scan_tmp_ints((int)n)));
       p->cap_cls_start = n;
     }
-    if ((size_t)nbins > p->cap_sparse) {
+    if (cell && (size_t)nbins > p->cap_sparse) {
       cudaFree(p->sparse_count);
       p->sparse_count = nullptr;
       p->cap_sparse = 0;
@@ -1002,10 +995,10 @@ static int bank_order(Plan<T>* p, int method, const int bs[3], int nbins, BankOr
       p->cap_sparse = nbins;
     }
     CFG_CUDA(cudaMemsetAsync(p->cls_count, 0, sizeof(int) * n, p->stream));
-    CFG_CUDA(cudaMemsetAsync(p->sparse_count, 0, sizeof(int) * (size_t)nbins, p->stream));
+    if (cell) CFG_CUDA(cudaMemsetAsync(p->sparse_count, 0, sizeof(int) * (size_t)nbins, p->stream));
     o->cls_count = p->cls_count;
     o->ncls = cells;
-    o->cell_order = 1;
+    o->cell_order = cell ? 1 : 2;
     o->cls_start = p->cls_start;
     o->sparse_count = p->sparse_count;
     o->dense_min = dense_run(p->dim);
@@ -1099,7 +1092,10 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   std::memset(&sc, 0, sizeof(sc));
   sc.raw = p->count;
   sc.raw_stride = sc.per = 1;
-  if (a.bank.cls_count && !a.bank.cell_order) {
+  if (a.bank.cell_order == 2) {
+    sc.cell_start = p->cls_start;
+    sc.ncell = a.bank.ncls;
+  } else if (a.bank.cls_count && !a.bank.cell_order) {
     sc.raw = a.bank.cls_count;
     sc.raw_stride = sc.per = a.bank.ncls;
   } else if (!a.bank.cls_count && p->nbins <= kCountStrideBins) {
@@ -1108,7 +1104,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   }
   a.raw = const_cast<int*>(sc.raw);
   a.raw_stride = sc.raw_stride;
-  if (!a.bank.cls_count || a.bank.cell_order)
+  if (!a.bank.cls_count || a.bank.cell_order == 1)
     CFG_CUDA(cudaMemsetAsync(a.raw, 0, sizeof(int) * (size_t)p->nbins * sc.raw_stride, p->stream));
   sc.nbins = p->nbins;
   sc.maxsub = ms;
@@ -1117,10 +1113,10 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   sc.sub_start = p->sub_start;
   sc.partial = p->scan_part;
   CFG_CUDA(launch_bin_count<T>(a, p->stream));
-  CFG_CUDA(launch_bin_scan(sc, p->stream));
   if (a.bank.cell_order)
-    CFG_CUDA(launch_scan(p->cls_count, p->cls_start, p->nbins * a.bank.ncls, 2, dense_run(p->dim), p->cls_tmp,
-                         p->stream));
+    CFG_CUDA(launch_scan(p->cls_count, p->cls_start, p->nbins * a.bank.ncls, a.bank.cell_order == 1 ? 2 : 0,
+                         dense_run(p->dim), p->cls_tmp, p->stream));
+  CFG_CUDA(launch_bin_scan(sc, p->stream));
   SubHdrArgs h;
   std::memset(&h, 0, sizeof(h));
   if (ms > 0) {

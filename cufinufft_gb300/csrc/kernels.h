@@ -28,6 +28,8 @@ cudaError_t interp_dim(int method, int ns, const SpreadArgs<T>& a, cudaStream_t 
 // at least dense_min points first, sorted by cell, then the others in arbitrary
 // order; cls_start is the exclusive scan of those dense counts over all
 // (bin, cell) keys, sparse_count a per-bin counter for the others.
+// cell_order = 2 sorts every point by cell (1D type 1, whose spread sums
+// neighbouring points in registers): cls_start scans all counts.
 // Points on one cell that make it dense for the cell-run spread: a run must
 // amortise the flush of ns^d tap sums, 36 in 2D at ns = 6, 343 in 3D at 7.
 constexpr int dense_run(int dim) { return dim == 3 ? 16 : 8; }
@@ -91,6 +93,8 @@ struct SubHdrArgs {
 struct BinScanArgs {
   const int* raw;
   int raw_stride, per, nbins, maxsub;
+  const int* cell_start;  // cell_order 2: scanned cell counts (ncell per bin) instead of raw
+  int ncell;
   int *count, *start, *sub_start;
   unsigned long long* partial;
 };

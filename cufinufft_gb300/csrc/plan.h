@@ -70,8 +70,9 @@ template <typename T> struct Plan {
   int* start = nullptr;
   int* sub_start = nullptr;
   unsigned long long* scan_part = nullptr;  // block sums of the bin scan
-  int* raw = nullptr;          // sector-strided bin counters (kCountStride), small nbins
-  size_t cap_bins = 0, cap_raw = 0;
+  int* raw = nullptr;          // the allocation: sector-strided counters (kCountStride, small
+                               // nbins), block sums, count, start, sub_start
+  size_t cap_bins = 0;         // its ints
   int* sub_to_bin = nullptr;
   SubHdr* sub_hdr = nullptr;  // [cap_sub] subproblem headers
   size_t cap_sub = 0;

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kPlaceThreads) k_bin_count(PlaceArgs<T> a) {
     const int b = point_bin<T, SRC>(a, i, i0, d, lc);
     int r;
     if (a.bank.cls_count) {
-      if (a.bank.cell_order) agg_rank(act, b, &a.count[b]);
+      if (a.bank.cell_order == 1) agg_rank(act, b, &a.count[b]);
       const int key = b * a.bank.ncls + order_class(a.bank, a.bs, lc);
       r = agg_rank(act, key, a.bank.cls_count + key);
     } else {
@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a, SubHd
     const int r = a.rank[i];
     int pos;
     if (!a.bank.cls_count) pos = a.start[b] + r;
+    else if (a.bank.cell_order == 2) pos = a.bank.cls_start[(long long)b * a.bank.ncls + order_class(a.bank, a.bs, lc)] + r;
     else if (a.bank.cell_order) pos = cell_position(a.bank, a.start, act, b, order_class(a.bank, a.bs, lc), r);
     else pos = a.start[b] + interleave_pos(a.bank, b, order_class(a.bank, a.bs, lc), r);
     a.idx[pos] = SRC == kSrcStored ? a.src_idx[i] : i;
@@ -439,6 +440,7 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned lo
 
 __device__ __forceinline__ int bin_total(const BinScanArgs& a, int b) {
   if (b >= a.nbins) return 0;
+  if (a.cell_start) return a.cell_start[(size_t)(b + 1) * a.ncell] - a.cell_start[(size_t)b * a.ncell];
   const int* c = a.raw + (size_t)b * a.raw_stride;
   int n = 0;
   if ((a.per & 3) == 0) {  // classes: 8 or 16 counters, 16-byte aligned

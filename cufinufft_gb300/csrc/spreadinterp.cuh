@@ -1476,6 +1476,7 @@ k_spread_sm_priv(SpreadArgs<T> a, int split) {
 
 }  // namespace cfg
 #include "spread_df.cuh"
+#include "spread_win.cuh"
 namespace cfg {
 
 // CUFINUFFT_SPREAD_PRIV=0: 2D subproblem spreading by the warp-cooperative
@@ -2044,10 +2045,10 @@ inline bool tc_spread_enabled() {
 }
 
 // Kernel family per stage (SpreadArgs::variant 0 = the measured default):
-// spreading is warp-cooperative for method 1; for method 2 it is the
-// slab-owned kernel in 3D and the private-tile kernel in 2D (the
-// warp-cooperative atomic kernel in 1D, and wherever their shared memory does
-// not fit), with the cell-run kernel on dense prefixes of the cell-run
+// spreading in 1D keeps windows of sums in registers (spread_win.cuh); in 2D
+// and 3D it is warp-cooperative for method 1, and for method 2 the slab-owned
+// kernel in 3D and the private-tile kernel in 2D (the warp-cooperative atomic
+// kernel wherever their shared memory does not fit), with the cell-run kernel on dense prefixes of the cell-run
 // layout; interpolation is warp-cooperative for method 1 and
 // one-thread-per-point for method 2 (double-float for FP64 plans at
 // tol >= 1e-13).  variant 1 forces one thread per point, 2 forces
@@ -2056,6 +2057,10 @@ template <typename T, int DIM, int NS>
 cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
   const bool wc = a.variant != 1;
+  if constexpr (DIM == 1) {
+    // 1D: windows in registers whatever the layout (it only orders the points)
+    if (a.variant == 0 && (sizeof(T) == 4 || a.fp64_df == 1)) return launch_spread_win<T, NS>(a, s);
+  }
   if (method == 1) {
     if (wc) {
       constexpr int PPW = 32 / spread_lanes<NS>();
