@@ -148,10 +148,8 @@ template <typename T> static void release(Plan<T>* p) {
   }
   p->line_fft = false;
   p->half_fft = false;
-  p->df_fft = false;
-  cudaFree(p->df_tmp);
-  p->df_tmp = nullptr;
-  for (int k = 0; k < 2; ++k) {
+  p->df_fft = p->line_df = false;
+  for (int k = 0; k < 4; ++k) {
     cudaFree(p->df_tw[k]);
     p->df_tw[k] = nullptr;
   }
@@ -252,55 +250,61 @@ static bool use_half_fft(const Plan<T>* p) {
   return true;
 }
 
-// Double-float FFT (fft_df.cu) for FP64 plans of dimension 2 whose fine
-// grid sides are powers of two <= 4096, when the tol gate allows it and no
-// other FFT form was asked for.
+// Double-float line FFTs (fft_df.cu) for FP64 plans, when the tol gate allows
+// it and no other FFT form was asked for: every axis up to 4096 points, or a 1D
+// grid that splits into two such factors.  Below upsampfac 2, where the
+// deconvolution amplifies the grid's rounding, only 2D power-of-two grids.
+static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
 template <typename T>
-static bool use_df_fft(const Plan<T>* p) {
-  if (sizeof(T) != 8 || !p->df_fft_ok || p->dim != 2 || (p->type != 1 && p->type != 2)) return false;
+static bool use_line_df(Plan<T>* p) {
+  if (sizeof(T) != 8 || !p->df_fft_ok || (p->type != 1 && p->type != 2)) return false;
   if (std::getenv("CUFINUFFT_FFT")) return false;  // line / half forms asked for
-  return fft_df_size_ok(p->nf[0]) && fft_df_size_ok(p->nf[1]);
+  const int cap = fft_df_cap();
+  const bool pow2 = p->dim == 2 && power_of_two(p->nf[0]) && power_of_two(p->nf[1]);
+  if (p->opts.upsampfac < 2.0 && !pow2) return false;
+  p->fold[0] = p->fold[1] = 0;
+  if (p->dim == 1 && p->nf[0] > cap) {
+    // the factor pair nearest to square
+    for (int a = (int)std::sqrt((double)p->nf[0]); a >= 2; --a)
+      if (p->nf[0] % a == 0) {
+        const int b = p->nf[0] / a;
+        if (b > cap || radix_plan(a).empty() || radix_plan(b).empty()) return false;
+        p->fold[0] = b;
+        p->fold[1] = a;
+        break;
+      }
+    return p->fold[0] > 0;
+  }
+  for (int k = 0; k < p->dim; ++k) {
+    const std::vector<int> r = radix_plan(p->nf[k]);
+    if (p->nf[k] > cap || r.empty() || r.size() > 24) return false;
+  }
+  p->df_fft = pow2;
+  return true;
 }
 
-// Its scratch grids and, per axis, W^k = exp(iflag 2 pi i k / nf), k < nf/2,
-// computed in extended precision and split into float pairs.
-template <typename T>
-static int make_df_fft(Plan<T>* p) {
-  const long double two_pi = 6.283185307179586476925286766559005768L;
-  const size_t Nf = (size_t)p->nf[0] * p->nf[1];
-  CFG_CUDA(cudaMalloc(&p->df_tmp, sizeof(double2) * Nf * p->maxbatch));
-  for (int k = 0; k < 2; ++k) {
-    const int n = p->nf[k];
-    std::vector<float4> h((size_t)n / 2);
-    for (int m = 0; m < n / 2; ++m) {
-      const long double a = two_pi * (long double)m / (long double)n * (p->iflag >= 0 ? 1 : -1);
-      const double re = (double)cosl(a), im = (double)sinl(a);
-      const float rh = (float)re, ih = (float)im;
-      h[m] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
-    }
-    CFG_CUDA(cudaMalloc(&p->df_tw[k], sizeof(float4) * h.size()));
-    CFG_CUDA(cudaMemcpyAsync(p->df_tw[k], h.data(), sizeof(float4) * h.size(), cudaMemcpyHostToDevice,
-                             p->stream));
-  }
-  CFG_CUDA(cudaStreamSynchronize(p->stream));
+// exp(iflag 2 pi i step m / n), m < count, as float pairs.
+static int df_twiddles(float4** out, int iflag, long long n, long long step, int count, cudaStream_t s) {
+  CFG_CUDA(cudaMalloc(out, sizeof(float4) * (size_t)count));
+  CFG_CUDA(launch_df_twiddles(*out, iflag >= 0 ? 1 : -1, n, step, count, s));
   return 0;
 }
 
-// 2D transform of B grids in -> out through the scratch: rows along x, a
-// transpose, rows along y, a transpose back.  in may equal out (type 1).
 template <typename T>
-static cudaError_t df_fft_exec(Plan<T>* p, const cplx_t<T>* in, cplx_t<T>* out, int B) {
-  if constexpr (sizeof(T) == 8) {
-    const int nx = p->nf[0], ny = p->nf[1];
-    cudaError_t e = launch_fft_df_rows(in, p->df_tmp, nx, (long long)B * ny, p->df_tw[0], p->stream);
-    if (e == cudaSuccess) e = launch_transpose_d2(p->df_tmp, out, ny, nx, B, p->stream);
-    if (e == cudaSuccess) e = launch_fft_df_rows(out, p->df_tmp, ny, (long long)B * nx, p->df_tw[1], p->stream);
-    if (e == cudaSuccess) e = launch_transpose_d2(p->df_tmp, out, nx, ny, B, p->stream);
-    return e;
+static int make_line_df(Plan<T>* p) {
+  int e = 0;
+  if (p->fold[0]) {
+    const long long L = p->nf[0];
+    if ((e = df_twiddles(&p->df_tw[0], p->iflag, p->fold[0], 1, p->fold[0], p->stream))) return e;
+    if ((e = df_twiddles(&p->df_tw[1], p->iflag, p->fold[1], 1, p->fold[1], p->stream))) return e;
+    if ((e = df_twiddles(&p->df_tw[2], p->iflag, L, 1024, (int)((L + 1023) / 1024), p->stream))) return e;
+    if ((e = df_twiddles(&p->df_tw[3], p->iflag, L, 1, 1024, p->stream))) return e;
   } else {
-    (void)p; (void)in; (void)out; (void)B;
-    return cudaErrorInvalidValue;
+    for (int k = 0; k < p->dim; ++k)
+      if ((e = df_twiddles(&p->df_tw[k], p->iflag, p->nf[k], 1, p->nf[k], p->stream))) return e;
   }
+  p->line_df = true;
+  return 0;
 }
 
 // Twiddle tables W^m = exp(iflag 2 pi i m / nf_d), m < nf_d, per axis, in
@@ -665,6 +669,74 @@ static std::vector<LineArgs<T>> line_passes(const Plan<T>* p, cplx_t<T>* fk, int
   return v;
 }
 
+// The same passes in double-float: the axis each pass runs along gives its
+// twiddles; a long 1D transform is its columns and rows.
+template <typename T>
+static std::vector<LineDfArgs> line_df_passes(const Plan<T>* p, cplx_t<T>* fk, int B) {
+  std::vector<LineDfArgs> v;
+  if constexpr (sizeof(T) == 8) {
+    auto radices = [](LineArgs<double>& a) {
+      const std::vector<int> r = radix_plan(a.L);
+      a.nrad = (int)r.size();
+      for (int s = 0; s < a.nrad; ++s) a.rad[s] = r[s];
+      a.p2 = 0;
+    };
+    if (p->fold[0]) {
+      const long long L = p->nf[0], N = p->N[0];
+      const bool t2 = p->type == 2;
+      LineDfArgs c, r;
+      std::memset(&c, 0, sizeof(c));
+      c.a.L = p->fold[0];
+      c.a.nlines = p->fold[1];
+      c.a.dir = p->iflag;
+      c.a.ntr = B;
+      c.a.A = 1;
+      c.Lfull = (int)L;
+      c.tw_hi = p->df_tw[2];
+      c.tw_lo = p->df_tw[3];
+      r = c;
+      c.fold = 1;
+      c.in_across = c.out_across = 1;
+      c.tw = p->df_tw[0];
+      c.a.in = t2 ? fk : p->fw;
+      c.a.out = p->fw;
+      c.a.si = line_side(t2 ? N : L, 0, 0, 1, t2 ? 1 : 0, t2 ? (int)N : 0);
+      c.a.so = line_side(L, 0, 0, 1, 0, 0);
+      c.a.fp = t2 ? p->fac[0] : nullptr;
+      r.fold = 2;
+      r.a.L = p->fold[1];
+      r.a.nlines = p->fold[0];
+      r.out_across = 1;
+      r.tw = p->df_tw[1];
+      r.a.in = p->fw;
+      r.a.out = t2 ? p->fw2 : fk;
+      r.a.si = line_side(L, p->fold[1], 0, 1, 0, 0);
+      r.a.A = p->fold[0];
+      r.a.so = line_side(t2 ? L : N, 0, 0, 1, t2 ? 0 : 1, t2 ? 0 : (int)N);
+      r.a.fp = t2 ? nullptr : p->fac[0];
+      r.a.fac_on_out = t2 ? 0 : 1;
+      radices(c.a);
+      radices(r.a);
+      v.push_back(c);
+      v.push_back(r);
+      return v;
+    }
+    // line_passes: type 2 runs the slowest axis first, type 1 the fastest
+    const std::vector<LineArgs<double>> passes = line_passes(p, fk, B);
+    for (size_t i = 0; i < passes.size(); ++i) {
+      const int axis = p->type == 2 ? p->dim - 1 - (int)i : (int)i;
+      LineDfArgs d;
+      std::memset(&d, 0, sizeof(d));
+      d.a = passes[i];
+      radices(d.a);
+      d.in_across = d.out_across = axis > 0;
+      d.tw = p->df_tw[axis];
+      v.push_back(d);
+    }
+  }
+  return v;
+}
+
 static int max_smem_optin(int device);
 
 // Kernel-width rule of the next makeplan calls on this thread (-1: from
@@ -861,17 +933,12 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   CFG_CUDA(cudaMalloc(&p->fw, sizeof(cplx_t<T>) * (size_t)Nf * p->maxbatch));
   for (int k = 0; k < dim; ++k) CFG_CUDA(cudaMalloc(&p->fac[k], sizeof(T) * (size_t)p->N[k]));
 
-  if (use_df_fft(p)) {
-    // double-float FFT: no cuFFT plan; scratch for the passes, twiddles per axis
-    e = make_df_fft(p);
+  if (use_line_df(p)) {
+    // double-float line passes: no cuFFT plan, no padding to clear; a long 1D
+    // transform's second pass transposes, out of place for type 2
+    e = make_line_df(p);
     if (e) return e;
-    if (type == 2) {
-      // as with cuFFT: fw holds only the amplified modes over zero padding,
-      // the transform writes fw2, interpolation reads fw2
-      CFG_CUDA(cudaMalloc(&p->fw2, sizeof(cplx_t<T>) * (size_t)Nf * p->maxbatch));
-      CFG_CUDA(cudaMemsetAsync(p->fw, 0, sizeof(cplx_t<T>) * (size_t)Nf * p->maxbatch, p->stream));
-    }
-    p->df_fft = true;
+    if (type == 2 && p->fold[0]) CFG_CUDA(cudaMalloc(&p->fw2, sizeof(cplx_t<T>) * (size_t)Nf * p->maxbatch));
   } else if (use_half_fft(p)) {
     // pruned power-of-two passes: no cuFFT plan; type 2 grid in fw2
     // (intermediates in fw), type 1 intermediates in fw2
@@ -1363,6 +1430,12 @@ static int execute_direct(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
           if (i + 1 == passes.size()) mark(p, ev[2]);  // last pass: deconvolution fused
           CFG_CUDA(launch_half_pass<T>(passes[i], p->stream));
         }
+      } else if (p->line_df) {
+        const std::vector<LineDfArgs> passes = line_df_passes(p, fk + (size_t)b0 * Nm, B);
+        for (size_t i = 0; i < passes.size(); ++i) {
+          if (i + 1 == passes.size()) mark(p, ev[2]);  // last pass: deconvolution fused
+          CFG_CUDA(launch_line_fft_df(passes[i], p->stream));
+        }
       } else if (p->line_fft) {
         const std::vector<LineArgs<T>> passes = line_passes(p, fk + (size_t)b0 * Nm, B);
         for (size_t i = 0; i < passes.size(); ++i) {
@@ -1370,8 +1443,7 @@ static int execute_direct(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
           CFG_CUDA(launch_line_fft<T>(passes[i], p->stream));
         }
       } else {
-        if (p->df_fft) CFG_CUDA(df_fft_exec(p, p->fw, p->fw, B));
-        else CFG_CUFFT(fft_exec(h, p->fw, p->iflag));
+        CFG_CUFFT(fft_exec(h, p->fw, p->iflag));
         mark(p, ev[2]);
         CFG_CUDA(launch_deconvolve<T>(p->dim, p->nf, p->N, p->fw, fk + (size_t)b0 * Nm, p->fac[0],
                                       p->fac[1], p->fac[2], B, p->stream));
@@ -1381,6 +1453,13 @@ static int execute_direct(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
         const std::vector<HalfPass<T>> passes = half_passes(p, fk + (size_t)b0 * Nm, B);
         for (size_t i = 0; i < passes.size(); ++i) {
           CFG_CUDA(launch_half_pass<T>(passes[i], p->stream));
+          if (i == 0) mark(p, ev[1]);  // first pass: amplification fused
+        }
+        mark(p, ev[2]);
+      } else if (p->line_df) {
+        const std::vector<LineDfArgs> passes = line_df_passes(p, fk + (size_t)b0 * Nm, B);
+        for (size_t i = 0; i < passes.size(); ++i) {
+          CFG_CUDA(launch_line_fft_df(passes[i], p->stream));
           if (i == 0) mark(p, ev[1]);  // first pass: amplification fused
         }
         mark(p, ev[2]);
@@ -1395,8 +1474,7 @@ static int execute_direct(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
         CFG_CUDA(launch_amplify_modes<T>(p->dim, p->nf, p->N, p->fw, fk + (size_t)b0 * Nm, p->fac[0],
                                          p->fac[1], p->fac[2], B, p->stream));
         mark(p, ev[1]);
-        if (p->df_fft) CFG_CUDA(df_fft_exec(p, p->fw, p->fw2, B));
-        else CFG_CUFFT(fft_exec(h, p->fw, p->fw2, p->iflag));
+        CFG_CUFFT(fft_exec(h, p->fw, p->fw2, p->iflag));
         mark(p, ev[2]);
       }
       a.fw_in = p->fw2 ? p->fw2 : p->fw;

@@ -255,15 +255,23 @@ struct HalfPass {
 template <typename T> cudaError_t launch_half_pass(const HalfPass<T>& a, cudaStream_t s);
 bool half_fft_size_ok(int nf);
 
-// Double-float FFT of FP64 grids (fft_df.cu): 1D transforms of length n (a
-// power of two <= 4096) over `rows` consecutive rows, twiddles tw[k] =
-// exp(sign 2 pi i k / n), k < n/2, as float pairs (re hi, re lo, im hi,
-// im lo); and the batched transpose of R x C planes of double2.
-bool fft_df_size_ok(int n);
-size_t fft_df_smem(int n);
-cudaError_t launch_fft_df_rows(const double2* in, double2* out, int n, long long rows, const float4* tw,
-                               cudaStream_t s);
-cudaError_t launch_transpose_d2(const double2* in, double2* out, int R, int C, int batch, cudaStream_t s);
+// Line FFTs of FP64 grids in double-float (fft_df.cu): LineArgs with its line
+// grouping left to the launcher, twiddles tw[m] = exp(dir 2 pi i m / L), m < L,
+// as (re hi, im hi, re lo, im lo); in_across / out_across: adjacent lines are
+// adjacent in memory on that side (else positions are).  fold 1 / 2: the
+// columns / rows pass of a long 1D transform of Lfull = L nlines points, with
+// exp(dir 2 pi i 1024 a / Lfull) and exp(dir 2 pi i b / Lfull), b < 1024.
+struct LineDfArgs {
+  LineArgs<double> a;
+  const float4* tw;
+  int in_across, out_across, fold, Lfull;
+  const float4* tw_hi;
+  const float4* tw_lo;
+};
+int fft_df_cap();  // longest line
+cudaError_t launch_line_fft_df(LineDfArgs d, cudaStream_t s);
+// exp(dir 2 pi i step m / n), m < count, as float pairs.
+cudaError_t launch_df_twiddles(float4* out, int dir, long long n, long long step, int count, cudaStream_t s);
 int half_fft_mp(int nf);
 // Pitch of the column buffers of the strided passes for n values per column
 // and Mp-point transforms (at least both, bank-conflict offset added).

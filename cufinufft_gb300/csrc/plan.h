@@ -44,11 +44,14 @@ template <typename T> struct Plan {
   // exp(iflag 2 pi i m / nf_d) and radix sequences
   bool line_fft = false;
   bool half_fft = false;  // pruned power-of-two passes (halffft.cu), tables in tw
-  // FP64 2D grids: double-float FFT (fft_df.cu) instead of cuFFT's Z2Z
-  bool df_fft = false;
+  // FP64 grids: double-float line FFTs (fft_df.cu) instead of cuFFT's Z2Z;
+  // twiddles per axis as float pairs (a long 1D transform of fold[0] x fold[1]
+  // points: per pass, then the two tables of the step between)
+  bool line_df = false;
+  bool df_fft = false;          // line_df on a 2D power-of-two grid (plan info)
   int df_fft_ok = 0;            // set at makeplan: precision, tol and switch allow it
-  double2* df_tmp = nullptr;    // maxbatch grids of scratch
-  float4* df_tw[2] = {nullptr, nullptr};  // twiddles per axis (float pairs)
+  float4* df_tw[4] = {nullptr, nullptr, nullptr, nullptr};
+  int fold[2] = {0, 0};
   C* tw[3] = {nullptr, nullptr, nullptr};
   std::vector<int> rad[3];
   int rem = 0;

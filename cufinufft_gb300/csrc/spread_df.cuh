@@ -19,19 +19,6 @@
 
 namespace cfg {
 
-// (h + l) 2^k as double by widening h and l through their exponent fields (an
-// FP64 addition is left; conversions would take the same narrow unit).
-__device__ __forceinline__ double df_widen(float v, int k) {
-  const unsigned b = __float_as_uint(v);
-  const int ef = (int)((b >> 23) & 0xffu);
-  const int e = ef + 896 + k;
-  if (ef == 0xff) return __longlong_as_double(((long long)((b & 0x80000000u) | 0x7ff80000u)) << 32);
-  if (ef == 0 || e <= 0) return 0.0;  // below 2^-126 of the block's largest, or of FP64's range
-  const unsigned hi = e >= 2047 ? 0x7ff00000u : ((unsigned)e << 20) | ((b >> 3) & 0xfffffu);
-  const unsigned lo = e >= 2047 ? 0u : b << 29;
-  return __longlong_as_double(((long long)((b & 0x80000000u) | hi) << 32) | lo);
-}
-
 // The shift that brings the largest finite strength of the block's points to
 // [1, 2): high words compare as integers.  smax is zeroed and the block
 // synchronised before the call.
