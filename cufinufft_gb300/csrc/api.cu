@@ -214,12 +214,13 @@ static int make_fft(Plan<T>* p, int batch, cufftHandle* h) {
 // axis length is 2,3,5-smooth and fits one block's shared memory (8192 FP32
 // / 4096 FP64 points); otherwise the whole-grid cuFFT path runs.
 
-// Radices (8, 4, 2, 5, 3) whose product is L; empty if L has another factor.
-static std::vector<int> radix_plan(int L) {
+// Radices (8, 4, 2, 5, 3, up to `most`) whose product is L; empty if L has
+// another factor.
+static std::vector<int> radix_plan(int L, int most = 8) {
   std::vector<int> r;
   if (L < 2) return r;
   for (int R : {8, 4, 2, 5, 3})
-    while (L % R == 0) {
+    while (R <= most && L % R == 0) {
       r.push_back(R);
       L /= R;
     }
@@ -676,7 +677,7 @@ static std::vector<LineDfArgs> line_df_passes(const Plan<T>* p, cplx_t<T>* fk, i
   std::vector<LineDfArgs> v;
   if constexpr (sizeof(T) == 8) {
     auto radices = [](LineArgs<double>& a) {
-      const std::vector<int> r = radix_plan(a.L);
+      const std::vector<int> r = radix_plan(a.L, 5);  // fft_df.cu has no radix 8
       a.nrad = (int)r.size();
       for (int s = 0; s < a.nrad; ++s) a.rad[s] = r[s];
       a.p2 = 0;

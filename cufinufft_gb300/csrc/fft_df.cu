@@ -1,17 +1,16 @@
 // fft_df.cu -- line FFTs of FP64 grids in double-float arithmetic (FP32 pairs).
 //
-// cuFFT's Z2Z transform is bound by GB300's FP64 unit: a radix-8 butterfly is
-// ~10 FP64 instructions per value at a sixty-fourth of the FP32 rate, against
-// ~50 packed FP32 instructions here.  A d-dimensional transform is one pass
+// cuFFT's Z2Z transform is bound by GB300's FP64 unit: a butterfly level is
+// ~3 FP64 instructions per value at a sixty-fourth of the FP32 rate, against
+// ~18 packed FP32 instructions here.  A d-dimensional transform is one pass
 // per axis over only the lines and positions that carry modes (LineArgs,
 // linemap.cuh), with the amplification fused into the first pass of type 2 and
 // the deconvolution into the last of type 1: the zero padding is neither
 // written, read nor transformed.
 //
-// A block transforms G lines: every thread holds eight to ten values in
-// registers, Stockham passes of radix 8, 4, 2, 5, 3 exchange them through one
-// padded shared buffer (read all, wait, write all), the first pass loads from
-// global memory and the last stores to it.  Values travel as (re hi, im hi, re
+// A block transforms G lines in one padded shared buffer by Stockham passes of
+// radix 4, 2, 5, 3, every thread holding four to six values in registers
+// between reading and writing.  Values travel as (re hi, im hi, re
 // lo, im lo); the block scales its lines by the power of two that brings the
 // largest input to [1, 2), so any FP64 range passes.  Along y and z a block's G
 // lines are adjacent, so a row segment of G cells is contiguous.
@@ -20,8 +19,16 @@
 // of x[n1 L2 + n2], multiplied by W_L^(n2 k1), then rows k1, whose output k2
 // lands at k1 + L1 k2.
 //
-// Measured (FFT with amplification or deconvolution; cuFFT with the mode-row
-// kernel before): @@
+// Four values per thread and 64 registers (radix 4 at most) rather than eight
+// with radix 8 and 128: the chains are latency, and 32 warps per SM hide more of
+// it than one exchange less saves (256^3: 0.87 against 0.99 ms; 2048^2: 0.277
+// against 0.275).  What bounds it now: instruction issue and latency, 30-40% of
+// cycles issued; the FMA pipe would allow a quarter of the time.
+//
+// Measured (FFT with amplification or deconvolution; cuFFT, or the unpruned 2D
+// double-float form, with the mode-row kernel before): 2048^2 type 2 403 -> 277
+// us, 256^3 type 2 3.71 -> 0.87 ms, 150x192x162 type 1 1.03 -> 0.41 ms, 405000
+// points type 2 672 -> 89 us.
 #include <cuda_runtime.h>
 
 #include "df.cuh"
@@ -30,8 +37,8 @@
 namespace cfg {
 namespace {
 
-constexpr int kDfThreadsMax = 512;
-constexpr int kDfValues = 8;  // values per thread (radix 5: 10, radix 3: 9)
+constexpr int kDfThreadsMax = 1024;
+constexpr int kDfValues = 4;  // values per thread (radix 5: 5, radix 3: 6)
 
 using Z = DF2;  // a complex value: h = (re, im), l its low parts
 
@@ -80,26 +87,6 @@ template <> struct DftDf<4> {
     v[3] = zsub(d02, d13);
   }
 };
-template <> struct DftDf<8> {
-  static __device__ __forceinline__ void run(Z* v, float dir) {
-    CFG_DF_CONST(kH, 0.70710678118654752440);  // 1/sqrt(2)
-    Z e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    DftDf<4>::run(e, dir);
-    DftDf<4>::run(o, dir);
-    // o_m *= exp(dir 2 pi i m / 8): (1 + dir i)/sqrt(2), dir i, (-1 + dir i)/sqrt(2)
-    const Z w1 = zscale(zadd(o[1], zmul_i(o[1], dir)), kH_h, kH_l);
-    const Z w2 = zmul_i(o[2], dir);
-    const Z w3 = zscale(zsub(zmul_i(o[3], dir), o[3]), kH_h, kH_l);
-    v[0] = zadd(e[0], o[0]);
-    v[4] = zsub(e[0], o[0]);
-    v[1] = zadd(e[1], w1);
-    v[5] = zsub(e[1], w1);
-    v[2] = zadd(e[2], w2);
-    v[6] = zsub(e[2], w2);
-    v[3] = zadd(e[3], w3);
-    v[7] = zsub(e[3], w3);
-  }
-};
 template <> struct DftDf<3> {
   static __device__ __forceinline__ void run(Z* v, float dir) {
     CFG_DF_CONST(kS, 0.86602540378443864676);  // sin(2 pi / 3)
@@ -134,15 +121,6 @@ template <> struct DftDf<5> {
 // Shared slot of element i of a line: one spare 16-byte slot every eight (128
 // bytes) spreads the strided Stockham writes over the banks.
 __device__ __forceinline__ int df_slot(int i) { return i + (i >> 3); }
-
-struct DfCtx {
-  const LineDfArgs* d;
-  const double2* in;
-  double2* out;
-  float4* buf;
-  int line0, Lp, shift;
-  unsigned* smax;
-};
 
 // A line on one side: where position w of it lies, and the factor of its modes.
 struct DfLine {
@@ -181,164 +159,151 @@ __device__ __forceinline__ long long df_index(const LineDfArgs& d, const LineSid
   return l.base + (long long)(s.pmode == 1 ? *mode : w) * l.step;
 }
 
+// One Stockham pass of radix R over the block's G lines in shared memory:
+// every thread reads its butterflies, waits, and writes them back in order.
+// The first pass reads FP64 values and splits them.
 template <int R>
-__device__ __forceinline__ void df_pass(DfCtx& c, int Ns, bool first, bool last) {
+__device__ __forceinline__ void df_pass(const LineDfArgs& d, float4* buf, int Lp, int Ns, bool first, int shift) {
   constexpr int NB = (kDfValues + R - 1) / R;  // butterflies per thread
-  const LineDfArgs& d = *c.d;
-  const LineArgs<double>& a = d.a;
-  const int L = a.L, G = a.G, nbf = L / R, total = G * nbf;
+  const int L = d.a.L, nbf = L / R, total = d.a.G * nbf;
   const float inv_nbf = 1.f / (float)nbf, inv_Ns = 1.f / (float)Ns;
-  const float dir = (float)a.dir;
-  // lanes along adjacent lines where those are contiguous in memory
-  const bool across = (first && d.in_across) || (last && d.out_across);
+  const float dir = (float)d.a.dir;
   Z v[NB][R];
-  int gs[NB], js[NB];
+  int at[NB], js[NB];
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
     const int u = threadIdx.x + b * blockDim.x;
-    if (across) {
-      gs[b] = u & (G - 1);
-      js[b] = u >> a.log2G;
-    } else {
-      gs[b] = (int)(((float)u + 0.5f) * inv_nbf);
-      js[b] = u - gs[b] * nbf;
+    const int g = (int)(((float)u + 0.5f) * inv_nbf);
+    js[b] = u - g * nbf;
+    at[b] = g * Lp;
+    if (u >= total) {
+      at[b] = -1;
+      continue;
     }
-    if (u >= total) gs[b] = -1;
-  }
-  if (first) {
-    double2 raw[NB][R];
-    unsigned m = 0;
-    const bool folded = d.fold == 1, per_mode = !a.fac_on_out && a.fp != nullptr && a.si.pmode;
+    const float4* l = buf + at[b];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      const int line = c.line0 + gs[b];
-      const bool on = gs[b] >= 0 && line < a.nlines;
-      DfLine l;
-      if (on) l = df_line(d, a.si, line, folded, !a.fac_on_out);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        raw[b][r] = make_double2(0.0, 0.0);
-        if (!on) continue;
-        int mode;
-        const long long at = df_index(d, a.si, l, js[b] + r * nbf, folded, &mode);
-        if (at < 0) continue;
-        raw[b][r] = c.in[at];
-        if (per_mode) {
-          const double f = l.f * a.fp[mode];
-          raw[b][r].x *= f;
-          raw[b][r].y *= f;
-        }
-        const unsigned x = (unsigned)__double2hiint(raw[b][r].x) & 0x7fffffffu;
-        const unsigned y = (unsigned)__double2hiint(raw[b][r].y) & 0x7fffffffu;
-        if (x < 0x7ff00000u) m = max(m, x);
-        if (y < 0x7ff00000u) m = max(m, y);
-      }
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(c.smax, m);
-    __syncthreads();
-    c.shift = 1023 - (int)(*c.smax >> 20);
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const DF re = df_split(raw[b][r].x, c.shift), im = df_split(raw[b][r].y, c.shift);
+    for (int r = 0; r < R; ++r) {
+      const float4 x = l[df_slot(js[b] + r * nbf)];
+      if (first) {
+        const double2 y = make_double2(__hiloint2double(__float_as_int(x.y), __float_as_int(x.x)),
+                                       __hiloint2double(__float_as_int(x.w), __float_as_int(x.z)));
+        const DF re = df_split(y.x, shift), im = df_split(y.y, shift);
         v[b][r] = Z{make_float2(re.h, im.h), make_float2(re.l, im.l)};
-      }
-  } else {
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      if (gs[b] < 0) continue;
-      const float4* l = c.buf + gs[b] * c.Lp;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const float4 x = l[df_slot(js[b] + r * nbf)];
+      } else {
         v[b][r] = Z{make_float2(x.x, x.y), make_float2(x.z, x.w)};
       }
     }
-    __syncthreads();  // every read of this pass is done before any write
   }
+  __syncthreads();  // every read of this pass is done before any write
   const int tstep = L / (Ns * R);
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
-    if (gs[b] < 0) continue;
+    if (at[b] < 0) continue;
     const int q = (int)(((float)js[b] + 0.5f) * inv_Ns), k = js[b] - q * Ns;
-    if (Ns > 1) {
+    if (!first) {
 #pragma unroll
       for (int r = 1; r < R; ++r) v[b][r] = zmul(v[b][r], __ldg(d.tw + r * k * tstep));
     }
     DftDf<R>::run(v[b], dir);
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[b][r] = znorm(v[b][r]);
     const int base = q * Ns * R + k;
-    if (!last) {
-      float4* l = c.buf + gs[b] * c.Lp;
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        l[df_slot(base + r * Ns)] = make_float4(v[b][r].h.x, v[b][r].h.y, v[b][r].l.x, v[b][r].l.y);
-      continue;
-    }
-    const int line = c.line0 + gs[b];
-    if (line >= a.nlines) continue;
-    const bool folded = d.fold != 0, per_mode = a.fac_on_out && a.fp != nullptr && a.so.pmode;
-    const DfLine l = df_line(d, a.so, line, folded, a.fac_on_out != 0);
+    float4* l = buf + at[b];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int w = base + r * Ns;
-      int mode;
-      const long long at = df_index(d, a.so, l, w, folded, &mode);
-      if (at < 0) continue;
-      Z o = v[b][r];
-      if (d.fold == 1) {  // W_L^(line w) as W_L^(1024 a) W_L^b
-        const int m = line * w;
-        o = zmul(zmul(o, __ldg(d.tw_hi + (m >> 10))), __ldg(d.tw_lo + (m & 1023)));
-      }
-      double2 x = make_double2(df_widen(o.h.x, -c.shift) + df_widen(o.l.x, -c.shift),
-                               df_widen(o.h.y, -c.shift) + df_widen(o.l.y, -c.shift));
-      if (per_mode) {
-        const double f = l.f * a.fp[mode];
-        x.x *= f;
-        x.y *= f;
-      }
-      c.out[at] = x;
+      const Z o = znorm(v[b][r]);
+      l[df_slot(base + r * Ns)] = make_float4(o.h.x, o.h.y, o.l.x, o.l.y);
     }
   }
-  if (!last) __syncthreads();
+  __syncthreads();
 }
 
-// POW2: radices 8, 4, 2 only (fewer registers)
+// POW2: radices 4 and 2 only (fewer registers).  Load, passes and store each
+// go through shared memory: the index and factor arithmetic of the pruned lines
+// stays out of the butterflies, whose registers decide the occupancy.
 template <bool POW2>
 __global__ void __launch_bounds__(kDfThreadsMax, 1)
 k_line_fft_df(const __grid_constant__ LineDfArgs d) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_max;
-  DfCtx c;
-  c.d = &d;
-  c.buf = reinterpret_cast<float4*>(smem_raw);
-  c.line0 = blockIdx.x * d.a.G;
-  c.Lp = d.a.L + (d.a.L >> 3) + 1;
-  c.smax = &s_max;
-  for (int t = blockIdx.y; t < d.a.ntr; t += gridDim.y) {
-    c.in = d.a.in + (long long)t * d.a.si.st;
-    c.out = d.a.out + (long long)t * d.a.so.st;
-    __syncthreads();  // the previous transform's reads of s_max and the buffer
+  const LineArgs<double>& a = d.a;
+  float4* buf = reinterpret_cast<float4*>(smem_raw);
+  const int line0 = blockIdx.x * a.G, L = a.L, total = a.G * L, Lp = L + (L >> 3) + 1;
+  const float inv_L = 1.f / (float)L;
+  for (int t = blockIdx.y; t < a.ntr; t += gridDim.y) {
+    __syncthreads();  // the previous transform's reads
     if (threadIdx.x == 0) s_max = 0;
     __syncthreads();
+    unsigned m = 0;
+    {
+      const double2* in = a.in + (long long)t * a.si.st;
+      const bool folded = d.fold == 1, per_mode = !a.fac_on_out && a.fp != nullptr && a.si.pmode;
+#pragma unroll 4
+      for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        const int g = d.in_across ? e & (a.G - 1) : (int)(((float)e + 0.5f) * inv_L);
+        const int w = d.in_across ? e >> a.log2G : e - g * L;
+        double2 v = make_double2(0.0, 0.0);
+        if (line0 + g < a.nlines) {
+          const DfLine l = df_line(d, a.si, line0 + g, folded, per_mode);
+          int mode;
+          const long long at = df_index(d, a.si, l, w, folded, &mode);
+          if (at >= 0) {
+            v = in[at];
+            if (per_mode) {
+              const double f = l.f * a.fp[mode];
+              v.x *= f;
+              v.y *= f;
+            }
+          }
+        }
+        const unsigned x = (unsigned)__double2hiint(v.x) & 0x7fffffffu, y = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
+        if (x < 0x7ff00000u) m = max(m, x);
+        if (y < 0x7ff00000u) m = max(m, y);
+        reinterpret_cast<double2*>(buf)[g * Lp + df_slot(w)] = v;
+      }
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
+    __syncthreads();
+    const int shift = 1023 - (int)(s_max >> 20);
     int Ns = 1;
-    for (int s = 0; s < d.a.nrad; ++s) {
-      const bool first = s == 0, last = s == d.a.nrad - 1;
-      switch (d.a.rad[s]) {
-        case 8: df_pass<8>(c, Ns, first, last); break;
-        case 4: df_pass<4>(c, Ns, first, last); break;
-        case 2: df_pass<2>(c, Ns, first, last); break;
+    for (int s = 0; s < a.nrad; ++s) {
+      const bool first = s == 0;
+      switch (a.rad[s]) {
+        case 4: df_pass<4>(d, buf, Lp, Ns, first, shift); break;
+        case 2: df_pass<2>(d, buf, Lp, Ns, first, shift); break;
         case 5:
-          if constexpr (!POW2) df_pass<5>(c, Ns, first, last);
+          if constexpr (!POW2) df_pass<5>(d, buf, Lp, Ns, first, shift);
           break;
         default:
-          if constexpr (!POW2) df_pass<3>(c, Ns, first, last);
+          if constexpr (!POW2) df_pass<3>(d, buf, Lp, Ns, first, shift);
           break;
       }
-      Ns *= d.a.rad[s];
+      Ns *= a.rad[s];
+    }
+    double2* out = a.out + (long long)t * a.so.st;
+    const bool folded = d.fold != 0, per_mode = a.fac_on_out && a.fp != nullptr && a.so.pmode;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+      const int g = d.out_across ? e & (a.G - 1) : (int)(((float)e + 0.5f) * inv_L);
+      const int w = d.out_across ? e >> a.log2G : e - g * L;
+      if (line0 + g >= a.nlines) continue;
+      const DfLine l = df_line(d, a.so, line0 + g, folded, per_mode);
+      int mode;
+      const long long at = df_index(d, a.so, l, w, folded, &mode);
+      if (at < 0) continue;
+      const float4 x = buf[g * Lp + df_slot(w)];
+      Z o = Z{make_float2(x.x, x.y), make_float2(x.z, x.w)};
+      if (d.fold == 1) {  // W_L^(line w) as W_L^(1024 a) W_L^b
+        const int k = (line0 + g) * w;
+        o = zmul(zmul(o, __ldg(d.tw_hi + (k >> 10))), __ldg(d.tw_lo + (k & 1023)));
+      }
+      double2 y = make_double2(df_widen(o.h.x, -shift) + df_widen(o.l.x, -shift),
+                               df_widen(o.h.y, -shift) + df_widen(o.l.y, -shift));
+      if (per_mode) {
+        const double f = l.f * a.fp[mode];
+        y.x *= f;
+        y.y *= f;
+      }
+      out[at] = y;
     }
   }
 }
@@ -351,8 +316,8 @@ cudaError_t launch_line_fft_df(LineDfArgs d, cudaStream_t s) {
   if (d.a.nlines <= 0 || d.a.ntr <= 0) return cudaSuccess;
   if (d.a.L > fft_df_cap() || d.a.nrad < 1) return cudaErrorInvalidValue;
   // lines per block: a power of two.  Across lines (y, z, long 1D) four to
-  // sixteen adjacent ones -- 64 to 256 contiguous bytes -- while they fit 512
-  // threads of eight values; along x as many as give 128 threads.
+  // sixteen adjacent ones -- 64 to 256 contiguous bytes -- while they fit a
+  // block; along x as many as give 128 threads.
   const bool across = d.in_across || d.out_across;
   int G = 1, lg = 0;
   while (G < 16 && 2 * G * d.a.L <= fft_df_cap() &&
