@@ -2176,10 +2176,16 @@ static cufinufft_tune_entry layout_class(const Plan<T>* p, int cls) {
   return e;
 }
 
+// The classes the autotuner and the selector choose among.  1D spreading runs one
+// kernel whatever the layout, so its cell-run classes are left out there
+// (set_layout and set_layout_class still take them).
 template <typename T>
 static std::vector<cufinufft_tune_entry> tune_candidates(const Plan<T>* p) {
   std::vector<cufinufft_tune_entry> c;
-  for (int k = 0; k < kLayoutClasses; ++k) c.push_back(layout_class(p, k));
+  for (int k = 0; k < kLayoutClasses; ++k) {
+    c.push_back(layout_class(p, k));
+    if (p->dim == 1 && c.back().method == 5) c.back().ms = -2.f;
+  }
   return c;
 }
 
@@ -2363,7 +2369,7 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
 template <typename T>
 static int apply_layout_class(Plan<T>* p, int cls) {
   if (cls < 0 || cls >= kLayoutClasses) return CUFINUFFT_ERR_ARG;
-  cufinufft_tune_entry c = tune_candidates(p)[cls];
+  cufinufft_tune_entry c = layout_class(p, cls);
   if (c.ms == -2.f) return CUFINUFFT_ERR_METHOD;
   int bs[3] = {c.binsizex, c.binsizey, c.binsizez};
   return set_layout_impl(p, c.method, bs, c.maxsubprobsize);

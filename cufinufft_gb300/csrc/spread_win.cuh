@@ -12,7 +12,7 @@
 // same and a jump adds the whole window.
 //
 // Bound: the kernel rows (FMA pipe and MUFU) and the gather of the strengths in
-// the caller's order.  1e7 ordered points, 1e6 modes, ns 7: spread ~50 us (shared
+// the caller's order.  1e7 ordered points, 1e6 modes, ns 7: spread 87 us (shared
 // atomics, lanes over taps: 598 us).
 #pragma once
 
@@ -22,64 +22,72 @@
 
 namespace cfg {
 
-constexpr int kWinThreads = 128;
-constexpr int kWinBatch = 4;   // points whose loads are in flight together
-constexpr int kWinMax = 16;    // points per thread at most
-// One wave of threads first (about 1024 per SM), then longer runs.
-inline int win_points(int M) {
-  const long long k = ((long long)M + 152 * 1024 - 1) / (152 * 1024);
-  return k < 1 ? 1 : (k > kWinMax ? kWinMax : (int)k);
+// A block stages its points in shared memory with coalesced loads: read where
+// they lie, a warp's threads, K points apart, touch 32 sectors per load (110 us of
+// the 1e7-point spread).  Thread t's point u sits at slot 17 t + u, so the lanes
+// of one read fall in distinct banks.
+constexpr int kWinMax = 16;    // points per thread at most (a power of two)
+constexpr int kWinPitch = kWinMax + 1;
+template <typename T> constexpr int win_threads() { return sizeof(T) == 4 ? 128 : 64; }
+// log2 of the points per thread: one wave of threads first (about 1024 per
+// SM), then longer runs.
+inline int win_log_points(int M) {
+  int lg = 0;
+  while ((1 << lg) < kWinMax && ((long long)M >> lg) > 152 * 1024) ++lg;
+  return lg;
 }
+__device__ __forceinline__ int win_slot(int i, int lg) { return (i >> lg) * kWinPitch + (i & ((1 << lg) - 1)); }
 
 template <int NS>
-__global__ void __launch_bounds__(kWinThreads)
-k_spread_win(SpreadArgs<float> a, int K) {
-  constexpr int HD = horner_degree<float>(NS);
+__global__ void __launch_bounds__(win_threads<float>())
+k_spread_win(SpreadArgs<float> a, int lg) {
+  constexpr int HD = horner_degree<float>(NS), NT = win_threads<float>();
+  __shared__ int s_cell[NT * kWinPitch];
+  __shared__ float s_d[NT * kWinPitch];
+  __shared__ float2 s_c[NT * kWinPitch];
   const int nf0 = a.g.nf[0];
-  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * K;
-  if (first >= a.M) return;
-  const int beg = (int)first, end = min(a.M, beg + K);
+  const long long first = (long long)blockIdx.x * (NT << lg);
+  const int np = (int)min((long long)(NT << lg), a.M - first);
   const float2* cin = a.c_in + (size_t)blockIdx.y * a.M;
   float2* grid = a.fw + (size_t)blockIdx.y * a.g.Nf;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < np; i += NT) {
+    const int p = (int)first + i, q = win_slot(i, lg);
+    s_cell[q] = a.pts.i0[0][p];
+    s_d[q] = a.pts.d[0][p];
+    s_c[q] = cin[a.pts.idx[p]];
+  }
+  __syncthreads();
+  const int mine = min(1 << lg, np - (int)(threadIdx.x << lg));
+  if (mine <= 0) return;
+  const int q0 = threadIdx.x * kWinPitch;
   float2 acc[NS];
 #pragma unroll
   for (int j = 0; j < NS; ++j) acc[j] = make_float2(0.f, 0.f);
-  int cur = a.pts.i0[0][beg];
+  int cur = s_cell[q0];
   auto flush = [&](int j) { red_add(grid + wrap_idx(cur + j, nf0), acc[j].x, acc[j].y); };
-  for (int p0 = beg; p0 < end; p0 += kWinBatch) {
-    int cell[kWinBatch];
-    float d[kWinBatch];
-    float2 c[kWinBatch];
+  for (int u = 0; u < mine; ++u) {
+    const int cell = s_cell[q0 + u];
+    const float2 c = s_c[q0 + u];
+    float k[NS];
+    kernel_row<float, NS, HD>(s_d[q0 + u], a.kc, k);
+    const int s = cell - cur;
+    if (s < 0 || s >= NS) {
 #pragma unroll
-    for (int u = 0; u < kWinBatch; ++u) {
-      const int p = min(p0 + u, end - 1);
-      cell[u] = a.pts.i0[0][p];
-      d[u] = a.pts.d[0][p];
-      c[u] = cin[a.pts.idx[p]];
+      for (int j = 0; j < NS; ++j) {
+        flush(j);
+        acc[j] = make_float2(0.f, 0.f);
+      }
+      cur = cell;
+    }
+    for (; cur < cell; ++cur) {
+      flush(0);
+#pragma unroll
+      for (int j = 0; j + 1 < NS; ++j) acc[j] = acc[j + 1];
+      acc[NS - 1] = make_float2(0.f, 0.f);
     }
 #pragma unroll
-    for (int u = 0; u < kWinBatch; ++u) {
-      if (p0 + u >= end) break;
-      float k[NS];
-      kernel_row<float, NS, HD>(d[u], a.kc, k);
-      const int s = cell[u] - cur;
-      if (s < 0 || s >= NS) {
-#pragma unroll
-        for (int j = 0; j < NS; ++j) {
-          flush(j);
-          acc[j] = make_float2(0.f, 0.f);
-        }
-        cur = cell[u];
-      }
-      for (; cur < cell[u]; ++cur) {
-        flush(0);
-#pragma unroll
-        for (int j = 0; j + 1 < NS; ++j) acc[j] = acc[j + 1];
-        acc[NS - 1] = make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int j = 0; j < NS; ++j) acc[j] = fma2(c[u], dup2(k[j]), acc[j]);
-    }
+    for (int j = 0; j < NS; ++j) acc[j] = fma2(c, dup2(k[j]), acc[j]);
   }
 #pragma unroll
   for (int j = 0; j < NS; ++j) flush(j);
@@ -88,23 +96,33 @@ k_spread_win(SpreadArgs<float> a, int K) {
 // FP64 plans in double-float (SpreadArgs::fp64_df 1): the window as float pairs,
 // a thread's strengths scaled by the power of two of the largest of them.
 template <int NS>
-__global__ void __launch_bounds__(kWinThreads)
-k_spread_win_df(SpreadArgs<double> a, int K) {
+__global__ void __launch_bounds__(win_threads<double>())
+k_spread_win_df(SpreadArgs<double> a, int lg) {
+  constexpr int NT = win_threads<double>();
   __shared__ float2 s_tab[64];
-  if (!a.kc.horner) {
-    df_table_fill(s_tab, a.kc);
-    __syncthreads();
-  }
+  __shared__ int s_cell[NT * kWinPitch];
+  __shared__ double s_d[NT * kWinPitch];
+  __shared__ double2 s_c[NT * kWinPitch];
+  if (!a.kc.horner) df_table_fill(s_tab, a.kc);
   const int nf0 = a.g.nf[0];
-  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * K;
-  if (first >= a.M) return;
-  const int beg = (int)first, end = min(a.M, beg + K);
+  const long long first = (long long)blockIdx.x * (NT << lg);
+  const int np = (int)min((long long)(NT << lg), a.M - first);
   const double2* cin = a.c_in + (size_t)blockIdx.y * a.M;
   double2* grid = a.fw + (size_t)blockIdx.y * a.g.Nf;
-  unsigned m = 0;
 #pragma unroll 4
-  for (int p = beg; p < end; ++p) {
-    const double2 v = cin[a.pts.idx[p]];
+  for (int i = threadIdx.x; i < np; i += NT) {
+    const int p = (int)first + i, q = win_slot(i, lg);
+    s_cell[q] = a.pts.i0[0][p];
+    s_d[q] = a.pts.d[0][p];
+    s_c[q] = cin[a.pts.idx[p]];
+  }
+  __syncthreads();
+  const int mine = min(1 << lg, np - (int)(threadIdx.x << lg));
+  if (mine <= 0) return;
+  const int q0 = threadIdx.x * kWinPitch;
+  unsigned m = 0;
+  for (int u = 0; u < mine; ++u) {
+    const double2 v = s_c[q0 + u];
     const unsigned x = (unsigned)__double2hiint(v.x) & 0x7fffffffu, y = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
     if (x < 0x7ff00000u) m = max(m, x);
     if (y < 0x7ff00000u) m = max(m, y);
@@ -114,16 +132,16 @@ k_spread_win_df(SpreadArgs<double> a, int K) {
   float2 s[NS], e[NS];
 #pragma unroll
   for (int j = 0; j < NS; ++j) s[j] = e[j] = make_float2(0.f, 0.f);
-  int cur = a.pts.i0[0][beg];
+  int cur = s_cell[q0];
   auto flush = [&](int j) {
     red_add(grid + wrap_idx(cur + j, nf0), df_widen(s[j].x, back) + df_widen(e[j].x, back),
             df_widen(s[j].y, back) + df_widen(e[j].y, back));
   };
-  for (int p = beg; p < end; ++p) {
-    const int cell = a.pts.i0[0][p];
-    const double2 v = cin[a.pts.idx[p]];
+  for (int u = 0; u < mine; ++u) {
+    const int cell = s_cell[q0 + u];
+    const double2 v = s_c[q0 + u];
     float kh[NS], kl[NS];
-    df_kernel_row<NS>(a.pts.d[0][p], a.kc, s_tab, kh, kl);
+    df_kernel_row<NS>(s_d[q0 + u], a.kc, s_tab, kh, kl);
     const int step = cell - cur;
     if (step < 0 || step >= NS) {
 #pragma unroll
@@ -153,11 +171,11 @@ k_spread_win_df(SpreadArgs<double> a, int K) {
 
 template <typename T, int NS>
 cudaError_t launch_spread_win(const SpreadArgs<T>& a, cudaStream_t s) {
-  const int K = win_points(a.M);
-  const long long threads = ((long long)a.M + K - 1) / K;
-  const dim3 grid((unsigned)((threads + kWinThreads - 1) / kWinThreads), a.ntr);
-  if constexpr (sizeof(T) == 4) k_spread_win<NS><<<grid, kWinThreads, 0, s>>>(a, K);
-  else k_spread_win_df<NS><<<grid, kWinThreads, 0, s>>>(a, K);
+  const int lg = win_log_points(a.M);
+  const long long per = (long long)win_threads<T>() << lg;
+  const dim3 grid((unsigned)((a.M + per - 1) / per), a.ntr);
+  if constexpr (sizeof(T) == 4) k_spread_win<NS><<<grid, win_threads<T>(), 0, s>>>(a, lg);
+  else k_spread_win_df<NS><<<grid, win_threads<T>(), 0, s>>>(a, lg);
   return cudaGetLastError();
 }
 
