@@ -800,6 +800,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   if (ier > 1) return ier;
   if (sp_fixed) p->sp = *sp_fixed;
   for (int k = 0; k < dim; ++k) p->N[k] = nmodes[k];
+  p->bins_default = p->opts.gpu_binsizex < 0 && p->opts.gpu_binsizey < 0 && p->opts.gpu_binsizez < 0;
   setup_binsize(dim, &p->opts);
 
   // method actually run (src/2d/spread2d_wrapper.cu:99-164,
@@ -866,6 +867,11 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   long long nbins = (long long)p->nb[0] * p->nb[1] * p->nb[2];
   if (nbins > (1LL << 24)) return CUFINUFFT_ERR_ARG;
   p->nbins = (int)nbins;
+  for (int k = 0; k < 3; ++k) {
+    p->sort_bs[k] = p->bs[k];
+    p->sort_nb[k] = p->nb[k];
+  }
+  p->sort_nbins = p->nbins;
   if (p->cell_order && (!cell_order_fits(p, p->bs, nbins) ||
                         run_smem_bytes(p, p->bs) > (size_t)max_smem_optin(p->device)))
     p->cell_order = false;  // too many (bin, cell) keys or taps: plain method 2
@@ -913,8 +919,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   }
 
   const long long Nf = grid_cells(p);
-  int e = alloc_bins(p, p->nbins);
-  if (e) return e;
+  int e = 0;
   if (p->spread_only) {
     // no grid, FFT or kernel Fourier series: execute spreads into / reads
     // from the caller's fk
@@ -1142,9 +1147,14 @@ template <typename T>
 static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   p->nsub = 0;
   p->nsub_exact = true;
+  const int nbins = p->sort_nbins;
+  {
+    const int e = alloc_bins(p, nbins);
+    if (e) return e;
+  }
   for (int k = 0; k < 3; ++k) {
-    a.bs[k] = p->bs[k];
-    a.nb[k] = p->nb[k];
+    a.bs[k] = p->sort_bs[k];
+    a.nb[k] = p->sort_nb[k];
   }
   a.dim = p->dim;
   a.M = p->M;
@@ -1152,9 +1162,10 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   a.rank = p->rank;
   a.start = p->start;
   if (p->M == 0) return 0;
-  const int method = p->tile_m1 ? 2 : p->method;
+  const int method = p->route ? p->route : p->method;
   const int ms = method == 2 ? p->opts.gpu_maxsubprobsize : 0;
-  int e = bank_order(p, method, p->bs, p->nbins, &a.bank, p->cell_order);  // zeroes its counters
+  const bool cell = p->cell_order && method == 2;
+  int e = bank_order(p, method, p->sort_bs, nbins, &a.bank, cell);  // zeroes its counters
   if (e) return e;
   BinScanArgs sc;
   std::memset(&sc, 0, sizeof(sc));
@@ -1166,15 +1177,15 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   } else if (a.bank.cls_count && !a.bank.cell_order) {
     sc.raw = a.bank.cls_count;
     sc.raw_stride = sc.per = a.bank.ncls;
-  } else if (!a.bank.cls_count && p->nbins <= kCountStrideBins) {
+  } else if (!a.bank.cls_count && nbins <= kCountStrideBins) {
     sc.raw = p->raw;
     sc.raw_stride = kCountStride;
   }
   a.raw = const_cast<int*>(sc.raw);
   a.raw_stride = sc.raw_stride;
   if (!a.bank.cls_count || a.bank.cell_order == 1)
-    CFG_CUDA(cudaMemsetAsync(a.raw, 0, sizeof(int) * (size_t)p->nbins * sc.raw_stride, p->stream));
-  sc.nbins = p->nbins;
+    CFG_CUDA(cudaMemsetAsync(a.raw, 0, sizeof(int) * (size_t)nbins * sc.raw_stride, p->stream));
+  sc.nbins = nbins;
   sc.maxsub = ms;
   sc.count = p->count;
   sc.start = p->start;
@@ -1182,14 +1193,14 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   sc.partial = p->scan_part;
   CFG_CUDA(launch_bin_count<T>(a, p->stream));
   if (a.bank.cell_order)
-    CFG_CUDA(launch_scan(p->cls_count, p->cls_start, p->nbins * a.bank.ncls, a.bank.cell_order == 1 ? 2 : 0,
+    CFG_CUDA(launch_scan(p->cls_count, p->cls_start, nbins * a.bank.ncls, a.bank.cell_order == 1 ? 2 : 0,
                          dense_run(p->dim), p->cls_tmp, p->stream));
   CFG_CUDA(launch_bin_scan(sc, p->stream));
   SubHdrArgs h;
   std::memset(&h, 0, sizeof(h));
   if (ms > 0) {
     // a bin of c > 0 points holds at most 1 + (c - 1) / ms subproblems
-    const int bound = (int)std::min<long long>((long long)std::min(p->nbins, p->M) + p->M / ms, 0x7fffffffLL);
+    const int bound = (int)std::min<long long>((long long)std::min(nbins, p->M) + p->M / ms, 0x7fffffffLL);
     if ((size_t)bound > p->cap_sub) {
       cudaFree(p->sub_to_bin);
       cudaFree(p->sub_hdr);
@@ -1201,7 +1212,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
       p->cap_sub = bound;
     }
     h.sub_start = p->sub_start;
-    h.nbins = p->nbins;
+    h.nbins = nbins;
     h.nsub = bound;
     h.maxsub = ms;
     h.sub_to_bin = p->sub_to_bin;
@@ -1209,7 +1220,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   }
   CFG_CUDA(launch_permute<T>(a, h, p->stream));
   if (ms == 0) return 0;
-  if (p->cell_order) {
+  if (cell) {
     if ((size_t)h.nsub > p->cap_sub_dense) {
       cudaFree(p->sub_dense);
       cudaFree(p->sub_ndense);
@@ -1224,12 +1235,12 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
     std::memset(&c, 0, sizeof(c));
     c.sub_to_bin = p->sub_to_bin;
     c.sub_start = p->sub_start;
-    c.sub_total = p->sub_start + p->nbins;
+    c.sub_total = p->sub_start + nbins;
     c.start = p->start;
     c.cls_count = p->cls_count;
     for (int k = 0; k < 3; ++k) {
       c.i0[k] = a.i0[k];
-      c.bs[k] = p->bs[k];
+      c.bs[k] = p->sort_bs[k];
     }
     c.dim = p->dim;
     c.maxsub = ms;
@@ -1244,7 +1255,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   }
   p->nsub = h.nsub;
   p->nsub_exact = false;
-  CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + p->nbins, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+  CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + nbins, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
   CFG_CUDA(cudaEventRecord(p->ev_total, p->stream));
   return 0;
 }
@@ -1272,6 +1283,30 @@ static bool route_tiles(const Plan<T>* p) {
   return (long long)p->M >= (long long)least * p->nbins;
 }
 
+// The kernels and bins of the coming sort: the plan's, or a route's own -- a
+// routed 3D tile takes larger bins than the default 16x16x2, whose halo is most
+// of the tile (1e6 points, 200x162x128 grid: FP32 ns 6 125 us, 16x16x4 110,
+// 16x16x8 104; FP64 ns 10 1577 us, 16x16x4 1413, 8x8x8 1259; ns 13 3532, 2917,
+// 3201).
+template <typename T>
+static void choose_route(Plan<T>* p) {
+  p->route = route_tiles(p) ? 2 : 0;
+  int bs[3] = {p->bs[0], p->bs[1], p->bs[2]};
+  if (p->route == 2 && p->dim == 3 && p->bins_default) {
+    const int big[3] = {is_single<T>() ? 16 : 8, is_single<T>() ? 16 : 8, 8};
+    int t[3];
+    for (int k = 0; k < 3; ++k) t[k] = std::min(big[k], p->nf[k]);
+    if (tile_cells(3, p->sp.ns, t) * sizeof(cplx_t<T>) + 4096 <= (size_t)max_smem_optin(p->device))
+      for (int k = 0; k < 3; ++k) bs[k] = t[k];
+  }
+  p->sort_nbins = 1;
+  for (int k = 0; k < 3; ++k) {
+    p->sort_bs[k] = bs[k];
+    p->sort_nb[k] = k < p->dim ? (p->nf[k] + bs[k] - 1) / bs[k] : 1;
+    p->sort_nbins *= p->sort_nb[k];
+  }
+}
+
 // The part of setpts that FP32, FP64 and chained plans share: `a` says where
 // the points come from (their source, coordinates and axis maps).
 template <typename T>
@@ -1287,13 +1322,13 @@ static int setpts_from(Plan<T>* p, int M, PlaceArgs<T> a) {
   a.M = M;
   e = choose_layout(p, a);  // gpu_method 0: before the sort, from the points' occupancy
   if (e) return e;
-  p->tile_m1 = route_tiles(p);
+  choose_route(p);
   a.idx = p->idx;
   for (int k = 0; k < 3; ++k) {
     a.i0[k] = p->i0[k];
     a.d[k] = p->d[k];
-    a.bs[k] = p->bs[k];
-    a.nb[k] = p->nb[k];
+    a.bs[k] = p->sort_bs[k];
+    a.nb[k] = p->sort_nb[k];
   }
   if (p->method == 1 && p->sort == 0) {
     CFG_CUDA(launch_place_unsorted<T>(a, p->stream));
@@ -1963,6 +1998,7 @@ template int plan_use_stream<double>(Plan<double>*, cudaStream_t);
 template <typename T>
 static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
   resolve_nsub(p, true);
+  int nsub = p->method == 2 ? p->nsub : 0;
   std::memset(info, 0, sizeof(*info));
   info->type = p->type;
   info->dim = p->dim;
@@ -1982,7 +2018,7 @@ static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
   info->binsizey = p->bs[1];
   info->binsizez = p->bs[2];
   info->nbins = p->nbins;
-  info->nsubprob = p->method == 2 ? p->nsub : 0;
+  info->nsubprob = nsub;
   info->kerevalmeth = p->opts.gpu_kerevalmeth;
   info->beta = p->sp.beta;
   info->es_c = p->sp.c;
@@ -2029,10 +2065,7 @@ static int adopt_layout(Plan<T>* p, int method, const int bsz[3], int maxsub) {
     return CUFINUFFT_ERR_SHMEM;
   if (cell && !cell_order_fits(p, bs, nbins)) return CUFINUFFT_ERR_ARG;
   if (cell && run_smem_bytes(p, bs) > (size_t)max_smem_optin(p->device)) return CUFINUFFT_ERR_SHMEM;
-  const int e = alloc_bins(p, (int)nbins);
-  if (e) return e;
   p->method = method;
-  p->tile_m1 = false;
   p->cell_order = cell;
   p->sort = 1;
   p->opts.gpu_method = cell ? 5 : method;
@@ -2062,6 +2095,7 @@ static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub)
   int e = adopt_layout(p, method, bsz, maxsub);
   if (e) return e;
   p->layout_set = true;
+  choose_route(p);
   if (!p->pts_set || p->M == 0) return 0;
   // fresh arrays for the re-sorted points
   PlaceArgs<T> a;

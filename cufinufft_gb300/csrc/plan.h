@@ -29,10 +29,14 @@ template <typename T> struct Plan {
   int variant = 0; // kernel family: 0 default, 1 one thread per point, 2 warp-cooperative
   bool auto_method = false;  // gpu_method 0: chosen by the library
   bool layout_set = false;   // set_layout / autotune: the layout is the caller's
-  bool tile_m1 = false;      // method 1 interpolation on the tile kernels (route_tiles)
+  int route = 0;             // the method run in place of `method` (0: that one), see choose_route
+  bool bins_default = false; // the caller left the bin sizes to the library
   int sort = 1;
   int bs[3] = {1, 1, 1}, nb[3] = {1, 1, 1};
   int nbins = 1;
+  // the bins the points are sorted by: those above, or a route's own
+  int sort_bs[3] = {1, 1, 1}, sort_nb[3] = {1, 1, 1};
+  int sort_nbins = 1;
   int device = 0;
   int M = 0, nsub = 0;
   bool planned = false, pts_set = false;
@@ -218,12 +222,12 @@ inline SpreadArgs<T> spread_args(Plan<T>* p) {
   for (int k = 0; k < 3; ++k) {
     a.pts.i0[k] = p->i0[k];
     a.pts.d[k] = p->d[k];
-    a.bins.bs[k] = p->bs[k];
-    a.bins.nb[k] = p->nb[k];
+    a.bins.bs[k] = p->sort_bs[k];
+    a.bins.nb[k] = p->sort_nb[k];
     a.g.nf[k] = p->nf[k];
   }
   a.pts.M = p->M;
-  a.bins.nbins = p->nbins;
+  a.bins.nbins = p->sort_nbins;
   a.bins.count = p->count;
   a.bins.start = p->start;
   a.bins.sub_start = p->sub_start;
@@ -264,16 +268,17 @@ int resolve_nsub(Plan<T>* p, bool wait);
 
 template <typename T>
 inline cudaError_t run_spread(Plan<T>* p, const SpreadArgs<T>& a) {
+  const int method = p->route ? p->route : p->method;
   switch (p->dim) {
-    case 1: return spread_dim<T, 1>(p->method, p->sp.ns, a, p->stream);
-    case 2: return spread_dim<T, 2>(p->method, p->sp.ns, a, p->stream);
-    default: return spread_dim<T, 3>(p->method, p->sp.ns, a, p->stream);
+    case 1: return spread_dim<T, 1>(method, p->sp.ns, a, p->stream);
+    case 2: return spread_dim<T, 2>(method, p->sp.ns, a, p->stream);
+    default: return spread_dim<T, 3>(method, p->sp.ns, a, p->stream);
   }
 }
 
 template <typename T>
 inline cudaError_t run_interp(Plan<T>* p, const SpreadArgs<T>& a) {
-  const int method = p->tile_m1 ? 2 : p->method;
+  const int method = p->route ? p->route : p->method;
   switch (p->dim) {
     case 1: return interp_dim<T, 1>(method, p->sp.ns, a, p->stream);
     case 2: return interp_dim<T, 2>(method, p->sp.ns, a, p->stream);
