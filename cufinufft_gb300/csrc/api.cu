@@ -1163,7 +1163,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   a.start = p->start;
   if (p->M == 0) return 0;
   const int method = p->route ? p->route : p->method;
-  const int ms = method == 2 ? p->opts.gpu_maxsubprobsize : 0;
+  const int ms = method == 2 ? p->sort_ms : 0;
   const bool cell = p->cell_order && method == 2;
   int e = bank_order(p, method, p->sort_bs, nbins, &a.bank, cell);  // zeroes its counters
   if (e) return e;
@@ -1260,44 +1260,77 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   return 0;
 }
 
-// Method 1 (the default of type 2) gathers every tap from L1 and L2, eight
-// or sixteen lanes to a point; from some density on, the subproblem kernel of
-// method 2 over the same bins is faster, its tile loaded once for all its
-// points: 2D and 3D, sorted points, a layout that the caller left alone.
-// Measured gather / tile times (us) by mean points per bin, default bins:
-//   FP32 tol 1e-6 2D: 31: 19.9 / 19.3, 123: 55.9 / 24.1 (1024^2); small calls
-//     123: 9.0 / 8.3 (256^2); tol 1e-3 123: 7.4 / 8.2 (256^2), 26.9 / 19.1
-//   FP32 tol 1e-6 3D: 15: 177 / 129, 59: 627 / 193 (96^3); tol 1e-3 58: 37 / 27
-//   FP64 tol 1e-9: 8: 101 / 213, 31: 353 / 223 (1024^2); 15: 702 / 494, 58:
-//     2724 / 632 (60^3); tol 1e-12 3D 14: 1051 / 1363, 58: 4092 / 1475
-// so FP32 takes the tile from 100 points per bin in 2D and 48 in 3D (the sort's
-// bank classes cost a little more than plain bins), FP64 from 28.
-template <typename T>
-static bool route_tiles(const Plan<T>* p) {
-  if (p->type != 2 || p->dim < 2 || p->method != 1 || !p->sort || p->auto_method || p->layout_set || p->variant != 0)
-    return false;
-  if (!is_single<T>() && !p->fp64_df) return false;
-  if (p->opts.gpu_maxsubprobsize < 256) return false;
-  if (tile_cells(p->dim, p->sp.ns, p->bs) * sizeof(cplx_t<T>) + 4096 > (size_t)max_smem_optin(p->device)) return false;
-  const int least = is_single<T>() ? (p->dim == 2 ? 100 : 48) : 28;
-  return (long long)p->M >= (long long)least * p->nbins;
-}
-
-// The kernels and bins of the coming sort: the plan's, or a route's own -- a
-// routed 3D tile takes larger bins than the default 16x16x2, whose halo is most
-// of the tile (1e6 points, 200x162x128 grid: FP32 ns 6 125 us, 16x16x4 110,
-// 16x16x8 104; FP64 ns 10 1577 us, 16x16x4 1413, 8x8x8 1259; ns 13 3532, 2917,
-// 3201).
+// The kernels, bins and subproblem cap of the coming sort.  A default plan --
+// no layout, bins or kernel variant asked for -- may run on others than it
+// reports; the values are the same up to the order of sums.
+//
+// Type 2: method 1 gathers every tap from L1 and L2, eight or sixteen lanes to a
+// point; the subproblem kernel loads a tile once for all its points.  With r =
+// taps of a mean bin's points / cells of its tile, gather / tile (us):
+//   FP32 2D tol 1e-6  r 0.8: 19.9 / 19.3, 3.1: 55.9 / 24.1 (1024^2); 3.1: 9.0 / 8.3 (256^2)
+//   FP32 3D tol 1e-5  r 0.6: 26.8 / 29.4, 1.5: 39.4 / 31.0 (64^3); 5.0: 23.7 / 16.7 (32^3)
+//   FP64 2D tol 1e-9  r 0.5: 101 / 213 (1024^2), 1.1: 66 / 53 (512^2), 1.8: 353 / 223
+//   FP64 3D tol 1e-9  r 0.8: 261 / 425, 2.1: 592 / 435 (64^3); 6.7: 258 / 91 (32^3)
+// so the tile runs from r = 1.5, in 2D FP32 (where the sort's bank classes cost
+// more than plain bins) from 2.5.  In 3D it takes larger bins than 16x16x2, whose
+// halo is most of the tile (1e6 points, 200x162x128 grid: FP32 ns 6 125 us,
+// 16x16x8 104; FP64 ns 10 1577 us, 8x8x8 1259; ns 13 3532, 3201).
+//
+// Type 1: bins whose private tiles or slabs keep more blocks on an SM.  32^2 or
+// 16x16x2 bins / these (us): FP32 2D 16^2 from 0.35 points per cell 1e6 points
+// 68 / 61 (512^2), below it 58 / 80 (4e5 points, 1024^2); FP64 2D 16^2 557 / 303
+// (1e6, 512^2), for ns > 11 from 0.15 points per cell 693 / 491 (below 585 / 684);
+// FP32 3D 16x8x4 1646 / 1465 (4e6, 64^3, ns 6) and 1970 / 1736 (ns 7); FP64 3D
+// 8^3 3936 / 3187 (1e6, 100x96x100, ns 10), for ns > 11 16x16x4 7563 / 6947.
+//
+// A subproblem is one block, so a crowded bin's thousand points take as long as
+// the whole call where there are few others: the cap falls with M (and the
+// transforms of a batch) until about two thousand blocks can run (1e5 clustered points, cap 1024 / this: FP32
+// 2D 32 / 20, 3D 230 / 57; FP64 2D 115 / 62, 3D 609 / 322; even points unchanged).
+// Interpolation reloads its tile for each, which pays down to 256 points
+// (1e5 clustered points, 3D: FP32 37 / 26, FP64 314 / 175).
 template <typename T>
 static void choose_route(Plan<T>* p) {
-  p->route = route_tiles(p) ? 2 : 0;
+  p->route = 0;
+  p->sort_ms = p->opts.gpu_maxsubprobsize;
   int bs[3] = {p->bs[0], p->bs[1], p->bs[2]};
-  if (p->route == 2 && p->dim == 3 && p->bins_default) {
-    const int big[3] = {is_single<T>() ? 16 : 8, is_single<T>() ? 16 : 8, 8};
+  const int ns = p->sp.ns;
+  const double density = (double)p->M / (double)grid_cells(p);
+  const bool open = p->dim >= 2 && p->sort && !p->auto_method && !p->layout_set && p->variant == 0 &&
+                    (is_single<T>() || p->fp64_df == 1 || (p->fp64_df && p->type == 2));
+  const auto fit = [&](int x, int y, int z) {  // x * y * z bins, where the tile (and four copies in 2D) fits
+    const int want[3] = {x, y, z};
     int t[3];
-    for (int k = 0; k < 3; ++k) t[k] = std::min(big[k], p->nf[k]);
-    if (tile_cells(3, p->sp.ns, t) * sizeof(cplx_t<T>) + 4096 <= (size_t)max_smem_optin(p->device))
-      for (int k = 0; k < 3; ++k) bs[k] = t[k];
+    for (int k = 0; k < 3; ++k) t[k] = k < p->dim ? std::min(want[k], p->nf[k]) : 1;
+    const size_t copies = p->type == 1 && p->dim == 2 ? 4 : 1;
+    if (copies * tile_cells(p->dim, ns, t) * sizeof(cplx_t<T>) + 16384 > (size_t)max_smem_optin(p->device)) return;
+    for (int k = 0; k < 3; ++k) bs[k] = t[k];
+  };
+  const auto cap = [&](int least, int share) {
+    int ms = least;
+    while (ms < 1024 && (long long)ms * share < (long long)p->M * p->maxbatch) ms *= 2;
+    p->sort_ms = std::min(p->sort_ms, ms);
+  };
+  if (open && p->type == 2 && p->method == 1 && p->opts.gpu_maxsubprobsize >= 256) {
+    if (p->dim == 3 && p->bins_default) is_single<T>() ? fit(16, 16, 8) : fit(8, 8, 8);
+    double taps = density, cells = 1.0;
+    for (int k = 0; k < p->dim; ++k) {
+      taps *= ns * (double)bs[k];
+      cells *= bs[k] + 2 * ((ns + 1) / 2);
+    }
+    if (taps >= (is_single<T>() && p->dim == 2 ? 2.5 : 1.5) * cells &&
+        cells * sizeof(cplx_t<T>) + 4096 <= (double)max_smem_optin(p->device)) {
+      p->route = 2;
+      cap(256, p->dim == 2 ? 1024 : 2048);
+    } else {
+      for (int k = 0; k < 3; ++k) bs[k] = p->bs[k];
+    }
+  } else if (open && p->type == 1 && p->method == 2 && !p->cell_order && p->bins_default) {
+    p->route = 2;
+    if (p->dim == 2 && (is_single<T>() ? density >= 0.35 : (ns <= 11 || density >= 0.15))) fit(16, 16, 1);
+    if (p->dim == 3 && is_single<T>()) fit(16, 8, 4);
+    if (p->dim == 3 && !is_single<T>() && ns <= 13) ns <= 11 ? fit(8, 8, 8) : fit(16, 16, 4);
+    cap(128, 2048);
   }
   p->sort_nbins = 1;
   for (int k = 0; k < 3; ++k) {
@@ -1995,10 +2028,41 @@ template int execute_plan<double>(Plan<double>*, cplx_t<double>*, cplx_t<double>
 template int plan_use_stream<float>(Plan<float>*, cudaStream_t);
 template int plan_use_stream<double>(Plan<double>*, cudaStream_t);
 
+// Subproblems of the plan's reported bins, for a plan sorted by a route's own.
+template <typename T>
+static int count_subproblems(Plan<T>* p, int* nsub) {
+  *nsub = 0;
+  if (p->M == 0) return 0;
+  std::vector<int> h((size_t)p->nbins);
+  PlaceArgs<T> a;
+  std::memset(&a, 0, sizeof(a));
+  a.src = kSrcStored;
+  a.dim = p->dim;
+  a.M = p->M;
+  for (int k = 0; k < 3; ++k) {
+    a.src_i0[k] = p->i0[k];
+    a.src_d[k] = p->d[k];
+    a.bs[k] = p->bs[k];
+    a.nb[k] = p->nb[k];
+  }
+  CFG_CUDA(cudaMalloc(&a.count, sizeof(int) * h.size()));
+  cudaError_t e = cudaMemsetAsync(a.count, 0, sizeof(int) * h.size(), p->stream);
+  if (e == cudaSuccess) e = launch_feature_count<T>(a, p->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(h.data(), a.count, sizeof(int) * h.size(), cudaMemcpyDeviceToHost, p->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+  cudaFree(a.count);
+  CFG_CUDA(e);
+  const int ms = p->opts.gpu_maxsubprobsize;
+  for (int c : h) *nsub += c / ms + (c % ms ? 1 : 0);
+  return 0;
+}
+
 template <typename T>
 static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
   resolve_nsub(p, true);
   int nsub = p->method == 2 ? p->nsub : 0;
+  if (p->route && p->method == 2) count_subproblems(p, &nsub);
   std::memset(info, 0, sizeof(*info));
   info->type = p->type;
   info->dim = p->dim;

@@ -293,23 +293,23 @@ static int batch_make(Batch<T>* b, int nplans, Plan<T>** plans) {
       task += ((long long)p->M + PPW - 1) / PPW;
     } else {
       for (int k = 0; k < 3; ++k) {
-        D.bins.bs[k] = p->bs[k];
-        D.bins.nb[k] = p->nb[k];
+        D.bins.bs[k] = p->sort_bs[k];
+        D.bins.nb[k] = p->sort_nb[k];
       }
-      D.bins.nbins = p->nbins;
+      D.bins.nbins = p->sort_nbins;
       D.bins.count = p->count;
       D.bins.start = p->start;
       D.bins.sub_start = p->sub_start;
       D.bins.sub_to_bin = p->sub_to_bin;
       D.bins.nsub = p->nsub;
-      D.bins.maxsub = p->opts.gpu_maxsubprobsize;
+      D.bins.maxsub = p->sort_ms;
       blk += (long long)p->nsub * p->ntransf;
-      b->smem = std::max(b->smem, tile_cells(p->dim, p->sp.ns, p->bs) * sizeof(cplx_t<T>));
+      b->smem = std::max(b->smem, tile_cells(p->dim, p->sp.ns, p->sort_bs) * sizeof(cplx_t<T>));
       if (b->type == 1 && p->cell_order && p->sub_dense) {
         D.sub_dense = p->sub_dense;
         BinTables bt;
         std::memset(&bt, 0, sizeof(bt));
-        for (int k = 0; k < 3; ++k) bt.bs[k] = p->bs[k];
+        for (int k = 0; k < 3; ++k) bt.bs[k] = p->sort_bs[k];
         const size_t rb = p->dim == 1 ? run_bytes<T, 1>(p->sp.ns, bt)
                           : (p->dim == 2 ? run_bytes<T, 2>(p->sp.ns, bt) : run_bytes<T, 3>(p->sp.ns, bt));
         b->smem_run = std::max(b->smem_run, rb);

@@ -34,9 +34,10 @@ template <typename T> struct Plan {
   int sort = 1;
   int bs[3] = {1, 1, 1}, nb[3] = {1, 1, 1};
   int nbins = 1;
-  // the bins the points are sorted by: those above, or a route's own
+  // the bins the points are sorted by, and their subproblems' cap: those above
+  // and of the options, or a route's own
   int sort_bs[3] = {1, 1, 1}, sort_nb[3] = {1, 1, 1};
-  int sort_nbins = 1;
+  int sort_nbins = 1, sort_ms = 0;
   int device = 0;
   int M = 0, nsub = 0;
   bool planned = false, pts_set = false;
@@ -234,7 +235,7 @@ inline SpreadArgs<T> spread_args(Plan<T>* p) {
   a.bins.sub_to_bin = p->sub_to_bin;
   a.bins.hdr = p->sub_hdr;
   a.bins.nsub = p->nsub;
-  a.bins.maxsub = p->opts.gpu_maxsubprobsize;
+  a.bins.maxsub = p->sort_ms;
   a.kc.beta = (T)p->sp.beta;
   a.kc.c = (T)p->sp.c;
   a.kc.e_beta = (T)std::exp(p->sp.beta);
