@@ -1280,7 +1280,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
 // 16x16x2 bins / these (us): FP32 2D 16^2 from 0.35 points per cell 1e6 points
 // 68 / 61 (512^2), below it 58 / 80 (4e5 points, 1024^2); FP64 2D 16^2 557 / 303
 // (1e6, 512^2), for ns > 11 from 0.15 points per cell 693 / 491 (below 585 / 684);
-// FP32 3D 16x8x4 1646 / 1465 (4e6, 64^3, ns 6) and 1970 / 1736 (ns 7); FP64 3D
+// FP32 3D 16x8x4 212 / 202 (4e5, 64^3, ns 8), 8^3 from col_density 1164 / 803 (4e6); FP64 3D
 // 8^3 3936 / 3187 (1e6, 100x96x100, ns 10), for ns > 11 16x16x4 7563 / 6947.
 //
 // A subproblem is one block, so a crowded bin's thousand points take as long as
@@ -1325,10 +1325,24 @@ static void choose_route(Plan<T>* p) {
     } else {
       for (int k = 0; k < 3; ++k) bs[k] = p->bs[k];
     }
+  } else if (is_single<T>() && p->type == 1 && p->dim == 3 && p->auto_method && !p->layout_set && p->cell_order &&
+             density >= col_density(ns, true)) {
+    // the chosen cell-run layout, in bins whose columns hold more to share
+    // (3.2e7 half-clustered points, 256^3: 8.14 -> 5.65 ms)
+    const int deep[3] = {std::min(8, p->nf[0]), std::min(8, p->nf[1]), std::min(8, p->nf[2])};
+    long long nb = 1;
+    for (int k = 0; k < 3; ++k) nb *= (p->nf[k] + deep[k] - 1) / deep[k];
+    if (cell_order_fits(p, deep, nb) && run_smem_bytes(p, deep) <= (size_t)max_smem_optin(p->device)) {
+      p->route = 2;
+      for (int k = 0; k < 3; ++k) bs[k] = deep[k];
+    }
   } else if (open && p->type == 1 && p->method == 2 && !p->cell_order && p->bins_default) {
     p->route = 2;
     if (p->dim == 2 && (is_single<T>() ? density >= 0.35 : (ns <= 11 || density >= 0.15))) fit(16, 16, 1);
-    if (p->dim == 3 && is_single<T>()) fit(16, 8, 4);
+    if (p->dim == 3 && is_single<T>()) {
+      if (density >= col_density(ns, false)) fit(8, 8, 8);  // spread_col.cuh
+      else fit(16, 8, 4);
+    }
     if (p->dim == 3 && !is_single<T>() && ns <= 13) ns <= 11 ? fit(8, 8, 8) : fit(16, 16, 4);
     cap(128, 2048);
   }

@@ -104,6 +104,11 @@ template <typename T> cudaError_t launch_bin_count(PlaceArgs<T> a, cudaStream_t 
 template <typename T> cudaError_t launch_permute(PlaceArgs<T> a, const SubHdrArgs& h, cudaStream_t s);
 template <typename T> cudaError_t launch_place_unsorted(PlaceArgs<T> a, cudaStream_t s);
 
+// Points per grid cell from which 3D FP32 spreading orders a bin's points by
+// column (spread_col.cuh): on plain bins -- narrow kernels need more to repay the
+// sort -- and on a cell-run layout, whose dense cells go to another kernel.
+constexpr double col_density(int ns, bool run) { return run || ns < 6 ? 1.0 : 0.4; }
+
 // Complex FP64 <-> FP32 conversion of n values.
 cudaError_t launch_narrow_complex(const double2* in, float2* out, long long n, cudaStream_t s);
 cudaError_t launch_widen_complex(const float2* in, double2* out, long long n, cudaStream_t s);

@@ -1130,7 +1130,8 @@ k_spread_sm_wc(SpreadArgs<T> a) {
 }
 
 // ---------------------------------------------------------------------------
-// Slab-owned 3D spreading (method 2, the default for sparse 3D subproblems).
+// Slab-owned 3D spreading (method 2; FP32 where cells hold few points, see
+// spread_col.cuh for the others, and FP64 without double-float kernels).
 // Shared FP32 atomicAdd runs at about a third of the int32 rate and costs
 // several shared wavefronts per warp instruction, which bound the
 // warp-cooperative kernel.  Here the tile's z-planes are owned: the block has
@@ -1477,6 +1478,7 @@ k_spread_sm_priv(SpreadArgs<T> a, int split) {
 }  // namespace cfg
 #include "spread_df.cuh"
 #include "spread_win.cuh"
+#include "spread_col.cuh"
 namespace cfg {
 
 // CUFINUFFT_SPREAD_PRIV=0: 2D subproblem spreading by the warp-cooperative
@@ -2073,6 +2075,7 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
     if (a.bins.nsub == 0) return cudaSuccess;
     // 3D sparse subproblems: the slab-owned kernel unless a variant is forced
     bool slab = false, split = false, priv = false;
+    [[maybe_unused]] bool col = false;
     [[maybe_unused]] SlabDfShape slab_df{0, 0, 0};
     if constexpr (DIM == 2) {
       priv = a.variant == 0 && priv_spread_enabled();
@@ -2094,6 +2097,10 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         if (a.fp64_df) slab_df = slab_df_shape(NS, a.bins, (size_t)optin - 2048);  // less its static part
         slab = slab_bytes<T>(NS, a.bins) <= (size_t)optin;
+        if constexpr (sizeof(T) == 4) {
+          col = slab && col_bins(a.bins) && col_bytes<NS>(a.bins) <= (size_t)optin &&
+                (double)a.M >= col_density(NS, a.run != 0) * (double)a.g.Nf;
+        }
       }
       // cell-run layout: the slab kernel also takes the sparse tails of the
       // dense subproblems (the tensor-core form walks whole subproblems)
@@ -2128,6 +2135,15 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
           cudaError_t e = prepare_smem(k_spread_sm_priv<T, NS>, smb);
           if (e != cudaSuccess) return e;
           k_spread_sm_priv<T, NS><<<dim3(a.bins.nsub, a.ntr), 32 * kPrivWarps, smb, s>>>(a, split ? 1 : 0);
+          return cudaGetLastError();
+        }
+      }
+      if constexpr (DIM == 3 && sizeof(T) == 4) {
+        if (col) {
+          const size_t smb = col_bytes<NS>(a.bins);
+          cudaError_t e = prepare_smem(k_spread_sm_col<NS>, smb);
+          if (e != cudaSuccess) return e;
+          k_spread_sm_col<NS><<<dim3(a.bins.nsub, a.ntr), 32 * ColRow<NS>::NW, smb, s>>>(a, split ? 1 : 0);
           return cudaGetLastError();
         }
       }
