@@ -228,10 +228,23 @@ static std::vector<int> radix_plan(int L, int most = 8) {
   return r;
 }
 
+static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
+
+// The pruned line FFT instead of cuFFT and the mode-row kernel: asked for
+// (CUFINUFFT_FFT=line), or an FP32 grid of at least 2^20 cells whose sides are
+// powers of two from 256 to 4096 -- cuFFT with amplification or deconvolution / the
+// line passes, us: 2048^2 38 / 28, 1024^2 16.7 / 15.3, 256^3 135 / 71; smaller grids
+// are latency, where cuFFT's passes are the shorter: 512^2 11.2 / 14.5.
 template <typename T>
 static bool use_line_fft(const Plan<T>* p) {
   const char* v = std::getenv("CUFINUFFT_FFT");
-  if (v == nullptr || std::strcmp(v, "line") != 0) return false;
+  if (v == nullptr) {
+    if (!is_single<T>() || p->dim < 2 || (p->type != 1 && p->type != 2) || grid_cells(p) < (1LL << 20)) return false;
+    for (int k = 0; k < p->dim; ++k)
+      if (!power_of_two(p->nf[k]) || p->nf[k] < 256 || p->nf[k] > 4096) return false;
+    return true;
+  }
+  if (std::strcmp(v, "line") != 0) return false;
   for (int k = 0; k < p->dim; ++k) {
     const std::vector<int> r = radix_plan(p->nf[k]);
     if (p->nf[k] > line_fft_cap<T>() || r.empty() || r.size() > 24) return false;
@@ -255,7 +268,6 @@ static bool use_half_fft(const Plan<T>* p) {
 // it and no other FFT form was asked for: every axis up to 4096 points, or a 1D
 // grid that splits into two such factors.  Below upsampfac 2, where the
 // deconvolution amplifies the grid's rounding, only 2D power-of-two grids.
-static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
 template <typename T>
 static bool use_line_df(Plan<T>* p) {
   if (sizeof(T) != 8 || !p->df_fft_ok || (p->type != 1 && p->type != 2)) return false;
@@ -444,18 +456,22 @@ static std::vector<HalfPass<T>> half_passes(const Plan<T>* p, cplx_t<T>* fk, int
 
 template <typename T>
 static int make_line_fft(Plan<T>* p) {
-  const long double two_pi = 6.283185307179586476925286766559005768L;
+  [[maybe_unused]] const long double two_pi = 6.283185307179586476925286766559005768L;
   for (int k = 0; k < p->dim; ++k) {
     const int L = p->nf[k];
     p->rad[k] = radix_plan(L);
-    std::vector<cplx_t<T>> h((size_t)L);
-    for (int m = 0; m < L; ++m) {
-      const long double ang = two_pi * (long double)m / (long double)L;
-      h[m].x = (T)(double)cosl(ang);
-      h[m].y = (T)(double)((long double)p->iflag * sinl(ang));
-    }
     CFG_CUDA(cudaMalloc(&p->tw[k], sizeof(cplx_t<T>) * (size_t)L));
-    CFG_CUDA(cudaMemcpy(p->tw[k], h.data(), sizeof(cplx_t<T>) * (size_t)L, cudaMemcpyHostToDevice));
+    if constexpr (sizeof(T) == 4) {
+      CFG_CUDA(launch_line_twiddles(p->tw[k], p->iflag, L, p->stream));
+    } else {
+      std::vector<cplx_t<T>> h((size_t)L);
+      for (int m = 0; m < L; ++m) {
+        const long double ang = two_pi * (long double)m / (long double)L;
+        h[m].x = (T)(double)cosl(ang);
+        h[m].y = (T)(double)((long double)p->iflag * sinl(ang));
+      }
+      CFG_CUDA(cudaMemcpy(p->tw[k], h.data(), sizeof(cplx_t<T>) * (size_t)L, cudaMemcpyHostToDevice));
+    }
   }
   CFG_CUDA(line_fft_prepare<T>());
   p->line_fft = true;

@@ -54,6 +54,9 @@ __device__ __forceinline__ C csub(C a, C b) {
   r.y = a.y - b.y;
   return r;
 }
+// FP32: both components in one packed instruction
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 // z * (dir i)
 template <typename C, typename S>
 __device__ __forceinline__ C cmul_i(C z, S dir) {
@@ -595,6 +598,150 @@ k_line_fft_p2(LineArgs<T> a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP32 power-of-two lines of 256 to 4096 points: the passes of k_line_fft_p2
+// with the length known to the compiler, so that shared and (along x) global
+// addresses step by constants and the padding test is one compare per value (the
+// modes' low half lies below L / 2, the high half above); complex sums are packed.
+// Bound by issue and the latency of three exchanges: 70-110 thread instructions per
+// value, 40-60% of issue slots.  FFT with deconvolution, k_line_fft_p2 / this / cuFFT
+// with the mode-row kernel (us): 2048^2 61 / 28 / 38, 256^3 123 / 71 / 135; 1024^2
+// type 2 - / 15.3 / 16.7.
+// ROWS: positions are contiguous on both sides; else lines are, and the pitch
+// spreads a half warp's 4 lines x 4 positions over the banks.
+__host__ __device__ constexpr int fx_pitch(int L, int G) { return L + L / 16 + (G < 16 ? 16 / G : 1); }
+template <int LGL, int R, bool LAST, bool ROWS>
+__device__ __forceinline__ void fx_pass(const LineArgs<float>& a, float2* buf, float2* out, int lgNs, int line0, int LP) {
+  constexpr int L = 1 << LGL, NB = 16 / R, LGR = R == 16 ? 4 : (R == 8 ? 3 : (R == 4 ? 2 : 1));
+  constexpr int LGNBF = LGL - LGR, nbf = 1 << LGNBF, kStep = nbf + nbf / 16;  // nbf >= 16: padded step
+  const int Ns = 1 << lgNs, T_ = blockDim.x;
+  constexpr bool lines_fast = LAST && !ROWS;
+  float2 v[NB][R];
+  int gg[NB], jj[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    p2_split(threadIdx.x + b * T_, LGNBF, a.log2G, lines_fast, gg[b], jj[b]);
+    const float2* l = buf + gg[b] * LP + sidx(jj[b]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[b][r] = l[r * kStep];
+  }
+  __syncthreads();  // every read of this pass is done before any write
+  const float dir = (float)a.dir;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int k = jj[b] & (Ns - 1);
+    twiddle_p2<float, R>(v[b], k << (LGL - lgNs - LGR), a.tw);
+    Dft<float, R>::run(v[b], dir);
+  }
+  if (!LAST) {
+    const int step = Ns + (Ns >> 4);  // Ns >= 16
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int k = jj[b] & (Ns - 1), q = jj[b] >> lgNs;
+      float2* l = buf + gg[b] * LP + sidx((q << (lgNs + LGR)) + k);
+#pragma unroll
+      for (int r = 0; r < R; ++r) l[r * step] = v[b][r];
+    }
+    __syncthreads();
+    return;
+  }
+  // last pass: nbf = Ns, output r of butterfly j lies at position j + r nbf
+  const LineSide& so = a.so;
+  const int hi = so.pmode ? (so.Np - 1) / 2 : L, lo = so.pmode ? L - so.Np / 2 : 0;
+  const long long sp = ROWS ? 1 : so.sp, step = (long long)nbf * sp;
+  const bool fac = a.fac_on_out != 0;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int line = line0 + gg[b], j = jj[b];
+    if (line >= a.nlines) continue;
+    const int lb = line / a.A, la = line - lb * a.A;
+    // of the low half and of the high half: where position j would lie, and its mode
+    const int m0 = j + (so.pmode ? so.Np / 2 : 0), m1 = j - (so.pmode ? L - so.Np / 2 : 0);
+    float2* p0 = out + side_line(so, la, lb) + (long long)(so.pmode == 1 ? m0 : j) * sp;
+    float2* p1 = out + side_line(so, la, lb) + (long long)(so.pmode == 1 ? m1 : j) * sp;
+    const float f0 = fac ? line_factor(a, la, lb, -1) : 1.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int w = j + r * nbf;
+      if (r < R / 2 ? w > hi : w < lo) continue;
+      float2 o = v[b][r];
+      if (fac) o = cscale(o, (a.fp && so.pmode) ? f0 * a.fp[(r < R / 2 ? m0 : m1) + r * nbf] : f0);
+      (r < R / 2 ? p0 : p1)[r * step] = o;
+    }
+  }
+}
+
+template <int LGL, bool ROWS>
+__global__ void __launch_bounds__(512, 2)
+k_line_fft_fx(const __grid_constant__ LineArgs<float> a) {
+  constexpr int L = 1 << LGL, LGNBF = LGL - 4, nbf = 1 << LGNBF;
+  constexpr int REM = 1 << (LGL & 3);  // the radix after the 16s (1: none)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float2* buf = reinterpret_cast<float2*>(smem_raw);
+  const int line0 = blockIdx.x * a.G;
+  const LineSide& si = a.si;
+  int g, j;
+  p2_split(threadIdx.x, LGNBF, a.log2G, !ROWS, g, j);
+  const int LP = fx_pitch(L, a.G), line = line0 + g;
+  const int lb = line / a.A, la = line - lb * a.A;
+  const bool fac = !a.fac_on_out && (a.fa || a.fb || a.fp);
+  const int hi = si.pmode ? (si.Np - 1) / 2 : L, lo = si.pmode ? L - si.Np / 2 : 0;
+  const int m0 = j + (si.pmode ? si.Np / 2 : 0), m1 = j - (si.pmode ? L - si.Np / 2 : 0);
+  const long long sp = ROWS ? 1 : si.sp, step = (long long)nbf * sp;
+  for (int t = blockIdx.y; t < a.ntr; t += gridDim.y) {
+    float2 v[16];
+    if (line < a.nlines) {
+      const float2* in = a.in + (long long)t * si.st + side_line(si, la, lb);
+      const float2* p0 = in + (long long)(si.pmode == 1 ? m0 : j) * sp;
+      const float2* p1 = in + (long long)(si.pmode == 1 ? m1 : j) * sp;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int w = j + r * nbf;
+        v[r] = make_float2(0.f, 0.f);
+        if (r < 8 ? w <= hi : w >= lo) v[r] = (r < 8 ? p0 : p1)[r * step];
+      }
+      if (fac) {
+        const float f0 = line_factor(a, la, lb, -1);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+          const int w = j + r * nbf;
+          if (r < 8 ? w <= hi : w >= lo)
+            v[r] = cscale(v[r], (a.fp && si.pmode) ? f0 * __ldg(a.fp + (r < 8 ? m0 : m1) + r * nbf) : f0);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 16; ++r) v[r] = make_float2(0.f, 0.f);
+    }
+    Dft<float, 16>::run(v, (float)a.dir);
+    float2* l = buf + g * LP + j * 17;  // sidx(16 j)
+#pragma unroll
+    for (int r = 0; r < 16; ++r) l[r] = v[r];
+    __syncthreads();
+    float2* out = a.out + (long long)t * a.so.st;
+    constexpr int N16 = LGL / 4;
+    if constexpr (REM == 1) {
+      if constexpr (N16 == 3) fx_pass<LGL, 16, false, ROWS>(a, buf, out, 4, line0, LP);
+      fx_pass<LGL, 16, true, ROWS>(a, buf, out, LGL - 4, line0, LP);
+    } else {
+      fx_pass<LGL, 16, false, ROWS>(a, buf, out, 4, line0, LP);
+      fx_pass<LGL, REM, true, ROWS>(a, buf, out, 8, line0, LP);
+    }
+    __syncthreads();  // the buffer is reused by the next transform
+  }
+}
+
+using FxKernel = void (*)(const LineArgs<float>);
+inline FxKernel fx_kernel(int L, bool rows) {
+  switch (L) {
+    case 256: return rows ? k_line_fft_fx<8, true> : k_line_fft_fx<8, false>;
+    case 512: return rows ? k_line_fft_fx<9, true> : k_line_fft_fx<9, false>;
+    case 1024: return rows ? k_line_fft_fx<10, true> : k_line_fft_fx<10, false>;
+    case 2048: return rows ? k_line_fft_fx<11, true> : k_line_fft_fx<11, false>;
+    default: return rows ? k_line_fft_fx<12, true> : k_line_fft_fx<12, false>;
+  }
+}
+
 // Longest line: 8192 points FP32, 4096 FP64 (two padded buffers of ~68 KB)
 // for the generic kernel.
 template <typename T> constexpr int line_cap() { return sizeof(T) == 4 ? 8192 : 4096; }
@@ -613,6 +760,14 @@ cudaError_t line_fft_prepare() {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        2 * (line_cap<T>() + line_cap<T>() / 16 + 1) * (int)sizeof(cplx_t<T>));
   if (e != cudaSuccess) return e;
+  if constexpr (sizeof(T) == 4) {
+    const int bytes = 2 * line_p2_elems<T>() * 18 / 16 * (int)sizeof(cplx_t<T>);
+    for (int L = 256; L <= 4096; L *= 2)
+      for (int rows = 0; rows < 2; ++rows)
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(fx_kernel(L, rows != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+  }
   // G * (L + L/16 + 1) <= E * 18/16 for E = G * L <= twice line_p2_elems, L >= 16
   return cudaFuncSetAttribute(k_line_fft_p2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               2 * line_p2_elems<T>() * 18 / 16 * (int)sizeof(cplx_t<T>));
@@ -625,12 +780,32 @@ cudaError_t launch_line_fft(const LineArgs<T>& a, cudaStream_t s) {
     const int threads = a.G * a.L / 16;
     const size_t smem = (size_t)a.G * (a.L + a.L / 16 + 1) * sizeof(cplx_t<T>);
     dim3 grid((a.nlines + a.G - 1) / a.G, a.ntr < 65535 ? a.ntr : 65535);
+    if constexpr (sizeof(T) == 4) {
+      if (a.L >= 256 && a.L <= 4096) {
+        const size_t bytes = (size_t)a.G * fx_pitch(a.L, a.G) * sizeof(float2);
+        fx_kernel(a.L, a.si.sp == 1 && a.so.sp == 1)<<<grid, threads, bytes, s>>>(a);
+        return cudaGetLastError();
+      }
+    }
     k_line_fft_p2<T><<<grid, threads, smem, s>>>(a);
     return cudaGetLastError();
   }
   const size_t smem = 2 * (size_t)a.G * (a.L + a.L / 16 + 1) * sizeof(cplx_t<T>);
   dim3 grid((a.nlines + a.G - 1) / a.G, a.ntr < 65535 ? a.ntr : 65535);
   k_line_fft<T, line_cap<T>()><<<grid, kLineThreads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+// exp(dir 2 pi i m / n), m < n, rounded from FP64.
+__global__ void k_line_twiddles(float2* out, double dir, int n) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= n) return;
+  double re, im;
+  sincospi(2.0 * (double)m / (double)n, &im, &re);
+  out[m] = make_float2((float)re, (float)(dir * im));
+}
+cudaError_t launch_line_twiddles(float2* out, int dir, int n, cudaStream_t s) {
+  k_line_twiddles<<<(n + 127) / 128, 128, 0, s>>>(out, (double)dir, n);
   return cudaGetLastError();
 }
 

@@ -226,6 +226,8 @@ struct LineArgs {
   int fac_on_out;
 };
 
+cudaError_t launch_line_twiddles(float2* out, int dir, int n, cudaStream_t s);
+
 // Pruned power-of-two passes (halffft.cu) for grids nf in {256, ..., 2048}
 // with at most nf/2 modes per axis: per axis F = nf / Mp warp FFTs of Mp
 // points (one per output or input class q, grid position F r + q) over the
