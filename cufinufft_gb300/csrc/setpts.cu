@@ -13,7 +13,8 @@
 //     apart (kCountStride), or all atomics meet in a handful of L2 sectors;
 //   * k_bin_scan turns the counters into bin counts, bin starts and
 //     subproblem starts in one pass (two launches beyond 4096 bins);
-//   * k_permute writes the sorted structure-of-arrays copy the spread and
+//   * k_permute (large 3D FP32 sets: k_permute and k_gather_points) writes the
+//     sorted structure-of-arrays copy the spread and
 //     interp kernels stream -- caller index, first tap and offset per axis --
 //     and, in further blocks of the same launch, the subproblem headers (binary
 //     search, balanced even when one bin holds most of the points).  The
@@ -171,8 +172,23 @@ __device__ __forceinline__ void write_header(const SubHdrArgs& h, const int* sta
   h.hdr[sidx] = o;
 }
 
-// Blocks [0, pblocks) permute, the others write headers.
 template <typename T, int SRC>
+__device__ __forceinline__ void write_point(const PlaceArgs<T>& a, int pos, int idx, const int i0[3], const T d[3]) {
+  a.idx[pos] = idx;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (k < a.dim) {
+      a.i0[k][pos] = i0[k];
+      a.d[k][pos] = d[k];
+    }
+  }
+}
+
+// Blocks [0, pblocks) permute, the others write headers.  WHOLE writes every
+// point's sorted copy, seven scattered words in 3D, each a sector of its own; not
+// WHOLE writes only where the point came from, and k_gather_points reads the points
+// in sorted order and writes the copies in full lines.
+template <typename T, int SRC, bool WHOLE>
 __global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a, SubHdrArgs h, int pblocks) {
   if ((int)blockIdx.x >= pblocks) {
     const int sidx = ((int)blockIdx.x - pblocks) * blockDim.x + threadIdx.x;
@@ -196,15 +212,20 @@ __global__ void __launch_bounds__(kPlaceThreads) k_permute(PlaceArgs<T> a, SubHd
     else if (a.bank.cell_order == 2) pos = a.bank.cls_start[(long long)b * a.bank.ncls + order_class(a.bank, a.bs, lc)] + r;
     else if (a.bank.cell_order) pos = cell_position(a.bank, a.start, act, b, order_class(a.bank, a.bs, lc), r);
     else pos = a.start[b] + interleave_pos(a.bank, b, order_class(a.bank, a.bs, lc), r);
-    a.idx[pos] = SRC == kSrcStored ? a.src_idx[i] : i;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      if (k < a.dim) {
-        a.i0[k][pos] = i0[k];
-        a.d[k][pos] = d[k];
-      }
-    }
+    if (WHOLE) write_point<T, SRC>(a, pos, SRC == kSrcStored ? a.src_idx[i] : i, i0, d);
+    else a.idx[pos] = i;
   }
+}
+
+template <typename T, int SRC>
+__global__ void __launch_bounds__(kPlaceThreads) k_gather_points(PlaceArgs<T> a) {
+  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos >= a.M) return;
+  const int i = a.idx[pos];
+  int i0[3], lc[3];
+  T d[3];
+  point_bin<T, SRC>(a, i, i0, d, lc);
+  write_point<T, SRC>(a, pos, SRC == kSrcStored ? a.src_idx[i] : i, i0, d);
 }
 
 // gpu_sort = 0 with method 1 keeps the caller's order (reference "GM",
@@ -243,17 +264,37 @@ static void set_magic(const int bs[3], unsigned magic[3]) {
     default: KERNEL<T, kSrcCoords><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break;  \
   }
 
+#define CFG_SRC_SWITCH2(KERNEL, ARG, GRID, ...)                                        \
+  switch (a.src) {                                                                     \
+    case kSrcStored: KERNEL<T, kSrcStored, ARG><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break; \
+    case kSrcNarrow: KERNEL<T, kSrcNarrow, ARG><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break; \
+    default: KERNEL<T, kSrcCoords, ARG><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break;  \
+  }
+
 template <typename T> cudaError_t launch_bin_count(PlaceArgs<T> a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
   set_magic(a.bs, a.magic);
   CFG_SRC_SWITCH(k_bin_count, place_grid(a.M), a)
   return cudaGetLastError();
 }
+// 3D FP32 points from which the permutation goes in two steps (one / two, us: 1e6
+// points in 64^3 modes 37 / 28, 4e6 195 / 92; 3e5 14.5 / 12.3).  In 2D ordered
+// trajectories scatter into few lines anyway (radial, 1e6: 9.6 / 17), and FP64
+// points would be placed on the grid once more, which is bound by the FP64 unit
+// (1e6: 118 / 219).
+constexpr int kGatherPoints = 250000;
 template <typename T> cudaError_t launch_permute(PlaceArgs<T> a, const SubHdrArgs& h, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
   set_magic(a.bs, a.magic);
   const int pb = place_grid(a.M), hb = (h.nsub + kPlaceThreads - 1) / kPlaceThreads;
-  CFG_SRC_SWITCH(k_permute, pb + hb, a, h, pb)
+  if (sizeof(T) == 8 || a.src == kSrcNarrow || a.dim < 3 || a.M < kGatherPoints) {
+    CFG_SRC_SWITCH2(k_permute, true, pb + hb, a, h, pb)
+  } else {
+    CFG_SRC_SWITCH2(k_permute, false, pb + hb, a, h, pb)
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    CFG_SRC_SWITCH(k_gather_points, (a.M + kPlaceThreads - 1) / kPlaceThreads, a)
+  }
   return cudaGetLastError();
 }
 template <typename T> cudaError_t launch_place_unsorted(PlaceArgs<T> a, cudaStream_t s) {
