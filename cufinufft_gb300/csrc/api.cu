@@ -1141,7 +1141,11 @@ int resolve_nsub(Plan<T>* p, bool wait) {
   if (wait) {
     CFG_CUDA(cudaEventSynchronize(p->ev_total));
   } else {
+    // another thread's global-mode capture would forbid (and be ended by) the query
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     const cudaError_t e = cudaEventQuery(p->ev_total);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (e == cudaErrorNotReady) {
       cudaGetLastError();
       return 0;

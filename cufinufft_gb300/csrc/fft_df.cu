@@ -335,7 +335,7 @@ cudaError_t launch_line_fft_df(LineDfArgs d, cudaStream_t s) {
   const int threads = ((G * d.a.L + kDfValues - 1) / kDfValues + 31) / 32 * 32;
   const size_t smem = (size_t)G * (d.a.L + d.a.L / 8 + 1) * sizeof(float4);
   const bool pow2 = (d.a.L & (d.a.L - 1)) == 0;
-  if (smem > 48 * 1024) {
+  if (smem > 47 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(pow2 ? k_line_fft_df<true> : k_line_fft_df<false>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

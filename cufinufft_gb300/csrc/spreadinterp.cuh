@@ -2035,7 +2035,7 @@ size_t tile_bytes(int ns, const BinTables& bt) {
 
 template <typename K>
 cudaError_t prepare_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes <= 47 * 1024) return cudaSuccess;  // 48 KB with the kernel's static part
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
@@ -2098,7 +2098,7 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
         if (a.fp64_df) slab_df = slab_df_shape(NS, a.bins, (size_t)optin - 2048);  // less its static part
         slab = slab_bytes<T>(NS, a.bins) <= (size_t)optin;
         if constexpr (sizeof(T) == 4) {
-          col = slab && col_bins(a.bins) && col_bytes<NS>(a.bins) <= (size_t)optin &&
+          col = slab && col_bins(a.bins) && col_bytes<NS>(a.bins) + 1024 <= (size_t)optin &&
                 (double)a.M >= col_density(NS, a.run != 0) * (double)a.g.Nf;
         }
       }

@@ -44,3 +44,31 @@ def test_columns_against_global_atomics(crowded, tol, modes, bins, maxsub):
     for out in outs[1:]:
         # FP32 sums of up to ~1e4 terms per cell in another order
         assert np.linalg.norm(out - outs[0]) / np.linalg.norm(outs[0]) < 1e-5
+
+
+@pytest.mark.parametrize("tol", [10.0 ** -k for k in range(2, 8)])
+@pytest.mark.parametrize("bins", [None, (8, 8, 8), (16, 8, 8)])
+def test_wide_kernels(tol, bins):
+    """Upsampling 1.25: widths up to 14, among them one whose block takes 48 KB of
+    shared memory to the byte.  The grids themselves (spreading only): the
+    deconvolution would amplify their rounding by orders of magnitude."""
+    import torch
+
+    from cufinufft_gb300 import cufinufft
+    rng = np.random.default_rng(5)
+    grid = (36, 48, 40)
+    M = 100000
+    pts = [torch.from_numpy(p).cuda() for p in NC.points(rng, 3, M, dtype=np.float32, edges=False)]
+    c = torch.from_numpy(NC.strengths(rng, M, dtype=np.complex64)).cuda()
+    outs = []
+    for method, b in ((1, (8, 8, 8)), (2, bins)):
+        plan = cufinufft(1, grid[::-1], eps=tol, dtype=np.float32, upsampfac=1.25, gpu_spreadinterponly=1)
+        plan.set_pts(*pts[::-1])
+        if b:
+            plan.set_layout(method, b)
+        fk = torch.zeros(grid, dtype=c.dtype, device="cuda")
+        plan.execute(c, fk)
+        torch.cuda.synchronize()
+        outs.append(fk.cpu().numpy().astype(np.complex128))  # squares leave FP32's range
+    # FP32 sums of ns^3 taps of 1.4 points per cell in another order
+    assert np.linalg.norm(outs[1] - outs[0]) / np.linalg.norm(outs[0]) < 1e-5
