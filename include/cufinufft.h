@@ -107,7 +107,7 @@ typedef struct cufinufft_plan_info {
   int type, dim, ms, mt, mu, nf1, nf2, nf3, ns, M, ntransf, maxbatchsize;
   int method, sort, binsizex, binsizey, binsizez, nbins, nsubprob, kerevalmeth;
   double beta, es_c;
-  int line_fft;   /* 1: pruned line FFTs (fftpass.cu), 0: cuFFT over the whole grid */
+  int line_fft;   /* 1: pruned line FFTs (fftpass.cu; FP32 power-of-two grids of 2^20 cells or more, or asked for) */
   int cell_order; /* 1: method 2 spreading over cell-ordered points (cell-run kernel) */
   int width_rule; /* kernel-width rule the plan was made under (cufinufft_set_width_rule) */
   int chain_fp32; /* 1: an FP64 plan running its spread/interp, FFT and deconvolution in FP32 */
