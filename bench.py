@@ -788,7 +788,9 @@ def run_ours(args, w: Workload, rank, world, local_rank, extra=False):
                               "note": "same calls as a continuous stream: two plans on two "
                                       "streams alternate so one step's copies overlap the "
                                       "other's compute; no L2 flush between steps"}},
-        "gpu_launches": 2 * int(math.ceil(w.ntransf / max(info["maxbatchsize"], 1))) * args.steps,
+        # spread or interp, and the line FFT's passes or the mode rows beside cuFFT
+        "gpu_launches": (1 + (w.dim if info["line_fft"] or info["df_fft"] else 1)) *
+                        int(math.ceil(w.ntransf / max(info["maxbatchsize"], 1))) * args.steps,
         "roofline": roof,
         "cpu_baseline": cpu,
         "clocks": clk,
