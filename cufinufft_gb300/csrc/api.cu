@@ -1184,7 +1184,9 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   if (p->M == 0) return 0;
   const int method = p->route ? p->route : p->method;
   const int ms = method == 2 ? p->sort_ms : 0;
-  const bool cell = p->cell_order && method == 2;
+  // (1D windows sort by cell whatever the layout, see bank_order)
+  const bool windows = p->dim == 1 && p->variant == 0 && (is_single<T>() || p->fp64_df == 1);
+  const bool cell = p->cell_order && method == 2 && !windows;
   int e = bank_order(p, method, p->sort_bs, nbins, &a.bank, cell);  // zeroes its counters
   if (e) return e;
   BinScanArgs sc;
@@ -2308,9 +2310,9 @@ static cufinufft_tune_entry layout_class(const Plan<T>* p, int cls) {
   return e;
 }
 
-// The classes the autotuner and the selector choose among.  1D spreading runs one
-// kernel whatever the layout, so its cell-run classes are left out there
-// (set_layout and set_layout_class still take them).
+// The classes the autotuner times.  1D spreading runs one kernel and one sort
+// whatever the layout, so its cell-run classes are left out there (the selector,
+// set_layout and set_layout_class still take them).
 template <typename T>
 static std::vector<cufinufft_tune_entry> tune_candidates(const Plan<T>* p) {
   std::vector<cufinufft_tune_entry> c;
@@ -2488,7 +2490,8 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - kSelMean[k]) / kSelStd[k];
   selector_forward(f, y);
   int best = -1;
-  const std::vector<cufinufft_tune_entry> cand = tune_candidates(p);
+  std::vector<cufinufft_tune_entry> cand;
+  for (int k = 0; k < kLayoutClasses; ++k) cand.push_back(layout_class(p, k));
   for (int k = 0; k < CUFINUFFT_MLP_CLASSES; ++k) {
     if (cand[k].ms == -2.f) continue;
     if (best < 0 || y[k] < y[best]) best = k;
