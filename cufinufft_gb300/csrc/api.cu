@@ -21,8 +21,10 @@
 
 #include "plan.h"
 #include "selector_weights.h"
+#include "selector_weights_chain.h"
 
-static_assert(sizeof(cfg::kSelParams) == sizeof(float) * CUFINUFFT_MLP_PARAMS,
+static_assert(sizeof(cfg::kSelParams) == sizeof(float) * CUFINUFFT_MLP_PARAMS &&
+                  sizeof(cfg::chain_selector::kSelParams) == sizeof(float) * CUFINUFFT_MLP_PARAMS,
               "selector weights do not match the network shape");
 
 namespace cfg {
@@ -234,12 +236,15 @@ static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
 // (CUFINUFFT_FFT=line), or an FP32 grid of at least 2^20 cells whose sides are
 // powers of two from 256 to 4096 -- cuFFT with amplification or deconvolution / the
 // line passes, us: 2048^2 38 / 28, 1024^2 16.7 / 15.3, 256^3 135 / 71; smaller grids
-// are latency, where cuFFT's passes are the shorter: 512^2 11.2 / 14.5.
+// are latency, where cuFFT's passes are the shorter: 512^2 11.2 / 14.5.  Not for the
+// FP32 chain of an FP64 plan (see order_kept): its complex128 results would move by
+// 2.5e-7, three times what a sparse type 1 differs by between two calls.
 template <typename T>
 static bool use_line_fft(const Plan<T>* p) {
   const char* v = std::getenv("CUFINUFFT_FFT");
   if (v == nullptr) {
-    if (!is_single<T>() || p->dim < 2 || (p->type != 1 && p->type != 2) || grid_cells(p) < (1LL << 20)) return false;
+    if (!is_single<T>() || p->chain || p->dim < 2 || (p->type != 1 && p->type != 2) || grid_cells(p) < (1LL << 20))
+      return false;
     for (int k = 0; k < p->dim; ++k)
       if (!power_of_two(p->nf[k]) || p->nf[k] < 256 || p->nf[k] > 4096) return false;
     return true;
@@ -1282,6 +1287,16 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   return 0;
 }
 
+// The FP32 chain of an FP64 plan of type 2 returns complex128 values whose low bits are
+// its FP32 sums': gathered taps and tiles add them in another order, 1e-7 apart.  It
+// runs the method that it reports (gpu_method 0: chosen by a network that retraining
+// leaves alone), so that its values do not follow measured lines.  (Type 1 meets in
+// atomics, in another order on every call.)
+template <typename T>
+static bool order_kept(const Plan<T>* p) {
+  return p->chain && p->type == 2;
+}
+
 // The kernels, bins and subproblem cap of the coming sort.  A default plan --
 // no layout, bins or kernel variant asked for -- may run on others than it
 // reports; the values are the same up to the order of sums.
@@ -1318,7 +1333,7 @@ static void choose_route(Plan<T>* p) {
   int bs[3] = {p->bs[0], p->bs[1], p->bs[2]};
   const int ns = p->sp.ns;
   const double density = (double)p->M / (double)grid_cells(p);
-  const bool open = p->dim >= 2 && p->sort && !p->auto_method && !p->layout_set && p->variant == 0 &&
+  const bool open = p->dim >= 2 && p->sort && !p->auto_method && !p->layout_set && p->variant == 0 && !order_kept(p) &&
                     (is_single<T>() || p->fp64_df == 1 || (p->fp64_df && p->type == 2));
   const auto fit = [&](int x, int y, int z) {  // x * y * z bins, where the tile (and four copies in 2D) fits
     const int want[3] = {x, y, z};
@@ -1756,6 +1771,7 @@ static int makeplan_chain(Plan<double>* p, int type, int dim, const int* nmodes,
   p->lo = new (std::nothrow) Plan<float>();
   if (!p->lo) return CUFINUFFT_ERR_ALLOC;
   p->lo->device = p->device;
+  p->lo->chain = true;
   ier = makeplan_impl<float>(p->lo, type, dim, nmodes, iflag, ntransf, tol, maxbatchsize, opts, &sp);
   if (ier) return ier;
   sync_from_lo(p);
@@ -2460,10 +2476,9 @@ static int features_impl(Plan<T>* p, float* f) {
 // The network's outputs for one normalised feature vector, on the host: the
 // sums of cufinufft_mlp_forward in the same order (a batch of one is 2 kflops;
 // two copies, three launches and a wait cost ~40 us).
-static void selector_forward(const float* x, float* y) {
+static void selector_forward(const float* w, const float* x, float* y) {
   constexpr int F = CUFINUFFT_MLP_FEATURES, H = CUFINUFFT_MLP_HIDDEN, K = CUFINUFFT_MLP_CLASSES;
   float h1[H], h2[H];
-  const float* w = kSelParams;
   auto dense = [&](const float* in, int ni, float* out, int no, bool relu) {
     const float* bias = w + no * ni;
     for (int o = 0; o < no; ++o) {
@@ -2480,15 +2495,18 @@ static void selector_forward(const float* x, float* y) {
 
 // gpu_method 0 with a trained network: predict the twelve classes' relative
 // times from the points' features and take the fastest runnable one for the
-// coming sort.
+// coming sort.  Type-2 chains have a network of their own (order_kept).
 template <typename T>
 static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   if (!kSelectorTrained || !p->auto_method || p->M == 0) return 0;
   float f[CUFINUFFT_MLP_FEATURES], y[CUFINUFFT_MLP_CLASSES];
   const int e = features_of(p, src, f);
   if (e) return e;
-  for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - kSelMean[k]) / kSelStd[k];
-  selector_forward(f, y);
+  const bool kept = order_kept(p);
+  const float* mean = kept ? chain_selector::kSelMean : kSelMean;
+  const float* sd = kept ? chain_selector::kSelStd : kSelStd;
+  for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - mean[k]) / sd[k];
+  selector_forward(kept ? chain_selector::kSelParams : kSelParams, f, y);
   int best = -1;
   std::vector<cufinufft_tune_entry> cand;
   for (int k = 0; k < kLayoutClasses; ++k) cand.push_back(layout_class(p, k));

@@ -100,6 +100,7 @@ template <typename T> struct Plan {
   // Its sort folds and rescales this side's FP64 points in FP64 (kSrcNarrow);
   // this side converts c / fk (c32, fk32).
   Plan<float>* lo = nullptr;
+  bool chain = false;        // this plan is such a `lo`
   cplx_t<float>* c32 = nullptr;
   size_t c32_cap = 0;
   cplx_t<float>* fk32 = nullptr;
