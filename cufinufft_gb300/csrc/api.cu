@@ -188,8 +188,6 @@ template <typename T> static void release(Plan<T>* p) {
   p->cap_sub_dense = 0;
   if (p->h_total) cudaFreeHost(p->h_total);
   p->h_total = nullptr;
-  if (p->ev_total) cudaEventDestroy(p->ev_total);
-  p->ev_total = nullptr;
   if (p->h_status) cudaFreeHost(p->h_status);
   p->h_status = nullptr;
   p->d_status = nullptr;
@@ -908,7 +906,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
   CFG_CUDA(cudaStreamCreate(&p->own));  // blocking: ordered after the legacy default stream
   p->stream = p->own;
   CFG_CUDA(cudaMallocHost(&p->h_total, sizeof(int)));
-  CFG_CUDA(cudaEventCreateWithFlags(&p->ev_total, cudaEventDisableTiming));
+  if (const int e = alloc_bins(p, p->nbins)) return e;
   if (type == 2) {
     CFG_CUDA(cudaHostAlloc(&p->h_status, 2 * sizeof(int), cudaHostAllocMapped));
     p->h_status[0] = p->h_status[1] = 0;
@@ -1059,7 +1057,7 @@ static int bank_order(Plan<T>* p, int method, const int bs[3], int nbins, BankOr
   // 1D spreading sums neighbouring points in registers: sorted by cell where
   // cells hold points to share (half a point each on average), plain bins below
   const bool by_cell = !cell && p->type == 1 && p->dim == 1 && p->variant == 0 && 2LL * p->M >= p->nf[0] &&
-                       (long long)nbins * bs[0] <= (1LL << 24);
+                       (long long)nbins * bs[0] <= (1LL << 24) && !capturing(p);  // (allocates)
   if (method != 2 && !by_cell) return 0;
   if (cell || by_cell) {
     int cells = 1;
@@ -1140,38 +1138,23 @@ static int execute_chain(Plan<double>* p, double2* c, double2* fk);
 template <typename T>
 static int execute_t3(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk);
 
+// Whether the plan stream is being captured into a caller's graph.
 template <typename T>
-int resolve_nsub(Plan<T>* p, bool wait) {
-  if (p->nsub_exact) return 0;
-  if (wait) {
-    CFG_CUDA(cudaEventSynchronize(p->ev_total));
-  } else {
-    // another thread's global-mode capture would forbid (and be ended by) the query
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t e = cudaEventQuery(p->ev_total);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e == cudaErrorNotReady) {
-      cudaGetLastError();
-      return 0;
-    }
-    CFG_CUDA(e);
+static bool capturing(const Plan<T>* p) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
   }
-  p->nsub = *p->h_total;
-  p->nsub_exact = true;
-  return 0;
+  return cs != cudaStreamCaptureStatusNone;
 }
-template int resolve_nsub<float>(Plan<float>*, bool);
-template int resolve_nsub<double>(Plan<double>*, bool);
 
-// The sort of setpts and set_layout on the plan stream, no readback waited for:
-// counters, ranks, starts, permutation, and for method 2 the subproblem
+// The sort of setpts and set_layout, queued on the plan stream: counters, ranks, starts, permutation, and for method 2 the subproblem
 // headers.  a: the point source and the sorted arrays to fill; the layout is
 // the plan's.
 template <typename T>
 static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   p->nsub = 0;
-  p->nsub_exact = true;
   const int nbins = p->sort_nbins;
   {
     const int e = alloc_bins(p, nbins);
@@ -1281,9 +1264,19 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
     CFG_CUDA(launch_classify_subproblems(c, p->stream));
   }
   p->nsub = h.nsub;
-  p->nsub_exact = false;
-  CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + nbins, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-  CFG_CUDA(cudaEventRecord(p->ev_total, p->stream));
+  return 0;
+}
+
+// Waits for the sort, whose last kernel still reads the caller's coordinates (they
+// may be freed or overwritten on any stream once setpts returns), and takes the number
+// of subproblems with it.  Placed and counted from arrays that change on the way, a
+// point's slot could lie outside the plan's own.
+template <typename T>
+static int finish_sort(Plan<T>* p) {
+  if (p->nsub > 0)
+    CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + p->sort_nbins, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+  CFG_CUDA(cudaStreamSynchronize(p->stream));
+  if (p->nsub > 0) p->nsub = *p->h_total;
   return 0;
 }
 
@@ -1333,7 +1326,8 @@ static void choose_route(Plan<T>* p) {
   int bs[3] = {p->bs[0], p->bs[1], p->bs[2]};
   const int ns = p->sp.ns;
   const double density = (double)p->M / (double)grid_cells(p);
-  const bool open = p->dim >= 2 && p->sort && !p->auto_method && !p->layout_set && p->variant == 0 && !order_kept(p) &&
+  // (a sort that is being captured must not allocate, nor wait for its readback)
+  const bool open = p->dim >= 2 && p->sort && !p->auto_method && !p->layout_set && p->variant == 0 && !order_kept(p) && !capturing(p) &&
                     (is_single<T>() || p->fp64_df == 1 || (p->fp64_df && p->type == 2));
   const auto fit = [&](int x, int y, int z) {  // x * y * z bins, where the tile (and four copies in 2D) fits
     const int want[3] = {x, y, z};
@@ -1401,7 +1395,6 @@ static int setpts_from(Plan<T>* p, int M, PlaceArgs<T> a) {
   if (e) return e;
   p->M = M;
   p->nsub = 0;
-  p->nsub_exact = true;
   a.dim = p->dim;
   a.M = M;
   e = choose_layout(p, a);  // gpu_method 0: before the sort, from the points' occupancy
@@ -1421,6 +1414,9 @@ static int setpts_from(Plan<T>* p, int M, PlaceArgs<T> a) {
     if (e) return e;
   }
   CFG_CUDA(cudaGetLastError());
+  // (in a caller's capture nothing runs yet, and there is nothing to wait for;
+  // method 2 needs its readback there and is refused)
+  if (M > 0 && (p->method == 2 || !capturing(p)) && (e = finish_sort(p))) return e;
   p->pts_set = true;
   return 0;
 }
@@ -1655,11 +1651,7 @@ static int execute_impl(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
   if (p->type == 3) return execute_t3(p, c, fk);
   if (const int e = take_status(p)) return e;
   if (p->timing || !p->planned || !graphs_enabled()) return execute_direct(p, c, fk);
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(p->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return execute_direct(p, c, fk);
-  }
+  if (capturing(p)) return execute_direct(p, c, fk);
   if (p->gexec && p->g_c == c && p->g_fk == fk && p->g_version == p->version) {
     CFG_CUDA(cudaGraphLaunch(p->gexec, p->stream));
     return 0;
@@ -1672,8 +1664,7 @@ static int execute_impl(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk) {
   p->last_c = c;
   p->last_fk = fk;
   p->last_version = p->version;
-  if (const int e = resolve_nsub(p, false)) return e;
-  if (!again || !p->nsub_exact) return execute_direct(p, c, fk);
+  if (!again) return execute_direct(p, c, fk);
   if (cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
     const int e = execute_direct(p, c, fk);
     cudaGraph_t g = nullptr;
@@ -2112,7 +2103,6 @@ static int count_subproblems(Plan<T>* p, int* nsub) {
 
 template <typename T>
 static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
-  resolve_nsub(p, true);
   int nsub = p->method == 2 ? p->nsub : 0;
   if (p->route && p->method == 2) count_subproblems(p, &nsub);
   std::memset(info, 0, sizeof(*info));
@@ -2196,7 +2186,6 @@ static int adopt_layout(Plan<T>* p, int method, const int bsz[3], int maxsub) {
   if (method == 2) p->opts.gpu_maxsubprobsize = maxsub;
   p->nbins = (int)nbins;
   p->nsub = 0;
-  p->nsub_exact = true;
   return 0;
 }
 
@@ -2236,7 +2225,7 @@ static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub)
     p->i0[k] = a.i0[k];
     p->d[k] = a.d[k];
   }
-  return resolve_nsub(p, true);
+  return finish_sort(p);
 }
 
 // Device time (ms) of the plan's spread (type 1) or interp (type 2) stage for
@@ -2244,7 +2233,6 @@ static int set_layout_impl(Plan<T>* p, int method, const int bsz[3], int maxsub)
 template <typename T>
 static int time_stage(Plan<T>* p, cplx_t<T>* scratch, cplx_t<T>* grid, int reps, float* ms) {
   CFG_CUDA(cudaStreamSynchronize(p->stream));
-  if (const int er = resolve_nsub(p, true)) return er;
   SpreadArgs<T> a = spread_args(p);
   a.ntr = p->maxbatch;
   cudaEvent_t e0, e1;

@@ -227,13 +227,6 @@ static int batch_make(Batch<T>* b, int nplans, Plan<T>** plans) {
     if (p->opts.gpu_kerevalmeth != 0) return CUFINUFFT_ERR_ARG;
     if (p->spread_only) return CUFINUFFT_ERR_ARG;  // the batch runs whole transforms
     if (p->type == 3) return CUFINUFFT_ERR_ARG;    // types 1 and 2 only
-    if (p->lo) {
-      const int e = resolve_nsub(p->lo, true);
-      if (e) return e;
-    } else {
-      const int e = resolve_nsub(p, true);
-      if (e) return e;
-    }
     b->plans.push_back(p);
   }
   CFG_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));

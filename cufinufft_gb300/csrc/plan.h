@@ -119,11 +119,7 @@ template <typename T> struct Plan {
   cplx_t<T>* t3_grid = nullptr;       // [ntransf nf] spread grid
   size_t t3_capM = 0, t3_capN = 0, t3_capG = 0;
   double* t3_part = nullptr;          // min/max partials (device)
-  // subproblem count: nsub is its upper bound (surplus headers are empty) until
-  // the pinned readback h_total of the last sort has landed (ev_total)
-  int* h_total = nullptr;
-  cudaEvent_t ev_total = nullptr;
-  bool nsub_exact = true;
+  int* h_total = nullptr;  // pinned readback of the subproblem count
   // interpolation tile-wait status (SpreadArgs::status): host-mapped, two ints
   int* h_status = nullptr;
   int* d_status = nullptr;
@@ -263,10 +259,6 @@ template <typename T>
 int execute_plan(Plan<T>* p, cplx_t<T>* c, cplx_t<T>* fk);
 template <typename T>
 int plan_use_stream(Plan<T>* p, cudaStream_t s);
-// The subproblem count of the last sort from its readback, if that has landed
-// (wait: once it has); until then nsub is an upper bound.
-template <typename T>
-int resolve_nsub(Plan<T>* p, bool wait);
 
 template <typename T>
 inline cudaError_t run_spread(Plan<T>* p, const SpreadArgs<T>& a) {

@@ -17,16 +17,15 @@
 //     sorted structure-of-arrays copy the spread and
 //     interp kernels stream -- caller index, first tap and offset per axis --
 //     and, in further blocks of the same launch, the subproblem headers (binary
-//     search, balanced even when one bin holds most of the points).  The
-//     number of subproblems stays on the device: headers are written for its
-//     upper bound, the surplus empty, and the host learns the number when it
-//     next needs it.
+//     search, balanced even when one bin holds most of the points).  Headers
+//     are written for the upper bound of their number, the surplus empty; the
+//     host learns the number with the one wait that ends setpts (the caller's
+//     coordinates are read until the last of these kernels).
 // Points come from the caller's coordinates, from the plan's stored first
 // taps and offsets (a new layout), or from FP64 coordinates for an FP32 chain
 // (placed in FP64, the offset rounded afterwards).
-// 1e5 points, 512^2 grid: 12 launches, a readback and ~45 us of device time ->
-// 5 launches, none waited for; set_pts and execute together 130 -> 33 us a call
-// in a stream of calls.
+// 1e5 points, 512^2 grid: 12 launches and ~45 us of device time -> 5 launches;
+// set_pts and execute together 132 -> 64 us a call in a stream of calls.
 #include "device_common.cuh"
 #include "kernels.h"
 
