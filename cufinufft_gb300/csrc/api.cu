@@ -2071,12 +2071,12 @@ template int execute_plan<double>(Plan<double>*, cplx_t<double>*, cplx_t<double>
 template int plan_use_stream<float>(Plan<float>*, cudaStream_t);
 template int plan_use_stream<double>(Plan<double>*, cudaStream_t);
 
-// Subproblems of the plan's reported bins, for a plan sorted by a route's own.
+// Counts over the plan's reported bins of its stored points, into h.  The points
+// are complete (setpts and set_layout wait for their sorts), so this runs on a
+// stream of its own, and leaves alone what is being captured on the plan's stream
+// or by other threads.
 template <typename T>
-static int count_subproblems(Plan<T>* p, int* nsub) {
-  *nsub = 0;
-  if (p->M == 0) return 0;
-  std::vector<int> h((size_t)p->nbins);
+static cudaError_t reported_counts(const Plan<T>* p, std::vector<int>* h) {
   PlaceArgs<T> a;
   std::memset(&a, 0, sizeof(a));
   a.src = kSrcStored;
@@ -2088,23 +2088,46 @@ static int count_subproblems(Plan<T>* p, int* nsub) {
     a.bs[k] = p->bs[k];
     a.nb[k] = p->nb[k];
   }
-  CFG_CUDA(cudaMalloc(&a.count, sizeof(int) * h.size()));
-  cudaError_t e = cudaMemsetAsync(a.count, 0, sizeof(int) * h.size(), p->stream);
-  if (e == cudaSuccess) e = launch_feature_count<T>(a, p->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h.data(), a.count, sizeof(int) * h.size(), cudaMemcpyDeviceToHost, p->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+  const size_t bytes = sizeof(int) * h->size();
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMalloc(&a.count, bytes);
+  if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, bytes, s);
+  if (e == cudaSuccess) e = launch_feature_count<T>(a, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->data(), a.count, bytes, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFree(a.count);
-  CFG_CUDA(e);
-  const int ms = p->opts.gpu_maxsubprobsize;
-  for (int c : h) *nsub += c / ms + (c % ms ? 1 : 0);
+  if (s) cudaStreamDestroy(s);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return e;
+}
+
+// Subproblems of the plan's reported bins: those of the sort, or, for a plan sorted
+// by a route's own bins, a count kept until the points or the layout change.
+template <typename T>
+static int reported_subproblems(Plan<T>* p, int* nsub) {
+  *nsub = p->method == 2 ? p->nsub : 0;
+  if (p->method != 2 || !p->route || !p->pts_set || p->M == 0) return 0;
+  if (p->info_version != p->version) {
+    DeviceGuard g(p->device);
+    if (!g.ok) return CUFINUFFT_ERR_CUDA;
+    std::vector<int> h((size_t)p->nbins);
+    CFG_CUDA(reported_counts(p, &h));
+    const int ms = p->opts.gpu_maxsubprobsize;
+    p->info_nsub = 0;
+    for (int c : h) p->info_nsub += c / ms + (c % ms ? 1 : 0);
+    p->info_version = p->version;
+  }
+  *nsub = p->info_nsub;
   return 0;
 }
 
 template <typename T>
-static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
-  int nsub = p->method == 2 ? p->nsub : 0;
-  if (p->route && p->method == 2) count_subproblems(p, &nsub);
+static int fill_info(Plan<T>* p, cufinufft_plan_info* info) {
+  int nsub = 0;
+  if (const int e = reported_subproblems(p, &nsub)) return e;
   std::memset(info, 0, sizeof(*info));
   info->type = p->type;
   info->dim = p->dim;
@@ -2134,6 +2157,7 @@ static void fill_info(Plan<T>* p, cufinufft_plan_info* info) {
   info->fp64_df = p->type == 2 && p->fp64_df && p->method == 2 ? 1 : 0;  // the subproblem interpolation only
   info->cell_order = p->cell_order ? 1 : 0;
   info->width_rule = p->width_rule;
+  return 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2775,19 +2799,17 @@ int cufinufft_set_width_rule(int rule, int* previous) { return cfg::set_width_ru
 int cufinufft_get_info(cufinufft_plan plan, cufinufft_plan_info* info) {
   if (!plan || !info) return CUFINUFFT_ERR_GENERIC;
   if (plan->p.lo) {
-    cfg::fill_info(plan->p.lo, info);
+    if (const int e = cfg::fill_info(plan->p.lo, info)) return e;
     info->beta = plan->p.sp.beta;  // the FP64 plan's kernel (the chain's is beta, c rounded to FP32)
     info->es_c = plan->p.sp.c;
     info->chain_fp32 = 1;
     return 0;
   }
-  cfg::fill_info(&plan->p, info);
-  return 0;
+  return cfg::fill_info(&plan->p, info);
 }
 int cufinufftf_get_info(cufinufftf_plan plan, cufinufft_plan_info* info) {
   if (!plan || !info) return CUFINUFFT_ERR_GENERIC;
-  cfg::fill_info(&plan->p, info);
-  return 0;
+  return cfg::fill_info(&plan->p, info);
 }
 
 }  // extern "C"

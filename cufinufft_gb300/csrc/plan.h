@@ -120,6 +120,9 @@ template <typename T> struct Plan {
   size_t t3_capM = 0, t3_capN = 0, t3_capG = 0;
   double* t3_part = nullptr;          // min/max partials (device)
   int* h_total = nullptr;  // pinned readback of the subproblem count
+  // subproblems of the reported bins, for the plan state of info_version (plan info)
+  int info_nsub = 0;
+  unsigned info_version = 0;
   // interpolation tile-wait status (SpreadArgs::status): host-mapped, two ints
   int* h_status = nullptr;
   int* d_status = nullptr;
