@@ -2039,6 +2039,11 @@ cudaError_t prepare_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Room for the static shared memory of a double-float kernel (its table of 64 float
+// pairs, the tile header, a maximum: ~560 bytes) beside the dynamic part; tiles that
+// leave less take the FP64 kernels.
+constexpr size_t kDfStaticSmem = 1024;
+
 // CUFINUFFT_TC_SPREAD=1: the dense runs of 3D FP32 cell-run subproblems go
 // to the tensor-core kernel (k_spread_sm_run_tc).
 inline bool tc_spread_enabled() {
@@ -2077,10 +2082,11 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
     bool slab = false, split = false, priv = false;
     [[maybe_unused]] bool col = false;
     [[maybe_unused]] SlabDfShape slab_df{0, 0, 0};
+    [[maybe_unused]] int optin = 0;
     if constexpr (DIM == 2) {
       priv = a.variant == 0 && priv_spread_enabled();
       if (priv) {  // the private copies and stages must fit (else the atomic kernel)
-        int dev = 0, optin = 0;
+        int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (e != cudaSuccess) return e;
@@ -2091,7 +2097,7 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
     if constexpr (DIM == 3) {
       slab = a.variant == 0 && slab_spread_enabled();
       if (slab) {  // its padded tile and staging must fit (else the atomic kernel)
-        int dev = 0, optin = 0;
+        int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (e != cudaSuccess) return e;
@@ -2112,8 +2118,8 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
     // run in FP64 registers costs five times the double-float taps, so the
     // cell-run layout needs no second kernel)
     if constexpr (sizeof(T) == 8 && DIM == 2) {
-      if (a.fp64_df && priv) {
-        const size_t smb = priv_df_bytes(NS, a.bins);
+      const size_t smb = priv_df_bytes(NS, a.bins);
+      if (a.fp64_df && priv && smb + kDfStaticSmem <= (size_t)optin) {
         cudaError_t e = prepare_smem(k_spread_sm_priv_df<NS>, smb);
         if (e != cudaSuccess) return e;
         k_spread_sm_priv_df<NS><<<dim3(a.bins.nsub, a.ntr), 32 * kPrivDfWarps, smb, s>>>(a);
