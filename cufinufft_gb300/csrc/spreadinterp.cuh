@@ -2229,6 +2229,16 @@ cudaError_t interp_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
     if (a.bins.nsub == 0) return cudaSuccess;
     if (!wc && a.bins.hdr == nullptr) return cudaErrorInvalidValue;  // k_interp_sm reads the headers
     size_t sm = tile_bytes<T, DIM>(NS, a.bins);
+    [[maybe_unused]] bool df = false;  // double-float, where its static part fits beside the tile
+    if constexpr (sizeof(T) == 8) {
+      if (!wc && a.fp64_df) {
+        int dev = 0, optin = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e != cudaSuccess) return e;
+        df = sm + kDfStaticSmem <= (size_t)optin;
+      }
+    }
     CUtensorMap gmap;
     int tma = 0;
     if (!wc) {
@@ -2242,12 +2252,12 @@ cudaError_t interp_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (e != cudaSuccess) return e;
-        if (smb <= (size_t)optin) sm = smb;
+        if (smb + (df ? kDfStaticSmem : 64) <= (size_t)optin) sm = smb;  // beside the static part
         else tma = 0;
       }
     }
     if constexpr (sizeof(T) == 8) {
-      if (!wc && a.fp64_df) {
+      if (df) {
         cudaError_t e = prepare_smem(k_interp_sm_df<DIM, NS>, sm);
         if (e != cudaSuccess) return e;
         k_interp_sm_df<DIM, NS><<<dim3(a.bins.nsub, a.ntr), interp_threads_f64<DIM>(), sm, s>>>(a, gmap, tma);

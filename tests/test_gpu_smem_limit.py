@@ -26,3 +26,9 @@ def _against_default_bins(ntype, modes, bins, tol, ns):
                                          ((18, 51), 1e-13, 14), ((33, 51), 1e-13, 14), ((66, 23), 1e-10, 11)])
 def test_spread_private_tiles(bins, tol, ns):
     _against_default_bins(1, (60, 44), bins, tol, ns)
+
+
+@pytest.mark.parametrize("modes,bins,tol,ns", [((20, 34, 20), (13, 26, 15), 1e-7, 8), ((20, 20, 34), (13, 15, 26), 1e-7, 8),
+                                               ((20, 24, 28), (13, 18, 22), 1e-7, 8), ((20, 24, 28), (13, 18, 21), 1e-7, 8)])
+def test_interpolation_tiles(bins, modes, tol, ns):
+    _against_default_bins(2, modes, bins, tol, ns)
