@@ -159,10 +159,13 @@ struct DeviceGuard {
   }
 };
 
+// (the error is taken out of the runtime's record, or the next launch check on this
+// thread, of any plan, would report it again)
 #define CFG_CUDA(call)                                             \
   do {                                                             \
     cudaError_t e_ = (call);                                       \
     if (e_ != cudaSuccess) {                                       \
+      cudaGetLastError();                                          \
       fprintf(stderr, "cufinufft: %s failed: %s\n", #call, cudaGetErrorString(e_)); \
       return e_ == cudaErrorMemoryAllocation ? CUFINUFFT_ERR_ALLOC : CUFINUFFT_ERR_CUDA; \
     }                                                              \
