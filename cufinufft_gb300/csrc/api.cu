@@ -922,6 +922,11 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
     const char* v = std::getenv("CUFINUFFT_FP64_DF");
     p->fp64_df = v && v[0] == '0' ? 0 : (v && v[0] == '1' ? 1 : (tol >= 1e-13 ? 1 : 0));
     if (type == 1 && p->spread_only) p->fp64_df = 0;
+    // Interpolation alone reads the caller's grid, which may span decades inside a
+    // tile, with no transform to spread the largest value's rounding: only the strict
+    // form of the tile kernel, for plans that asked for tiles (1e8 beside ones, ns 11:
+    // biased sums lose half the digits of the ones).
+    if (type == 2 && p->spread_only && p->fp64_df) p->fp64_df = 2;
     // Below upsampfac 2 the deconvolution factors amplify the grid's rounding
     // (1.25: ten thousandfold at ns 16, where it would show beside the
     // kernel's error: 7.79e-10 -> 7.95e-10 in 2D type 1).  Type 1 keeps FP64
@@ -1328,7 +1333,7 @@ static void choose_route(Plan<T>* p) {
   const double density = (double)p->M / (double)grid_cells(p);
   // (a sort that is being captured must not allocate, nor wait for its readback)
   const bool open = p->dim >= 2 && p->sort && !p->auto_method && !p->layout_set && p->variant == 0 && !order_kept(p) && !capturing(p) &&
-                    (is_single<T>() || p->fp64_df == 1 || (p->fp64_df && p->type == 2));
+                    (is_single<T>() || p->fp64_df == 1 || (p->fp64_df && p->type == 2 && !p->spread_only));
   const auto fit = [&](int x, int y, int z) {  // x * y * z bins, where the tile (and four copies in 2D) fits
     const int want[3] = {x, y, z};
     int t[3];
