@@ -1191,13 +1191,15 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   std::memset(&sc, 0, sizeof(sc));
   sc.raw = p->count;
   sc.raw_stride = sc.per = 1;
+  const long long keys = (long long)nbins * (a.bank.cls_count ? a.bank.ncls : 1);
+  a.crowded_keys = a.bank.cell_order != 1 && crowded_sort(keys, p->M) ? (int)keys : 0;
   if (a.bank.cell_order == 2) {
     sc.cell_start = p->cls_start;
     sc.ncell = a.bank.ncls;
   } else if (a.bank.cls_count && !a.bank.cell_order) {
     sc.raw = a.bank.cls_count;
     sc.raw_stride = sc.per = a.bank.ncls;
-  } else if (!a.bank.cls_count && nbins <= kCountStrideBins) {
+  } else if (!a.bank.cls_count && nbins <= kCountStrideBins && !a.crowded_keys) {
     sc.raw = p->raw;
     sc.raw_stride = kCountStride;
   }

@@ -74,8 +74,20 @@ template <typename T> struct PlaceArgs {
   // plain bin order: the counter of bin b is raw[b raw_stride] (zeroed)
   int* raw;
   int raw_stride;
+  int crowded_keys;        // counters in all (adjacent ones) where blocks count for themselves first, else 0
   BankOrder bank;
 };
+// Sorts whose points crowd few counters: every atomic of the chip (one per distinct
+// counter and warp) would meet on them, so a block counts its points in shared memory
+// and adds each counter once.  set_pts, by warps / by blocks (us), 2e6 points: FP32 6
+// bins 266 / 62, 59 bins 318 / 76, 64 bank classes 396 / 112, 600 cells 302 / 104, 4096
+// cells 167 / 113; FP64 6 bins 335 / 190, 600 cells 351 / 201, 2048 classes 336 / 346;
+// 4e5 points, 4096 counters 69 / 63, 1e5 points in 600 cells 60 / 53; fewer points
+// do not fill the chip so (2e4: 43 / 49).
+constexpr int kCrowdedKeys = 4096, kCrowdedPoints = 128, kCrowdedLeast = 65536;
+inline bool crowded_sort(long long keys, long long M) {
+  return keys <= kCrowdedKeys && M >= kCrowdedLeast && M >= kCrowdedPoints * keys;
+}
 // Bins whose counters, one int each, would share few L2 sectors (all atomics
 // of a sort meet there: 1e5 points in 256 bins, 19 us) get a sector each.
 constexpr int kCountStride = 8, kCountStrideBins = 8192;

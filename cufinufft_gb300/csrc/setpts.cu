@@ -10,7 +10,9 @@
 //     counts sum to the bin's -- with one warp-aggregated atomic (one per
 //     distinct key in a warp, so clustered points do not serialise on one
 //     counter); a few thousand bins or fewer keep their counters a sector
-//     apart (kCountStride), or all atomics meet in a handful of L2 sectors;
+//     apart (kCountStride), or all atomics meet in a handful of L2 sectors,
+//     and where many points share a counter blocks count in shared memory
+//     first (k_bin_count_crowded);
 //   * k_bin_scan turns the counters into bin counts, bin starts and
 //     subproblem starts in one pass (two launches beyond 4096 bins);
 //   * k_permute (large 3D FP32 sets: k_permute and k_gather_points) writes the
@@ -142,7 +144,40 @@ __global__ void __launch_bounds__(kPlaceThreads) k_bin_count(PlaceArgs<T> a) {
   }
 }
 
-// Subproblem headers (k_sub_headers' part of k_permute): the subproblem's bin
+// The same for few counters (crowded_sort): a block ranks its points in shared
+// memory, reserves its share of every counter with one atomic, and adds the base it
+// got.  Key and rank of a point wait in one register (12 + 13 bits).
+template <typename T, int SRC, int U>
+__global__ void __launch_bounds__(kPlaceThreads) k_bin_count_crowded(PlaceArgs<T> a) {
+  __shared__ int s_count[kCrowdedKeys];
+  static_assert(kCrowdedKeys <= 1 << 12 && U * kPlaceThreads <= 1 << 13, "key and rank share an int");
+  for (int k = threadIdx.x; k < a.crowded_keys; k += kPlaceThreads) s_count[k] = 0;
+  __syncthreads();
+  const long long base = (long long)blockIdx.x * (U * kPlaceThreads) + threadIdx.x;
+  int at[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + u * kPlaceThreads;
+    if (i >= a.M) continue;
+    int i0[3], lc[3];
+    T d[3];
+    const int b = point_bin<T, SRC>(a, (int)i, i0, d, lc);
+    const int key = a.bank.cls_count ? b * a.bank.ncls + order_class(a.bank, a.bs, lc) : b;
+    at[u] = key << 13 | atomicAdd(&s_count[key], 1);
+  }
+  __syncthreads();
+  int* counter = a.bank.cls_count ? a.bank.cls_count : a.raw;
+  for (int k = threadIdx.x; k < a.crowded_keys; k += kPlaceThreads)
+    if (s_count[k]) s_count[k] = atomicAdd(counter + k, s_count[k]);
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + u * kPlaceThreads;
+    if (i < a.M) a.rank[i] = s_count[at[u] >> 13] + (at[u] & 0x1fff);
+  }
+}
+
+// Subproblem headers (a part of k_permute): the subproblem's bin
 // by binary search, its point range (subproblem js of bin b: points start[b] +
 // js maxsub, at most maxsub of them) and its tile origin (the bin's first
 // cell); subproblems past the total, up to the bound the host launches with,
@@ -270,9 +305,20 @@ static void set_magic(const int bs[3], unsigned magic[3]) {
     default: KERNEL<T, kSrcCoords, ARG><<<GRID, kPlaceThreads, 0, s>>>(__VA_ARGS__); break;  \
   }
 
+template <typename T, int U> static cudaError_t count_crowded(const PlaceArgs<T>& a, cudaStream_t s) {
+  CFG_SRC_SWITCH2(k_bin_count_crowded, U, (a.M + U * kPlaceThreads - 1) / (U * kPlaceThreads), a)
+  return cudaGetLastError();
+}
 template <typename T> cudaError_t launch_bin_count(PlaceArgs<T> a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
   set_magic(a.bs, a.magic);
+  if (a.crowded_keys > 0) {
+    // points per thread: many share a block's counters, few even out the blocks (FP64
+    // placement is arithmetic)
+    const bool wide = a.M >= 152 * 32 * kPlaceThreads;
+    if (sizeof(T) == 8 || a.src == kSrcNarrow) return wide ? count_crowded<T, 8>(a, s) : count_crowded<T, 4>(a, s);
+    return wide ? count_crowded<T, 32>(a, s) : count_crowded<T, 8>(a, s);
+  }
   CFG_SRC_SWITCH(k_bin_count, place_grid(a.M), a)
   return cudaGetLastError();
 }
