@@ -255,6 +255,7 @@ inline SpreadArgs<T> spread_args(Plan<T>* p) {
   a.sub_ndense = a.run ? p->sub_ndense : nullptr;
   a.status = p->d_status;
   a.tma_wait_test = p->tma_wait_test;
+  a.unsorted = p->method == 1 && p->sort == 0 ? 1 : 0;
   a.fp64_df = p->fp64_df;
   return a;
 }
