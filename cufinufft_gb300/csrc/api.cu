@@ -1322,7 +1322,7 @@ static bool order_kept(const Plan<T>* p) {
 // 16x16x2 bins / these (us): FP32 2D 16^2 from 0.35 points per cell 1e6 points
 // 68 / 61 (512^2), below it 58 / 80 (4e5 points, 1024^2); FP64 2D 16^2 557 / 303
 // (1e6, 512^2), for ns > 11 from 0.15 points per cell 693 / 491 (below 585 / 684);
-// FP32 3D 16x8x4 212 / 202 (4e5, 64^3, ns 8), 8^3 from col_density 1164 / 803 (4e6); FP64 3D
+// FP32 3D 16x8x4 212 / 202 (4e5, 64^3, ns 8), 8^3 for columns (column_spread) 1164 / 803 (4e6); FP64 3D
 // 8^3 3936 / 3187 (1e6, 100x96x100, ns 10), for ns > 11 16x16x4 7563 / 6947.
 //
 // A subproblem is one block, so a crowded bin's thousand points take as long as
@@ -1354,6 +1354,7 @@ static void choose_route(Plan<T>* p) {
     while (ms < 1024 && (long long)ms * share < (long long)p->M * p->maxbatch) ms *= 2;
     p->sort_ms = std::min(p->sort_ms, ms);
   };
+  const int deep[3] = {std::min(8, p->nf[0]), std::min(8, p->nf[1]), std::min(8, p->nf[2])};
   if (open && p->type == 2 && p->method == 1 && p->opts.gpu_maxsubprobsize >= 256) {
     if (p->dim == 3 && p->bins_default) is_single<T>() ? fit(16, 16, 8) : fit(8, 8, 8);
     double taps = density, cells = 1.0;
@@ -1369,10 +1370,9 @@ static void choose_route(Plan<T>* p) {
       for (int k = 0; k < 3; ++k) bs[k] = p->bs[k];
     }
   } else if (is_single<T>() && p->type == 1 && p->dim == 3 && p->auto_method && !p->layout_set && p->cell_order &&
-             density >= col_density(ns, true)) {
+             column_spread(ns, true, density, deep, p->sort_ms)) {
     // the chosen cell-run layout, in bins whose columns hold more to share
     // (3.2e7 half-clustered points, 256^3: 8.14 -> 5.65 ms)
-    const int deep[3] = {std::min(8, p->nf[0]), std::min(8, p->nf[1]), std::min(8, p->nf[2])};
     long long nb = 1;
     for (int k = 0; k < 3; ++k) nb *= (p->nf[k] + deep[k] - 1) / deep[k];
     if (cell_order_fits(p, deep, nb) && run_smem_bytes(p, deep) <= (size_t)max_smem_optin(p->device)) {
@@ -1381,13 +1381,11 @@ static void choose_route(Plan<T>* p) {
     }
   } else if (open && p->type == 1 && p->method == 2 && !p->cell_order && p->bins_default) {
     p->route = 2;
-    if (p->dim == 2 && (is_single<T>() ? density >= 0.35 : (ns <= 11 || density >= 0.15))) fit(16, 16, 1);
-    if (p->dim == 3 && is_single<T>()) {
-      if (density >= col_density(ns, false)) fit(8, 8, 8);  // spread_col.cuh
-      else fit(16, 8, 4);
-    }
-    if (p->dim == 3 && !is_single<T>() && ns <= 13) ns <= 11 ? fit(8, 8, 8) : fit(16, 16, 4);
     cap(128, 2048);
+    if (p->dim == 2 && (is_single<T>() ? density >= 0.35 : (ns <= 11 || density >= 0.15))) fit(16, 16, 1);
+    const bool columns = p->dim == 3 && is_single<T>() && column_spread(ns, false, density, deep, p->sort_ms);
+    if (p->dim == 3 && is_single<T>()) columns ? fit(8, 8, 8) : fit(16, 8, 4);
+    if (p->dim == 3 && !is_single<T>() && ns <= 13) ns <= 11 ? fit(8, 8, 8) : fit(16, 16, 4);
   }
   p->sort_nbins = 1;
   for (int k = 0; k < 3; ++k) {

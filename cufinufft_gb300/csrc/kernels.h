@@ -116,10 +116,22 @@ template <typename T> cudaError_t launch_bin_count(PlaceArgs<T> a, cudaStream_t 
 template <typename T> cudaError_t launch_permute(PlaceArgs<T> a, const SubHdrArgs& h, cudaStream_t s);
 template <typename T> cudaError_t launch_place_unsorted(PlaceArgs<T> a, cudaStream_t s);
 
-// Points per grid cell from which 3D FP32 spreading orders a bin's points by
-// column (spread_col.cuh): on plain bins -- narrow kernels need more to repay the
-// sort -- and on a cell-run layout, whose dense cells go to another kernel.
-constexpr double col_density(int ns, bool run) { return run || ns < 6 ? 1.0 : 0.4; }
+// Whether 3D FP32 spreading of a method-2 layout orders a subproblem's points by column
+// (spread_col.cuh) rather than by plane alone (the slab kernel): where a column of a
+// mean subproblem holds points to share.  density: points per grid cell; run: cell-run
+// layout, whose dense cells go to another kernel.  Execute, slab / columns (us), 192^3
+// cells: ns 6, 8^3 bins of at most 1024 points, density 0.7 2083 / 1499, 2 5676 / 2931;
+// 16x16x2 bins of at most 256 points (one a column) 0.7 2211 / 2299.  Narrow kernels
+// have few taps to save and need more: ns 5, 8^3 bins, density 1 (eight points a column)
+// 1660 / 1822, 2 (sixteen) 3206 / 2894; at most 256 points 3482 / 5259; 16x16x2 bins 2996 /
+// 3857; ns 4 1341 / 1197, 2552 / 1976, 2799 / 3287, 2194 / 2379.
+inline bool column_spread(int ns, bool run, double density, const int bs[3], int maxsub) {
+  const double cells = (double)bs[0] * bs[1] * bs[2];
+  const double points = density * cells < maxsub ? density * cells : (double)maxsub;
+  const double column = points / ((double)bs[0] * bs[1]);
+  if (ns < 6) return column >= 12.0 && (!run || density >= 4.0);
+  return density >= (run ? 1.0 : 0.4) && points >= 64.0 && (column >= 1.2 || density >= 2.0);
+}
 
 // Complex FP64 <-> FP32 conversion of n values.
 cudaError_t launch_narrow_complex(const double2* in, float2* out, long long n, cudaStream_t s);

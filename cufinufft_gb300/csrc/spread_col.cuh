@@ -23,8 +23,8 @@
 // Spread stage, slab / this kernel (us), best bins of each: even points, ns 8: 4e6
 // in 128^3 cells 1609 / 803, 3.2e7 in 256^3 12284 / 5981; half of them clustered
 // 12391 / 6450; 0.5 points per cell 3294 / 2855, 0.2 202 / 239; 1.9 points per cell ns
-// 7 1736 / 820, ns 6 1465 / 775, ns 4 616 / 529 (0.5: 175 / 199) -- hence
-// col_density.  Cell-run layout, 3.2e7 half-clustered points 8267 / 5650.
+// 7 1736 / 820, ns 6 1465 / 775, ns 4 616 / 529 (0.5: 175 / 199); the line is
+// column_spread's.  Cell-run layout, 3.2e7 half-clustered points 8267 / 5650.
 #pragma once
 
 #include "df.cuh"

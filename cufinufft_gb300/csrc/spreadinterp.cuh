@@ -2108,7 +2108,7 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
         slab = slab_bytes<T>(NS, a.bins) <= (size_t)optin;
         if constexpr (sizeof(T) == 4) {
           col = slab && col_bins(a.bins) && col_bytes<NS>(a.bins) + 1024 <= (size_t)optin &&
-                (double)a.M >= col_density(NS, a.run != 0) * (double)a.g.Nf;
+                column_spread(NS, a.run != 0, (double)a.M / (double)a.g.Nf, a.bins.bs, a.bins.maxsub);
         }
       }
       // cell-run layout: the slab kernel also takes the sparse tails of the
