@@ -1386,6 +1386,17 @@ static void choose_route(Plan<T>* p) {
     const bool columns = p->dim == 3 && is_single<T>() && column_spread(ns, false, density, deep, p->sort_ms);
     if (p->dim == 3 && is_single<T>()) columns ? fit(8, 8, 8) : fit(16, 8, 4);
     if (p->dim == 3 && !is_single<T>() && ns <= 13) ns <= 11 ? fit(8, 8, 8) : fit(16, 16, 4);
+    // A cap below an even bin's points splits every bin, which costs a tile each time:
+    // not where the bins fill the chip by themselves (us, split / whole: 2D FP32 32^2 bins,
+    // 2e5 points, 1000^2 cells 45 / 38; 3D columns, 1.3e5, 64^3 106 / 81, half of them
+    // clustered 100 / 71; planes, 4.4e5, 96^3 146 / 132, clustered 131 / 155).
+    double mean = (double)p->M, bins = 1.0;
+    for (int k = 0; k < p->dim; ++k) bins *= (p->nf[k] + bs[k] - 1) / bs[k];
+    mean /= bins;
+    const bool shared = p->dim == 2 ? is_single<T>() && bs[0] > 16 : columns;
+    if (bins >= (shared ? 2 * 152 : 1000) && (shared || p->dim == 3))
+      while (p->sort_ms < (shared ? 1024 : 512) && p->sort_ms < 1.25 * mean) p->sort_ms *= 2;
+    p->sort_ms = std::min(p->sort_ms, p->opts.gpu_maxsubprobsize);
   }
   p->sort_nbins = 1;
   for (int k = 0; k < 3; ++k) {
