@@ -1055,12 +1055,6 @@ static size_t run_smem_bytes(const Plan<T>* p, const int bs[3]) {
          (size_t)(256 / 32) * 32 * sizeof(cplx_t<T>);
 }
 
-// 1D spreading by register windows (spread_win.cuh), whatever the layout.
-template <typename T>
-static bool spreads_windows(const Plan<T>* p) {
-  return p->type == 1 && p->dim == 1 && p->variant == 0 && (is_single<T>() || p->fp64_df == 1);
-}
-
 template <typename T>
 static int bank_order(Plan<T>* p, int method, const int bs[3], int nbins, BankOrder* o,
                       bool cell = false) {
@@ -1184,7 +1178,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   const int method = p->route ? p->route : p->method;
   const int ms = method == 2 ? p->sort_ms : 0;
   // (1D windows sort by cell whatever the layout, see bank_order)
-  const bool cell = p->cell_order && method == 2 && !spreads_windows(p);
+  const bool cell = p->cell_order && method == 2 && !layout_is_order(p);
   int e = bank_order(p, method, p->sort_bs, nbins, &a.bank, cell);  // zeroes its counters
   if (e) return e;
   BinScanArgs sc;

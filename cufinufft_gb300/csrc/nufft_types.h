@@ -126,7 +126,7 @@ template <typename T> struct SpreadArgs {
   // next call on the plan reads; null: not recorded.
   int* status;
   int tma_wait_test;        // nonzero: every tile's first wait gives up at once (tests)
-  int unsorted;             // the points are in the caller's order
+  int windows;              // 1D type 1: register windows (spreads_windows)
   int fp64_df;              // FP64: double-float kernels (1), or only the tile interpolation, strictest form (2)
 };
 

@@ -218,6 +218,25 @@ inline AxisMap<T> axis_map(int nf, int ns) {
   return a;
 }
 
+// 1D spreading by register windows (spread_win.cuh), whatever the layout, which only
+// orders the points.  FP32 points in the caller's order may jump every time, a whole
+// window of sums each: 1e6 points, 300 modes, execute 154 us by a warp's lanes, 390 by
+// windows (ordered 5e4: 19 and 13); in double-float the rows cost more than that (2e5
+// modes 793 / 190).  Few FP32 points on few-point cells do not repay a thread's run
+// either: method 1, lanes / windows, 2e3 points, 1001 modes 13 / 15, 2e5, 2e4 modes 21 /
+// 24, but 1e6, 2e5 modes 48 / 40; method 2 (16 / 13 by a tile's atomics) 11 by lanes
+// and 13 by windows for 2e3 points, 300 modes.
+template <typename T>
+inline bool layout_is_order(const Plan<T>* p) {
+  return p->type == 1 && p->dim == 1 && p->variant == 0 && (is_single<T>() || p->fp64_df == 1);
+}
+template <typename T>
+inline bool spreads_windows(const Plan<T>* p) {
+  if (!layout_is_order(p) || !is_single<T>()) return layout_is_order(p);
+  const bool few = (long long)p->M * p->maxbatch < (p->method == 1 ? 250000 : 25000) && p->M < 16LL * p->nf[0];
+  return !few && !(p->method == 1 && p->sort == 0);
+}
+
 template <typename T>
 inline SpreadArgs<T> spread_args(Plan<T>* p) {
   SpreadArgs<T> a;
@@ -255,7 +274,7 @@ inline SpreadArgs<T> spread_args(Plan<T>* p) {
   a.sub_ndense = a.run ? p->sub_ndense : nullptr;
   a.status = p->d_status;
   a.tma_wait_test = p->tma_wait_test;
-  a.unsorted = p->method == 1 && p->sort == 0 ? 1 : 0;
+  a.windows = spreads_windows(p) ? 1 : 0;
   a.fp64_df = p->fp64_df;
   return a;
 }

@@ -2065,11 +2065,8 @@ cudaError_t spread_ns(int method, const SpreadArgs<T>& a, cudaStream_t s) {
   if (a.M == 0) return cudaSuccess;
   const bool wc = a.variant != 1;
   if constexpr (DIM == 1) {
-    // 1D: windows in registers whatever the layout (it only orders the points).  FP32
-    // points in the caller's order may jump every time, a whole window of sums each:
-    // 1e6 points, 300 modes, execute 154 us by a warp's lanes, 390 by windows (ordered
-    // 5e4: 19 and 13); in double-float the rows cost more than that (2e5 modes 793 / 190).
-    if (a.variant == 0 && (sizeof(T) == 4 ? !a.unsorted : a.fp64_df == 1)) return launch_spread_win<T, NS>(a, s);
+    if (a.windows) return launch_spread_win<T, NS>(a, s);
+    if (sizeof(T) == 4 && a.variant == 0) method = 1;  // too few points for a tile as well
   }
   if (method == 1) {
     if (wc) {
