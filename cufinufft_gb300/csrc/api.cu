@@ -934,8 +934,8 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
     if (p->fp64_df && p->opts.upsampfac < 2.0) p->fp64_df = type == 2 ? 2 : 0;
   }
   if constexpr (sizeof(T) == 8) {
-    // double-float FFT of 2D power-of-two grids (types 1 and 2), under the
-    // same tol gate; CUFINUFFT_FP64_DF_FFT=0 keeps cuFFT's Z2Z
+    // double-float line FFTs (which grids: use_line_df), under the same tol
+    // gate; CUFINUFFT_FP64_DF_FFT=0 keeps cuFFT's Z2Z
     const char* v = std::getenv("CUFINUFFT_FP64_DF_FFT");
     const char* w = std::getenv("CUFINUFFT_FP64_DF");
     const bool gate = w && w[0] == '0' ? false : (w && w[0] == '1' ? true : tol >= 1e-13);

@@ -198,7 +198,6 @@ __device__ __forceinline__ DF df_from(double v) {
   r.l = __double2float_rn(v - (double)r.h);
   return r;
 }
-__device__ __forceinline__ double df_to(DF a) { return (double)a.h + (double)a.l; }
 // s + e = a + b exactly
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   s = __fadd_rn(a, b);
@@ -226,7 +225,6 @@ __device__ __forceinline__ DF df_mul(DF a, DF b) {
   return df_renorm(p, e);
 }
 // acc + a * b
-__device__ __forceinline__ DF df_fma(DF a, DF b, DF acc) { return df_add(acc, df_mul(a, b)); }
 
 // ---- packed FP32 pairs (sm_100+) -----------------------------------------
 // c + a * b on both halves of a float2 in one instruction (CUDA's

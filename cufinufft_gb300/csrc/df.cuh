@@ -20,7 +20,6 @@ __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y
 struct DF2 {
   float2 h, l;
 };
-__device__ __forceinline__ DF2 df2(float2 h, float2 l) { return DF2{h, l}; }
 __device__ __forceinline__ DF2 df2_dup(DF a) { return DF2{dup2(a.h), dup2(a.l)}; }
 // s + e = a + b exactly (Knuth); fast_two_sum2 needs |a| >= |b| (Dekker)
 __device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e) {

@@ -23,7 +23,8 @@
 // R-point DFT in registers and writes them to (j/Ns) Ns R + k + r Ns of a
 // second buffer; passes alternate between the two.  Radices 8, 4, 2, 5, 3 cover the 2,3,5-smooth
 // lengths next235beven produces.  Twiddles exp(dir 2 pi i m / L) come from a
-// per-axis table computed on the host in extended precision.
+// per-axis table, rounded from FP64 on the device (FP32) or from extended
+// precision on the host (FP64).
 #include "device_common.cuh"
 #include "linemap.cuh"
 

@@ -127,7 +127,7 @@ template <typename T> struct Plan {
   int* h_status = nullptr;
   int* d_status = nullptr;
   int tma_wait_test = 0;   // CUFINUFFT_TMA_WAIT_TEST=1 at makeplan
-  int fp64_df = 0;         // FP64 type 2: double-float subproblem interpolation
+  int fp64_df = 0;         // FP64: double-float spreading and interpolation (SpreadArgs::fp64_df)
   // execute as a CUDA graph (timing off): captured when a call repeats the
   // last one's caller arrays and plan state (`version` counts setpts /
   // set_layout); g_*: what the graph was captured for, last_*: the last call

@@ -332,14 +332,20 @@ template <typename T> cudaError_t launch_permute(PlaceArgs<T> a, const SubHdrArg
   if (a.M == 0) return cudaSuccess;
   set_magic(a.bs, a.magic);
   const int pb = place_grid(a.M), hb = (h.nsub + kPlaceThreads - 1) / kPlaceThreads;
-  if (sizeof(T) == 8 || a.src == kSrcNarrow || a.dim < 3 || a.M < kGatherPoints) {
-    CFG_SRC_SWITCH2(k_permute, true, pb + hb, a, h, pb)
-  } else {
-    CFG_SRC_SWITCH2(k_permute, false, pb + hb, a, h, pb)
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    CFG_SRC_SWITCH(k_gather_points, (a.M + kPlaceThreads - 1) / kPlaceThreads, a)
+  if constexpr (sizeof(T) == 4) {
+    if (a.src != kSrcNarrow && a.dim == 3 && a.M >= kGatherPoints) {
+      const int gb = (a.M + kPlaceThreads - 1) / kPlaceThreads;
+      if (a.src == kSrcStored) {
+        k_permute<T, kSrcStored, false><<<pb + hb, kPlaceThreads, 0, s>>>(a, h, pb);
+        k_gather_points<T, kSrcStored><<<gb, kPlaceThreads, 0, s>>>(a);
+      } else {
+        k_permute<T, kSrcCoords, false><<<pb + hb, kPlaceThreads, 0, s>>>(a, h, pb);
+        k_gather_points<T, kSrcCoords><<<gb, kPlaceThreads, 0, s>>>(a);
+      }
+      return cudaGetLastError();
+    }
   }
+  CFG_SRC_SWITCH2(k_permute, true, pb + hb, a, h, pb)
   return cudaGetLastError();
 }
 template <typename T> cudaError_t launch_place_unsorted(PlaceArgs<T> a, cudaStream_t s) {

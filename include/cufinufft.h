@@ -18,8 +18,9 @@
  *   - the stages may be repeated: 1234, 123334 and 1232334 are valid;
  *   - return value 0 = success; makeplan swallows the tolerance warning (1).
  * Differences, by design:
- *   - setpts copies the bin-sorted, rescaled points into plan memory, so the
- *     coordinate arrays may be freed or reused after setpts returns;
+ *   - setpts copies the bin-sorted, rescaled points into plan memory and waits
+ *     for that, so the coordinate arrays may be freed or reused after setpts
+ *     returns (recorded into a caller's graph: once the graph has run);
  *   - CUDA and cuFFT failures are returned as error codes (the reference
  *     calls exit() inside the library);
  *   - work is queued on a plan-owned blocking stream (ordered after the
@@ -79,10 +80,11 @@ int cufinufftf_setpts(int M, float* x, float* y, float* z, int N, float* s,
 
 /* Run ntransf transforms: type 1 reads c (ntransf*M) and writes fk
  * (ntransf*N1*N2*N3); type 2 reads fk and writes c.  Replaces
- * CUFINUFFT_EXECUTE, src/cufinufft.cu:495-569.  With stage timing off the
- * launch sequence is captured as a CUDA graph the first time a pair (c, fk)
- * is seen and replayed after that; setpts / set_layout, or other arrays,
- * capture it again (CUFINUFFT_GRAPH=0: direct launches every time). */
+ * CUFINUFFT_EXECUTE, src/cufinufft.cu:495-569.  With stage timing off a call
+ * that repeats the one before it (same c, fk, points and layout) captures the
+ * launch sequence as a CUDA graph and later ones replay it; after setpts /
+ * set_layout, or with other arrays, the next call launches directly again
+ * (CUFINUFFT_GRAPH=0: every call does). */
 int cufinufft_execute(cuDoubleComplex* c, cuDoubleComplex* fk,
                       cufinufft_plan plan);
 int cufinufftf_execute(cuFloatComplex* c, cuFloatComplex* fk,
@@ -113,7 +115,8 @@ typedef struct cufinufft_plan_info {
   int chain_fp32; /* 1: an FP64 plan running its spread/interp, FFT and deconvolution in FP32 */
   int half_fft;   /* 1: pruned power-of-two FFT passes (halffft.cu) instead of cuFFT */
   int fp64_df;    /* 1: an FP64 type-2 method-2 plan interpolating in double-float (FP32 pairs) */
-  int df_fft;     /* 1: an FP64 2D plan transforming its grid in double-float (fft_df.cu) */
+  int df_fft;     /* 1: an FP64 plan of a 2D power-of-two grid that transforms it in double-float (fft_df.cu;
+                   *    other grids do so without this flag) */
 } cufinufft_plan_info;
 int cufinufft_get_info(cufinufft_plan plan, cufinufft_plan_info* info);
 int cufinufftf_get_info(cufinufftf_plan plan, cufinufft_plan_info* info);
