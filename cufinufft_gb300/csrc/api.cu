@@ -905,7 +905,7 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
 
   CFG_CUDA(cudaStreamCreate(&p->own));  // blocking: ordered after the legacy default stream
   p->stream = p->own;
-  CFG_CUDA(cudaMallocHost(&p->h_total, sizeof(int)));
+  CFG_CUDA(cudaHostAlloc(&p->h_total, sizeof(int), cudaHostAllocMapped));
   if (const int e = alloc_bins(p, p->nbins)) return e;
   if (type == 2) {
     CFG_CUDA(cudaHostAlloc(&p->h_status, 2 * sizeof(int), cudaHostAllocMapped));
@@ -1207,6 +1207,7 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
   sc.start = p->start;
   sc.sub_start = p->sub_start;
   sc.partial = p->scan_part;
+  if (ms > 0) CFG_CUDA(cudaHostGetDevicePointer(&sc.total, p->h_total, 0));  // (a copy of its own took 3 us)
   CFG_CUDA(launch_bin_count<T>(a, p->stream));
   if (a.bank.cell_order)
     CFG_CUDA(launch_scan(p->cls_count, p->cls_start, nbins * a.bank.ncls, a.bank.cell_order == 1 ? 2 : 0,
@@ -1279,8 +1280,6 @@ static int sort_points(Plan<T>* p, PlaceArgs<T> a) {
 // point's slot could lie outside the plan's own.
 template <typename T>
 static int finish_sort(Plan<T>* p) {
-  if (p->nsub > 0)
-    CFG_CUDA(cudaMemcpyAsync(p->h_total, p->sub_start + p->sort_nbins, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
   CFG_CUDA(cudaStreamSynchronize(p->stream));
   if (p->nsub > 0) p->nsub = *p->h_total;
   return 0;
@@ -1430,7 +1429,7 @@ static int setpts_from(Plan<T>* p, int M, PlaceArgs<T> a) {
   }
   CFG_CUDA(cudaGetLastError());
   // (in a caller's capture nothing runs yet, and there is nothing to wait for;
-  // method 2 needs its readback there and is refused)
+  // method 2 needs its subproblem count there and is refused)
   if (M > 0 && (p->method == 2 || !capturing(p)) && (e = finish_sort(p))) return e;
   p->pts_set = true;
   return 0;

@@ -108,6 +108,7 @@ struct BinScanArgs {
   const int* cell_start;  // cell_order 2: scanned cell counts (ncell per bin) instead of raw
   int ncell;
   int *count, *start, *sub_start;
+  int* total;             // pinned host word for the number of subproblems, or null
   unsigned long long* partial;
 };
 int bin_scan_partials(int nbins);

@@ -119,7 +119,7 @@ template <typename T> struct Plan {
   cplx_t<T>* t3_grid = nullptr;       // [ntransf nf] spread grid
   size_t t3_capM = 0, t3_capN = 0, t3_capG = 0;
   double* t3_part = nullptr;          // min/max partials (device)
-  int* h_total = nullptr;  // pinned readback of the subproblem count
+  int* h_total = nullptr;  // subproblem count of the last sort (pinned; written by the bin scan)
   // subproblems of the reported bins, for the plan state of info_version (plan info)
   int info_nsub = 0;
   unsigned info_version = 0;
