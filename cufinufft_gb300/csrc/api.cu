@@ -2542,7 +2542,17 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   }
   if (best < 0) return 0;
   const int bs[3] = {cand[best].binsizex, cand[best].binsizey, cand[best].binsizez};
-  return adopt_layout(p, cand[best].method, bs, cand[best].maxsubprobsize);
+  int ms = cand[best].maxsubprobsize;
+  if (p->type == 2 && cand[best].method == 2 && ms < 1024 && !order_kept(p)) {
+    // bins that fill subproblems of 1024 only load their tiles more often in smaller
+    // ones (2.6e7 points, 66x56x64 cells, ns 5, 16x16x4 bins: cap 256 1027 us, 1024 806;
+    // 4e6, 400^2, 32^2 bins 79 / 68), which the network takes the other way where there
+    // are far more points than it was trained on
+    long long bins = 1;
+    for (int k = 0; k < p->dim; ++k) bins *= (p->nf[k] + bs[k] - 1) / bs[k];
+    if (p->M >= 1024 * bins) ms = 1024;
+  }
+  return adopt_layout(p, cand[best].method, bs, ms);
 }
 
 template <typename T>

@@ -1,0 +1,38 @@
+"""gpu_method 0, type 2, bins of more than 1024 points each: whatever class the network
+takes, full subproblems (their number is at most one more per bin than 1024 points each
+need), and the result of the gather kernels up to FP32 rounding."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("modes,M,eps,spread", [((33, 28, 32), 26000000, 1e-3, 0.05), ((33, 28, 32), 8000000, 1e-5, None),
+                                                ((200, 180), 6000000, 1e-4, None)])
+def test_full_subproblems(modes, M, eps, spread):
+    import torch
+
+    from cufinufft_gb300 import cufinufft
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    pts = []
+    for _ in modes:
+        x = (torch.rand(M, generator=g, device="cuda") * 2 - 1) * 3.1415
+        if spread:
+            x[M // 2:] = 0.4 + spread * torch.randn(M - M // 2, generator=g, device="cuda")
+        pts.append(x)
+    fk = torch.randn(modes, generator=g, device="cuda", dtype=torch.complex64)
+    outs = []
+    for method in (0, 1):
+        plan = cufinufft(2, modes, eps=eps, dtype=np.float32, gpu_method=method)
+        plan.set_pts(*pts)
+        i = plan.info()
+        c = torch.zeros(M, dtype=torch.complex64, device="cuda")
+        if method == 1:
+            plan.set_layout(1, (32,) * len(modes))
+        plan.execute(c, fk)
+        torch.cuda.synchronize()
+        outs.append(c)
+        if method == 0 and i["method"] == 2 and M >= 1024 * i["nbins"]:
+            assert i["nsubprob"] <= M // 1024 + i["nbins"], i
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2e-5
