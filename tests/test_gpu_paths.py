@@ -29,7 +29,7 @@ def _names(ntype, modes, M, dt, tol, **kw):
     ((64, 128), 1e-9, 2), ((9, 15, 27), 1e-9, 3), ((9, 15, 27), 1e-14, 0), ((50, 81), 1e-5, 0), ((2100, 10), 1e-9, 0)])
 def test_df_fft(monkeypatch, ntype, modes, tol, passes):
     names = _names(ntype, modes, 3000, np.float64, tol)
-    assert names.count("k_line_fft_df") == passes and ("fft<" in names) == (passes == 0)
+    assert names.count("k_line_fft_df") == passes and ("fft" in names.replace("k_line_fft", "")) == (passes == 0)
     monkeypatch.setenv("CUFINUFFT_FP64_DF_FFT", "0")
     assert "k_line_fft_df" not in _names(ntype, modes, 3000, np.float64, tol)
 
