@@ -2529,6 +2529,10 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   const int e = features_of(p, src, f);
   if (e) return e;
   const bool kept = order_kept(p);
+  // trained on single transforms, the network has no say on their number: its weights
+  // for that input are the random ones it began with (three transforms, type 1:
+  // 4e5 points, 3D FP32, 1003 us by them, 614 without; 1e5 points, 2D FP32 210 / 133)
+  if (!kept) f[8] = 0.f;
   const float* mean = kept ? chain_selector::kSelMean : kSelMean;
   const float* sd = kept ? chain_selector::kSelStd : kSelStd;
   for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - mean[k]) / sd[k];
