@@ -233,7 +233,8 @@ inline bool layout_is_order(const Plan<T>* p) {
 template <typename T>
 inline bool spreads_windows(const Plan<T>* p) {
   if (!layout_is_order(p) || !is_single<T>()) return layout_is_order(p);
-  const bool few = (long long)p->M * p->maxbatch < (p->method == 1 ? 250000 : 25000) && p->M < 16LL * p->nf[0];
+  const bool few = (long long)p->M * p->maxbatch < (p->method == 1 || p->auto_method ? 250000 : 25000) &&
+                   p->M < 16LL * p->nf[0];
   return !few && !(p->method == 1 && p->sort == 0);
 }
 

@@ -64,3 +64,10 @@ def test_fp32_tile_route(modes, M, kw, kernel):
 def test_fp32_line_fft(ntype, modes, line):
     names = _names(ntype, modes, 3000, np.float32, 1e-5)
     assert ("k_line_fft_fx" in names) == line and names.count("k_line_fft") == (len(modes) if line else 0)
+
+
+@pytest.mark.parametrize("M,kw,windows", [
+    (30000, {}, True), (3000, {}, False), (30000, dict(gpu_method=1), False), (300000, dict(gpu_method=1), True),
+    (30000, dict(gpu_method=0), False), (300000, dict(gpu_method=0), True)])
+def test_fp32_1d_spread(M, kw, windows):
+    assert ("k_spread_win<" in _names(1, (20001,), M, np.float32, 1e-5, **kw)) == windows
