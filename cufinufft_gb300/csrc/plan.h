@@ -225,7 +225,13 @@ inline AxisMap<T> axis_map(int nf, int ns) {
 // modes 793 / 190).  Few FP32 points on few-point cells do not repay a thread's run
 // either: method 1, lanes / windows, 2e3 points, 1001 modes 13 / 15, 2e5, 2e4 modes 21 /
 // 24, but 1e6, 2e5 modes 48 / 40; method 2 (16 / 13 by a tile's atomics) 11 by lanes
-// and 13 by windows for 2e3 points, 300 modes.
+// and 13 by windows for 2e3 points, 300 modes; gpu_method 0, whose classes in 1D differ in
+// bins alone, 17 and 21 for 3e4 points, 5003 modes.  Nor do sparse ones, whatever their
+// number, where a run's next point has left the window behind: below half a point per
+// cell (where the sort keeps bins) 4e5 points, 1.8e6 cells 49 / 54, four transforms of
+// them 138 / 191 (method 2 by a tile's atomics 167); with several transforms, which hide
+// what one waits for, below one: 1e6 points 178 / 216, on a line in order 190 / 164; 4e5,
+// 6e5 cells 71 / 88 and 69 / 64.
 template <typename T>
 inline bool layout_is_order(const Plan<T>* p) {
   return p->type == 1 && p->dim == 1 && p->variant == 0 && (is_single<T>() || p->fp64_df == 1);
@@ -235,7 +241,8 @@ inline bool spreads_windows(const Plan<T>* p) {
   if (!layout_is_order(p) || !is_single<T>()) return layout_is_order(p);
   const bool few = (long long)p->M * p->maxbatch < (p->method == 1 || p->auto_method ? 250000 : 25000) &&
                    p->M < 16LL * p->nf[0];
-  return !few && !(p->method == 1 && p->sort == 0);
+  const bool sparse = (p->maxbatch > 1 ? 1LL : 2LL) * p->M < p->nf[0];
+  return !few && !sparse && !(p->method == 1 && p->sort == 0);
 }
 
 template <typename T>

@@ -18,8 +18,9 @@ def _names(ntype, modes, M, dt, tol, **kw):
     rng = np.random.default_rng(M)
     plan = cufinufft(ntype, modes[::-1], eps=tol, dtype=dt, **kw)
     plan.set_pts(*[torch.from_numpy(p).cuda() for p in NC.points(rng, len(modes), M, dtype=dt, edges=False)][::-1])
-    c = torch.from_numpy(NC.strengths(rng, M, dtype=cd)).cuda()
-    fk = torch.from_numpy(NC.coeffs(rng, modes, dtype=cd)).cuda()
+    nt = kw.get("n_trans", 1)
+    c = torch.from_numpy(NC.strengths(rng, M, nt, dtype=cd)).cuda()
+    fk = torch.from_numpy(NC.coeffs(rng, modes, nt, dtype=cd)).cuda()
     return launched(lambda: plan.execute(c, fk))
 
 
@@ -71,3 +72,11 @@ def test_fp32_line_fft(ntype, modes, line):
     (30000, dict(gpu_method=0), False), (300000, dict(gpu_method=0), True)])
 def test_fp32_1d_spread(M, kw, windows):
     assert ("k_spread_win<" in _names(1, (20001,), M, np.float32, 1e-5, **kw)) == windows
+
+
+@pytest.mark.parametrize("M,nt,windows", [(100000, 1, True), (99999, 1, False), (200000, 4, True), (199999, 4, False)])
+def test_sparse_1d_points(M, nt, windows):
+    from cufinufft_gb300 import cufinufft
+    assert cufinufft(1, (100000,), eps=1e-5, dtype=np.float32).info()["nf1"] == 200000
+    kw = dict(gpu_method=2, n_trans=nt, maxbatchsize=nt)
+    assert ("k_spread_win<" in _names(1, (100000,), M, np.float32, 1e-5, **kw)) == windows
