@@ -2548,13 +2548,16 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   const int bs[3] = {cand[best].binsizex, cand[best].binsizey, cand[best].binsizez};
   int ms = cand[best].maxsubprobsize;
   if (p->type == 2 && cand[best].method == 2 && ms < 1024 && !order_kept(p)) {
-    // bins that fill subproblems of 1024 only load their tiles more often in smaller
-    // ones (2.6e7 points, 66x56x64 cells, ns 5, 16x16x4 bins: cap 256 1027 us, 1024 806;
-    // 4e6, 400^2, 32^2 bins 79 / 68), which the network takes the other way where there
-    // are far more points than it was trained on
+    // Crowded bins only load their tiles more often in smaller subproblems, which the
+    // network takes the other way where there are far more points than it was trained on.
+    // Cap 256 / 1024 (us), FP32, 4e6 points, 400^2 cells: ns 4..7, bins of 16 to 64, even,
+    // clustered and radial 73 / 60 to 92 / 83; 8e6 and 2.5e7, 66x60x64 cells 595 / 353 (16x16x2,
+    // ns 5, even) to 2091 / 2127 (8^3, ns 7, radial).  Fewer points need the small blocks:
+    // 1e6, 400^2 33 / 41 (32^2, ns 7, radial), 2e6, 66x60x64 203 / 234 (8^3, ns 7, radial); so
+    // do radial ones of some 1500 a bin (3e7, 8^3, 2931 / 3169).
     long long bins = 1;
     for (int k = 0; k < p->dim; ++k) bins *= (p->nf[k] + bs[k] - 1) / bs[k];
-    if (p->M >= 1024 * bins) ms = 1024;
+    if (p->M >= 4096 * std::max(bins, 1024LL)) ms = 1024;
   }
   return adopt_layout(p, cand[best].method, bs, ms);
 }
