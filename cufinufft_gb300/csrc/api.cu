@@ -2533,6 +2533,7 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   // for that input are the random ones it began with (three transforms, type 1:
   // 4e5 points, 3D FP32, 1003 us by them, 614 without; 1e5 points, 2D FP32 210 / 133)
   if (!kept) f[8] = 0.f;
+  const bool sparse = f[7] < 0.f, even = f[11] < 1.f;  // under a point per cell; peak under twice the mean
   const float* mean = kept ? chain_selector::kSelMean : kSelMean;
   const float* sd = kept ? chain_selector::kSelStd : kSelStd;
   for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - mean[k]) / sd[k];
@@ -2545,6 +2546,14 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
     if (best < 0 || y[k] < y[best]) best = k;
   }
   if (best < 0) return 0;
+  // 2D FP32 type 2: the network's classes lie close together for one call, not for plans
+  // that run side by side, where the chip is full and each tile load counts.  Below a point
+  // per cell 32^2 bins instead of 16^2 make the single call faster too (0.94 of the time on
+  // average over a sweep; 1.01 above), and so do whole bins of even points where there are
+  // enough of them (0.94, below).  61 plans of a batch, 9e4 to 9e5 points each, ns 6: 1004 us
+  // without, 964 with both.
+  const bool flat = is_single<T>() && p->dim == 2 && p->type == 2 && cand[best].method == 2 && !kept;
+  if (flat && sparse && best <= 4 && cand[best + 2].ms != -2.f) best += 2;
   const int bs[3] = {cand[best].binsizex, cand[best].binsizey, cand[best].binsizez};
   int ms = cand[best].maxsubprobsize;
   if (p->type == 2 && cand[best].method == 2 && ms < 1024 && !order_kept(p)) {
@@ -2557,7 +2566,7 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
     // do radial ones of some 1500 a bin (3e7, 8^3, 2931 / 3169).
     long long bins = 1;
     for (int k = 0; k < p->dim; ++k) bins *= (p->nf[k] + bs[k] - 1) / bs[k];
-    if (p->M >= 4096 * std::max(bins, 1024LL)) ms = 1024;
+    if (p->M >= 4096 * std::max(bins, 1024LL) || (flat && even && bins >= 2 * 152)) ms = 1024;
   }
   return adopt_layout(p, cand[best].method, bs, ms);
 }

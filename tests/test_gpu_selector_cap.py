@@ -36,3 +36,22 @@ def test_full_subproblems(modes, M, eps, spread):
         if method == 0 and i["method"] == 2 and M >= 4096 * max(i["nbins"], 1024):
             assert i["nsubprob"] <= M // 1024 + i["nbins"], i
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2e-5
+
+
+@pytest.mark.parametrize("modes,M,sparse", [((438, 671), 1100000, True), ((323, 219), 274583, True), ((314, 515), 435715, True),
+                                            ((239, 501), 142454, True), ((235, 296), 911085, False), ((180, 200), 150001, False)])
+def test_even_points_of_a_plan_among_others(modes, M, sparse):
+    """2D FP32 type 2, uniform points: no 16^2 bins below one point per cell, and the bins
+    that fill the chip are not split at 256 points."""
+    import torch
+
+    from cufinufft_gb300 import cufinufft
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    plan = cufinufft(2, modes, eps=1e-5, dtype=np.float32, gpu_method=0)
+    plan.set_pts(*[(torch.rand(M, generator=g, device="cuda") * 2 - 1) * 3.1415 for _ in modes])
+    i = plan.info()
+    assert (M < i["nf1"] * i["nf2"]) == sparse
+    if i["method"] == 2:
+        assert not sparse or min(i["binsizex"], i["binsizey"]) >= 32, i
+        assert i["nbins"] < 304 or i["nsubprob"] <= M // 1024 + i["nbins"], i
