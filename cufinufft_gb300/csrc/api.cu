@@ -277,7 +277,8 @@ static bool use_line_df(Plan<T>* p) {
   if (std::getenv("CUFINUFFT_FFT")) return false;  // line / half forms asked for
   const int cap = fft_df_cap();
   const bool pow2 = p->dim == 2 && power_of_two(p->nf[0]) && power_of_two(p->nf[1]);
-  if (p->opts.upsampfac < 2.0 && !pow2) return false;
+  const bool wide = p->type == 1 && p->sp.ns > 14 && !p->fp64_df;  // (see fp64_df)
+  if ((p->opts.upsampfac < 2.0 || wide) && !pow2) return false;
   p->fold[0] = p->fold[1] = 0;
   if (p->dim == 1 && p->nf[0] > cap) {
     // the factor pair nearest to square
@@ -919,9 +920,13 @@ static int makeplan_impl(Plan<T>* p, int type, int dim, const int* nmodes, int i
     // at any tol.  Type-1 spreading without a transform keeps FP64: there an
     // infinite strength stays one (as a float pair it becomes a NaN, which a
     // transform spreads over every mode either way).
+    // Type 1 wider than 14 keeps FP64 too: that kernel's own error, 4e-14 and less, does
+    // not cover the sums' (1001 modes, clustered points, tol 1e-13 by the tolerance rule: 7e-15
+    // -> 1.1e-14; at width 14 3.96e-13 -> 3.99e-13 at most; type 2 unchanged at any).
     const char* v = std::getenv("CUFINUFFT_FP64_DF");
+    const bool wide = type == 1 && p->sp.ns > 14 && !(v && v[0] == '1');
     p->fp64_df = v && v[0] == '0' ? 0 : (v && v[0] == '1' ? 1 : (tol >= 1e-13 ? 1 : 0));
-    if (type == 1 && p->spread_only) p->fp64_df = 0;
+    if (type == 1 && (p->spread_only || wide)) p->fp64_df = 0;
     // Interpolation alone reads the caller's grid, which may span decades inside a
     // tile, with no transform to spread the largest value's rounding: only the strict
     // form of the tile kernel, for plans that asked for tiles (1e8 beside ones, ns 11:
