@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(kPlaceThreads) k_bin_count_crowded(PlaceArgs<T
 // Subproblem headers (a part of k_permute): the subproblem's bin
 // by binary search, its point range (subproblem js of bin b: points start[b] +
 // js maxsub, at most maxsub of them) and its tile origin (the bin's first
-// cell); subproblems past the total, up to the bound the host launches with,
-// are empty.
+// cell); those past the total, up to the bound that the tables are written for, are
+// empty and no later launch reaches them.
 __device__ __forceinline__ void write_header(const SubHdrArgs& h, const int* start, const int* count,
                                              const int* bs, const int* nb, int sidx) {
   const int total = h.sub_start[h.nbins];
