@@ -2538,7 +2538,7 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   // for that input are the random ones it began with (three transforms, type 1:
   // 4e5 points, 3D FP32, 1003 us by them, 614 without; 1e5 points, 2D FP32 210 / 133)
   if (!kept) f[8] = 0.f;
-  const bool sparse = f[7] < 0.f, even = f[11] < 1.f;  // under a point per cell; peak under twice the mean
+  const bool sparse = f[7] < 2.f, even = f[11] < 1.f;  // under four points per cell; peak under twice the mean
   const float* mean = kept ? chain_selector::kSelMean : kSelMean;
   const float* sd = kept ? chain_selector::kSelStd : kSelStd;
   for (int k = 0; k < CUFINUFFT_MLP_FEATURES; ++k) f[k] = (f[k] - mean[k]) / sd[k];
@@ -2552,12 +2552,22 @@ static int choose_layout(Plan<T>* p, const PlaceArgs<T>& src) {
   }
   if (best < 0) return 0;
   // 2D FP32 type 2: the network's classes lie close together for one call, not for plans
-  // that run side by side, where the chip is full and each tile load counts.  Below a point
-  // per cell 32^2 bins instead of 16^2 make the single call faster too (0.94 of the time on
-  // average over a sweep; 1.01 above), and so do whole bins of even points where there are
-  // enough of them (0.94, below).  61 plans of a batch, 9e4 to 9e5 points each, ns 6: 1004 us
-  // without, 964 with both.
-  const bool flat = is_single<T>() && p->dim == 2 && p->type == 2 && cand[best].method == 2 && !kept;
+  // that run side by side, where the chip is full and each tile load counts.  Below four
+  // points per cell 32^2 bins instead of 16^2 cost the single call nothing (a sweep's
+  // average: 0.94 of the time below one point, 1.00 to four, 1.01 above), and whole bins
+  // of even points make it faster where there are enough of them (0.94, below).  61 plans
+  // of a batch, 9e4 to 9e5 points each: ns 6 1004 us without, 964 with both; ns 5 963 with
+  // 32^2 below one point only, 955 below four.
+  // Gathers (2780 us for the 61 plans) only where they are predicted ahead by 15%: nearer
+  // ones are no faster (0.99 on average), two of the ns 5 plans took them (955 -> 950).
+  const bool plane = is_single<T>() && p->dim == 2 && p->type == 2 && !kept;
+  if (plane && best < 3) {
+    int tiles = -1;
+    for (int k = 3; k < 9; ++k)
+      if (cand[k].ms != -2.f && (tiles < 0 || y[k] < y[tiles])) tiles = k;
+    if (tiles >= 0 && y[tiles] - y[best] < 0.2f) best = tiles;
+  }
+  const bool flat = plane && cand[best].method == 2;
   if (flat && sparse && best <= 4 && cand[best + 2].ms != -2.f) best += 2;
   const int bs[3] = {cand[best].binsizex, cand[best].binsizey, cand[best].binsizez};
   int ms = cand[best].maxsubprobsize;

@@ -39,9 +39,10 @@ def test_full_subproblems(modes, M, eps, spread):
 
 
 @pytest.mark.parametrize("modes,M,sparse", [((438, 671), 1100000, True), ((323, 219), 274583, True), ((314, 515), 435715, True),
-                                            ((239, 501), 142454, True), ((235, 296), 911085, False), ((180, 200), 150001, False)])
+                                            ((239, 501), 142454, True), ((235, 296), 911085, True), ((180, 200), 150001, True),
+                                            ((180, 200), 700000, False)])
 def test_even_points_of_a_plan_among_others(modes, M, sparse):
-    """2D FP32 type 2, uniform points: no 16^2 bins below one point per cell, and the bins
+    """2D FP32 type 2, uniform points: no 16^2 bins below four points per cell, and the bins
     that fill the chip are not split at 256 points."""
     import torch
 
@@ -51,7 +52,7 @@ def test_even_points_of_a_plan_among_others(modes, M, sparse):
     plan = cufinufft(2, modes, eps=1e-5, dtype=np.float32, gpu_method=0)
     plan.set_pts(*[(torch.rand(M, generator=g, device="cuda") * 2 - 1) * 3.1415 for _ in modes])
     i = plan.info()
-    assert (M < i["nf1"] * i["nf2"]) == sparse
+    assert (M < 4 * i["nf1"] * i["nf2"]) == sparse
     if i["method"] == 2:
         assert not sparse or min(i["binsizex"], i["binsizey"]) >= 32, i
         assert i["nbins"] < 304 or i["nsubprob"] <= M // 1024 + i["nbins"], i
